@@ -75,6 +75,9 @@ struct dg_ctx {
   float* blk_part = nullptr;           // fp32 partial planes of the output projection, [4][rows][hidden]
   uint16_t* topk_scores = nullptr;     // dg_attn_denoise_topk: bf16 score plane [Hkv][canvas * G][ld]
   size_t topk_elems = 0;
+  uint4* bits = nullptr;               // dg_attn_denoise_bitmap: the packed bitmap [canvas][tiles] and its live-tile flags
+  uint8_t* bits_live = nullptr;
+  size_t bits_tiles = 0;               // capacity in 128-key tiles, for kMaxCanvas rows
   size_t blk_rows = 0, blk_hidden = 0, blk_qe = 0, blk_ke = 0;
   CUtensorMap blk_tm_xn, blk_tm_o;
   struct WMap {
@@ -277,6 +280,20 @@ static int32_t ensure_stage(dg_ctx* ctx, size_t q_elems, size_t kv_elems) {
   return DG_OK;
 }
 
+static int32_t ensure_bits(dg_ctx* ctx, size_t tiles) {
+  if (tiles <= ctx->bits_tiles) return DG_OK;
+  DG_CUDA(cudaStreamSynchronize(ctx->stream));
+  cudaFree(ctx->bits);
+  cudaFree(ctx->bits_live);
+  ctx->bits = nullptr;
+  ctx->bits_live = nullptr;
+  ctx->bits_tiles = 0;
+  DG_CUDA(cudaMalloc(&ctx->bits, tiles * kMaxCanvas * sizeof(uint4)));
+  DG_CUDA(cudaMalloc(&ctx->bits_live, tiles * pack_attend_runs(kMaxCanvas)));
+  ctx->bits_tiles = tiles;
+  return DG_OK;
+}
+
 // ------------------------------------------------------------------------------------------
 // context
 // ------------------------------------------------------------------------------------------
@@ -357,6 +374,8 @@ extern "C" int32_t dg_ctx_destroy(dg_ctx* c) {
   cudaFree(c->blk_o);
   cudaFree(c->blk_part);
   cudaFree(c->topk_scores);
+  cudaFree(c->bits);
+  cudaFree(c->bits_live);
   for (cudaEvent_t e : c->ev) cudaEventDestroy(e);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
@@ -765,6 +784,7 @@ struct AttnCall {
   bool q_prenormed = false;
   bool early_q = false;          // the table was not written by the append launched just before
   const uint8_t* attend = nullptr;
+  bool packed = false;           // the bitmap's packed form is in the context's buffers: the tensor kernels take it
   void* out = nullptr;           // bf16, or NULL for partial
   float* out_o = nullptr;
   float* out_m = nullptr;
@@ -813,6 +833,17 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     const int32_t rr = check_ring_span(kv, p.mask, d.canvas);
     if (rr != DG_OK) return rr;
   }
+  if (a.packed) {
+    // the bitmap alone decides what a row sees: every tile up to the end of the canvas is a candidate
+    dg_layer_desc open = d;
+    open.mask_mode = DG_MASK_NONE;
+    p.mask = make_mask(open, a.kv_len, 0, 0xffffffffu, 1);
+    p.bits = c->bits;
+    p.bits_live = c->bits_live;
+    p.n_bits = (a.kv_len + d.canvas + 127u) / 128u;
+    p.n_live_rows = pack_attend_runs(d.canvas);
+    p.early_q = 0u;
+  }
   p.C = d.canvas;
   p.Hq = d.n_q_heads;
   p.Hkv = d.n_kv_heads;
@@ -836,7 +867,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     p.ap_write_end = a.ap_write_end;
   }
 
-  const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general && a.attend == nullptr &&
+  const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general && (a.attend == nullptr || a.packed) &&
                       (a.q_prenormed || fused_q_prologue_ok(d));
   if (a.ap_k != nullptr && !(tensor && d.head_dim == 256))
     return fail(DG_ERR_INVALID_ARG, "internal: in-launch append needs the head_dim-256 tensor kernel");
@@ -854,7 +885,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     // The two value halves split the score work and exchange P unless the single form is asked for; on top of
     // that, pairs of query tiles of one KV head share their K and V stages (cta_group::2) when the head has an
     // even number of tiles (pair mode 1 = the exchange alone, 2 = automatic)
-    const bool pair5 = !fixed && c->pair_mode != 0;
+    const bool pair5 = !fixed && c->pair_mode != 0 && !a.packed;
     const bool quad5 = pair5 && c->pair_mode == 2 && sm100_query_tiles(p.C, p.G, 1) % 2 == 0;
     p.n_splits = choose_splits(c, q_tiles5 * 2, pair5 ? sm100_hd512x_key_steps(p.mask) : sm100_hd512_key_tiles(p.mask));
     p.cluster_splits = 1;
@@ -894,7 +925,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
   // more than the per-tile saving returns below about a hundred key tiles.
   const uint32_t tiles_per_head = sm100_query_tiles(p.C, p.G, 1);
   const uint32_t k_tiles = sm100_key_tiles(p.mask);
-  const bool pair = !fixed && (c->pair_mode == 1 || (c->pair_mode == 2 && tiles_per_head >= 2 && k_tiles >= 96));
+  const bool pair = !fixed && !a.packed && (c->pair_mode == 1 || (c->pair_mode == 2 && tiles_per_head >= 2 && k_tiles >= 96));
   const uint32_t q_tiles = pair ? sm100_pair_query_tiles(p.C, p.G, p.Hkv) : sm100_query_tiles(p.C, p.G, p.Hkv);
   if (q_tiles > (fixed ? fixed->n_counters : kMaxQueryTiles)) return fail(DG_ERR_UNSUPPORTED, "too many query tiles");
   p.n_splits = choose_splits(c, q_tiles * c->concurrent, k_tiles);
@@ -913,7 +944,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     p.ws_o = fixed->o;
     p.ws_ml = fixed->ml;
     p.ws_counters = fixed->counters;
-  } else if (p.n_splits % 2 == 0) {
+  } else if (p.n_splits % 2 == 0 && !a.packed) {   // under a bitmap the splits meet as fp32 in the workspace
     if (pair) p.cluster_splits = 2;
     else if (p.n_splits == 2 || p.n_splits == 4 || p.n_splits == 8) p.cluster_splits = p.n_splits;
   }
@@ -961,7 +992,18 @@ static int32_t denoise_one(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, uint32_
   // leaves nothing queued (a split-KV group then stays in step with its peers)
   r = check_ring_span(kv, make_mask(d, kv_len, a.t0, a.t1, a.include_canvas), d.canvas);
   if (r != DG_OK) return r;
-  const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general && attend == nullptr;
+  const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general;
+  // A bitmap is packed for the tensor kernels on every geometry they have: the packing reads it once (about 3 us for
+  // 256 x 2,304), the CUDA-core kernel that other head_dims use visits keys one by one
+  if (tensor && attend != nullptr) {
+    const uint32_t T = kv_len + d.canvas;
+    r = ensure_bits(c, (size_t(T) + 127) / 128);
+    if (r != DG_OK) return r;
+    const cudaError_t e = launch_pack_attend(attend, d.canvas, T, c->bits, c->bits_live, launch_stream(c));
+    if (e != cudaSuccess) return fail_cuda(e, "launch_pack_attend");
+    c->last_launches += 1;
+    a.packed = true;
+  }
   if (tensor && !fused_q_prologue_ok(d)) {
     // partial / proportional rotary: run the stand-alone Q prologue into the staging buffer
     r = ensure_stage(c, size_t(d.canvas) * d.n_q_heads * d.head_dim, 0);

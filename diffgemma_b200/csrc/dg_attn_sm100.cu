@@ -87,7 +87,11 @@ __device__ __forceinline__ void row_group_sync(uint32_t smw) {
 // per pair and is read from it half as often.  tm_k then has boxes {64 d, 64 keys}.  No load uses
 // multicast.
 // blockIdx.z selects one of the independent canvases of the launch: its parameters and tensor maps.
-template <bool PAIR>
+// BITS (single-CTA form only): visibility comes from a packed decoder bitmap instead of the mask rule.  P then goes to
+// the PV MMAs as the sum of two bf16 (its rounding and what that rounding left), twice the PV work, and key splits meet
+// as fp32 in the workspace: what this path replaces kept P and its partial sums in fp32.  4,096 rows x 2,304 keys of
+// 2 KV heads: 1,933 us in the CUDA-core kernel (a warp per key, bound by L2), 43.6 us here with the packing kernel.
+template <bool PAIR, bool BITS>
 __global__ void __launch_bounds__(one::THREADS, 1)
 dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   using namespace one;
@@ -133,14 +137,15 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
                                 : mbar_wait(bar_addr(bar_base, idx), parity, flag);
   };
 
+  static_assert(!(PAIR && BITS), "the bitmap form runs one CTA per query tile");
+  uint32_t* live = reinterpret_cast<uint32_t*>(smem + OFF_ML);   // BITS: tiles with a visible key (no cluster merge then)
   // both CTAs of a pair walk the same key tiles: schedule from the pair's first canvas row
   const uint32_t row_first = ((PAIR ? (mt & ~1u) : mt) * BM) / p.G;
   const uint32_t row_last = (((PAIR ? (mt | 1u) : mt) + 1u) * BM - 1u) / p.G;
   const TileSched ts = tile_sched(mk, row_first < p.C ? row_first : p.C - 1, row_last < p.C ? row_last : p.C - 1);
-  const uint32_t n_tiles = ts.nA + ts.nB;
-  const uint32_t v_begin = uint32_t((uint64_t(split) * n_tiles) / p.n_splits);
-  const uint32_t v_end = uint32_t((uint64_t(split + 1) * n_tiles) / p.n_splits);
-  const uint32_t n_local = v_end - v_begin;
+  uint32_t n_tiles = ts.nA + ts.nB;
+  uint32_t v_begin = uint32_t((uint64_t(split) * n_tiles) / p.n_splits);
+  uint32_t v_end = uint32_t((uint64_t(split + 1) * n_tiles) / p.n_splits);
 
   // Q prologue, first half: a warp copies its eight raw query rows asynchronously into their final
   // (swizzled) place, lane c the 16-byte chunk c of each row.  When Q does not come from the kernel
@@ -206,6 +211,14 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   // that kernel (the table is cached across steps at the same positions) they skip the wait, so the
   // whole Q prologue overlaps the append; the loaders always wait before they touch the cache.
   if (!(p.early_q && warp < SM_WARPS)) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (BITS) {   // never early: the packed bitmap comes from the kernel ahead
+    build_live_words(p, live);
+    __syncthreads();
+    n_tiles = count_live_tiles(p, live);
+    v_begin = uint32_t((uint64_t(split) * n_tiles) / p.n_splits);
+    v_end = uint32_t((uint64_t(split + 1) * n_tiles) / p.n_splits);
+  }
+  const uint32_t n_local = v_end - v_begin;
   stamp(p, 1);
   volatile uint32_t* abort_flag = &ctl[1];
   const bool prof = p.stamps != nullptr;
@@ -394,11 +407,13 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     const uint32_t p2_full0 = PAIR ? lead_bar(B_P2_FULL) : bar_addr(bar_base, B_P2_FULL);
     const uint32_t p2_full1 = PAIR ? lead_bar(B_P2_FULL + 1) : bar_addr(bar_base, B_P2_FULL + 1);
 
+    TileWalk<BITS> walk(p, ts, live, v_begin);
     for (uint32_t n = 0; n < n_local; ++n) {
-      const uint32_t v = v_begin + n;
-      const uint32_t jt = v < ts.nA ? ts.a0 + v : ts.b0 + (v - ts.nA);
+      const uint32_t jt = walk.next();
       const uint32_t k0 = jt * BN;
       const uint32_t b = n & 1u;
+      uint4 vis = make_uint4(0u, 0u, 0u, 0u);
+      if (BITS) vis = p.bits[size_t(i_row) * p.n_bits + jt];
       // warp-uniform outcome: the TMEM instructions below need the whole warp
       if (!__all_sync(0xffffffffu, timed_wait(prof, w_s, [&] { return wait_bar(B_S_FULL + b, (n >> 1) & 1u, abort_flag); }))) break;
       tc_fence_after();
@@ -410,7 +425,14 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       tmem_ld16(t_lane + TM_S + b * 128u + 64u + qd * (CPT / 2), *reinterpret_cast<uint32_t(*)[16]>(&sraw[16]));
       tmem_wait_ld();
 
-      if (!mask_range_full(mk, rv, k0, BN)) {
+      if (BITS) {
+        // bit e of `seen`: is key e of this thread's two runs visible to the row
+        const uint32_t sh = (qd & 1u) * 16u;
+        const uint32_t seen = (((qd < 2u ? vis.x : vis.y) >> sh) & 0xffffu) | (((qd < 2u ? vis.z : vis.w) >> sh) << 16);
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          if (!((seen >> e) & 1u)) sraw[e] = 0xff800000u;
+      } else if (!mask_range_full(mk, rv, k0, BN)) {
 #pragma unroll
         for (int e = 0; e < 32; ++e)
           if (!mask_visible_row(mk, rv, k0 + (e < 16 ? 0u : 48u) + qd * (CPT / 2) + e)) sraw[e] = 0xff800000u;  // -inf
@@ -457,7 +479,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       uint64_t ls2[2] = {0ull, 0ull};   // (0.f, 0.f)
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-        uint32_t pk[8];
+        uint32_t pk[8], pl[8];
 #pragma unroll
         for (int e = 0; e < 16; e += 2) {
           float x0, x1;
@@ -465,8 +487,10 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
           const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
           ls2[(e >> 1) & 1] = add_f32x2(ls2[(e >> 1) & 1], pack_f32x2(p0, p1));
           pk[e >> 1] = pack_bf16x2(p0, p1);
+          if (BITS) pl[e >> 1] = pack_bf16x2(p0 - __uint_as_float(pk[e >> 1] << 16), p1 - __uint_as_float(pk[e >> 1] & 0xffff0000u));
         }
         tmem_st8(t_lane + TM_S + b * 128u + uint32_t(hf) * 32u + qd * (CPT / 4), pk);
+        if (BITS) tmem_st8(t_lane + TM_S + b * 128u + 64u + uint32_t(hf) * 32u + qd * (CPT / 4), pl);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -489,9 +513,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     // ---------------------------------------------------------------- K loader
     if (lane == 0) {
       bool canvas_ready = p.ap_vectors == 0u || mk.can_hi <= mk.kv_len;
+      TileWalk<BITS> walk(p, ts, live, v_begin);
       for (uint32_t n = 0; n < n_local; ++n) {
-        const uint32_t v = v_begin + n;
-        const uint32_t jt = v < ts.nA ? ts.a0 + v : ts.b0 + (v - ts.nA);
+        const uint32_t jt = walk.next();
         if (!canvas_ready && jt * BN + BN > mk.kv_len) {
           if (!wait_counter_gpu(p.ap_ctl + 1, p.ap_vectors, abort_flag)) break;
           canvas_ready = true;
@@ -520,9 +544,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     // ---------------------------------------------------------------- V loader
     if (lane == 0) {
       bool canvas_ready = p.ap_vectors == 0u || mk.can_hi <= mk.kv_len;
+      TileWalk<BITS> walk(p, ts, live, v_begin);
       for (uint32_t n = 0; n < n_local; ++n) {
-        const uint32_t v = v_begin + n;
-        const uint32_t jt = v < ts.nA ? ts.a0 + v : ts.b0 + (v - ts.nA);
+        const uint32_t jt = walk.next();
         if (!canvas_ready && jt * BN + BN > mk.kv_len) {
           if (!wait_counter_gpu(p.ap_ctl + 1, p.ap_vectors, abort_flag)) break;
           canvas_ready = true;
@@ -635,6 +659,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
               const uint64_t db = mkdesc(vb + j * (2048u >> 4), HI_MNMAJ);
               if (PAIR) umma_ts_pair(tmem + TM_O, p_tmem + j * 8u, db, IDESC_PV, (n | hf | j) != 0u);
               else umma_ts(tmem + TM_O, p_tmem + j * 8u, db, IDESC_PV, (n | hf | j) != 0u);
+              if (BITS) umma_ts(tmem + TM_O, p_tmem + 64u + j * 8u, db, IDESC_PV, 1u);
             }
             if (hf == 1) {
               commit(B_V_EMPTY + (n & 1u));
@@ -1165,10 +1190,12 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
 }
 
 cudaError_t sm100_attn_configure() {
-  return cudaFuncSetAttribute(dg_attn_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES));
+  const cudaError_t e = cudaFuncSetAttribute(dg_attn_sm100_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES));
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(dg_attn_sm100_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES));
 }
 cudaError_t sm100_pair_configure() {
-  return cudaFuncSetAttribute(dg_attn_sm100_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES));
+  return cudaFuncSetAttribute(dg_attn_sm100_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES));
 }
 
 // How many clusters of (cluster_x, cluster_y, 1) CTAs of the kernel the device can hold at once.
@@ -1186,7 +1213,7 @@ static int max_active_clusters(uint32_t cluster_y) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, dg_attn_sm100_kernel<PAIR>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, dg_attn_sm100_kernel<PAIR, false>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
@@ -1206,7 +1233,7 @@ uint32_t sm100_key_tiles(const MaskParams& mk) {
   return t.nA + t.nB;
 }
 
-template <bool PAIR>
+template <bool PAIR, bool BITS>
 static cudaError_t launch(const AttnParams* ps, const CUtensorMap* const* tm_k, const CUtensorMap* const* tm_v, uint32_t n,
                           cudaStream_t st) {
   if (n == 0 || n > kMaxBatchLaunch) return cudaErrorInvalidValue;
@@ -1241,26 +1268,26 @@ static cudaError_t launch(const AttnParams* ps, const CUtensorMap* const* tm_k, 
   }
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  return cudaLaunchKernelEx(&cfg, dg_attn_sm100_kernel<PAIR>, bat);
+  return cudaLaunchKernelEx(&cfg, dg_attn_sm100_kernel<PAIR, BITS>, bat);
 }
 
 cudaError_t launch_attn_sm100(const AttnParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
                               cudaStream_t st) {
   const CUtensorMap* k = &tm_k;
   const CUtensorMap* v = &tm_v;
-  return launch<false>(&p, &k, &v, 1, st);
+  return p.bits != nullptr ? launch<false, true>(&p, &k, &v, 1, st) : launch<false, false>(&p, &k, &v, 1, st);
 }
 // tm_k64: K tensor map with boxes {64 d, 64 keys, 1}
 cudaError_t launch_attn_sm100_pair(const AttnParams& p, const CUtensorMap& tm_k64, const CUtensorMap& tm_v,
                                    cudaStream_t st) {
   const CUtensorMap* k = &tm_k64;
   const CUtensorMap* v = &tm_v;
-  return launch<true>(&p, &k, &v, 1, st);
+  return launch<true, false>(&p, &k, &v, 1, st);
 }
 // n <= kMaxBatchLaunch independent canvases in one launch (same geometry, split count and kernel form)
 cudaError_t launch_attn_sm100_batch(const AttnParams* p, const CUtensorMap* const* tm_k, const CUtensorMap* const* tm_v,
                                     uint32_t n, bool pair, cudaStream_t st) {
-  return pair ? launch<true>(p, tm_k, tm_v, n, st) : launch<false>(p, tm_k, tm_v, n, st);
+  return pair ? launch<true, false>(p, tm_k, tm_v, n, st) : launch<false, false>(p, tm_k, tm_v, n, st);
 }
 
 }  // namespace dg

@@ -56,6 +56,75 @@ __host__ __device__ inline TileSched tile_sched(const MaskParams& mk, uint32_t r
   return t;
 }
 
+// Key tiles of a launch under a decoder bitmap (p.bits): the 128-key tiles in which any canvas row sees a key, as a
+// bit per tile in shared memory, so that padding and windows expressed as a bitmap cost no tile visits.
+constexpr uint32_t LIVE_WORDS = 32;                       // up to 1,024 tiles = 131,072 keys; longer ranges visit every tile
+__device__ __forceinline__ void build_live_words(const AttnParams& p, uint32_t* live) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, n_warps = blockDim.x >> 5;
+  for (uint32_t w = warp; w < LIVE_WORDS; w += n_warps) {
+    const uint32_t j = w * 32u + lane;
+    uint32_t any = 0u;
+    if (j < p.n_bits)
+      for (uint32_t c = 0; c < p.n_live_rows; ++c) any |= p.bits_live[size_t(c) * p.n_bits + j];
+    const uint32_t word = __ballot_sync(0xffffffffu, any != 0u);
+    if (lane == 0) live[w] = word;
+  }
+}
+__device__ __forceinline__ uint32_t count_live_tiles(const AttnParams& p, const uint32_t* live) {
+  if (p.n_bits > LIVE_WORDS * 32u) return p.n_bits;
+  uint32_t n = 0;
+  for (uint32_t w = 0; w * 32u < p.n_bits; ++w) n += __popc(live[w]);
+  return n;
+}
+
+// Hands out a CTA's key tiles in order, starting with number v of its schedule.  With BITS the schedule is the live
+// tiles, else the two intervals of TileSched.
+template <bool BITS>
+struct TileWalk {
+  TileSched ts;
+  uint32_t v;
+  const uint32_t* live = nullptr;
+  uint32_t word = 0, w = 0;
+  __device__ __forceinline__ TileWalk(const AttnParams& p, const TileSched& t, const uint32_t* live_words, uint32_t v0) : ts(t), v(v0) {
+    if (BITS && p.n_bits <= LIVE_WORDS * 32u) {
+      live = live_words;
+      word = live[0];
+      uint32_t skip = v0;
+      while (w + 1u < LIVE_WORDS && skip >= uint32_t(__popc(word))) {
+        skip -= __popc(word);
+        word = live[++w];
+      }
+      for (; skip > 0u; --skip) word &= word - 1u;
+    }
+  }
+  __device__ __forceinline__ uint32_t next() {
+    if (BITS && live != nullptr) {
+      while (word == 0u && w + 1u < LIVE_WORDS) word = live[++w];
+      const uint32_t b = word ? __ffs(word) - 1u : 0u;
+      word &= word - 1u;
+      return w * 32u + b;
+    }
+    const uint32_t n = v++;
+    return n < ts.nA ? ts.a0 + n : ts.b0 + (n - ts.nA);
+  }
+};
+
+// The same for the 64-key tiles of the head_dim-512 kernels: both halves of every 128-key tile.
+struct TileWalk64Bits {
+  TileWalk<true> walk;
+  uint32_t half, cur = 0;
+  __device__ __forceinline__ TileWalk64Bits(const AttnParams& p, const TileSched& t, const uint32_t* live_words, uint32_t v0)
+      : walk(p, t, live_words, v0 >> 1), half(v0 & 1u) {
+    if (half) cur = walk.next();
+  }
+  __device__ __forceinline__ uint32_t next() {
+    if (half == 0u) cur = walk.next();
+    const uint32_t jt = 2u * cur + half;
+    half ^= 1u;
+    return jt;
+  }
+};
+
 __device__ __forceinline__ uint32_t bar_addr(uint32_t bar_base, uint32_t idx) { return bar_base + idx * 8u; }
 
 // Phase time stamps (globaltimer, ns) of one CTA, written by thread 0 when a stamp buffer is given:

@@ -25,6 +25,8 @@
 //     counter merges.  Every wait is bounded.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "dg_attn_sm100_hd512.cuh"
 #include "dg_kernels.h"
 
@@ -52,6 +54,8 @@ __device__ __forceinline__ void row_pair_sync(uint32_t smw) {
   asm volatile("bar.sync %0, %1;" ::"r"(smw + 1u), "n"(h5::NTR * 32) : "memory");
 }
 
+// BITS: visibility from a packed decoder bitmap, P as the sum of two bf16 (as in the head_dim-256 kernel)
+template <bool BITS>
 __global__ void __launch_bounds__(h5::THREADS, 1)
 dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_k,
                            const __grid_constant__ CUtensorMap tm_v) {
@@ -80,11 +84,10 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
 
   const uint32_t row_first = (mt * BM) / p.G;
   const uint32_t row_last = ((mt + 1u) * BM - 1u) / p.G;
-  const TileSched ts = tile_sched64(mk, row_first < p.C ? row_first : p.C - 1, row_last < p.C ? row_last : p.C - 1);
-  const uint32_t n_tiles = ts.nA + ts.nB;
-  const uint32_t v_begin = uint32_t((uint64_t(split) * n_tiles) / p.n_splits);
-  const uint32_t v_end = uint32_t((uint64_t(split + 1) * n_tiles) / p.n_splits);
-  const uint32_t n_local = v_end - v_begin;
+  uint32_t* live = reinterpret_cast<uint32_t*>(smem + O_BAR + 128u);   // BITS: 128 bytes behind the barriers and ctl
+  static_assert(B_COUNT * 8 + 12 <= 128 && LIVE_WORDS * 4 <= 128, "barrier block too small for the live-tile words");
+  const TileSched ts = BITS ? tile_sched(mk, 0, p.C - 1)
+                            : tile_sched64(mk, row_first < p.C ? row_first : p.C - 1, row_last < p.C ? row_last : p.C - 1);
 
   // ------------------------------------------------------------------ set-up
   if (tid == 0) {
@@ -113,6 +116,15 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
   // everything this kernel reads was written by kernels launched before it on the stream
   asm volatile("griddepcontrol.wait;" ::: "memory");
   volatile uint32_t* abort_flag = &ctl[1];
+  if (BITS) {
+    build_live_words(p, live);
+    __syncthreads();
+  }
+  const uint32_t n_tiles = BITS ? 2u * count_live_tiles(p, live) : ts.nA + ts.nB;
+  const uint32_t v_begin = uint32_t((uint64_t(split) * n_tiles) / p.n_splits);
+  const uint32_t v_end = uint32_t((uint64_t(split + 1) * n_tiles) / p.n_splits);
+  const uint32_t n_local = v_end - v_begin;
+  using Walk = typename std::conditional<BITS, TileWalk64Bits, TileWalk<false>>::type;
 
   const uint32_t smw = warp & 3u, half = (warp >> 2) & 1u;
   const uint32_t r = smw * 32 + lane;
@@ -131,17 +143,23 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
     const uint32_t t_lane = tmem + ((smw * 32u) << 16);
     const float sc = p.scale_log2;
 
+    Walk walk(p, ts, live, v_begin);
     for (uint32_t n = 0; n < n_local; ++n) {
-      const uint32_t v = v_begin + n;
-      const uint32_t jt = v < ts.nA ? ts.a0 + v : ts.b0 + (v - ts.nA);
+      const uint32_t jt = walk.next();
       const uint32_t k0 = jt * TN;
       const uint32_t b = n & 1u;
+      uint32_t seen = 0u;   // this thread's 32 keys
+      if (BITS) seen = reinterpret_cast<const uint32_t*>(p.bits + size_t(i_row) * p.n_bits + (jt >> 1))[(jt & 1u) * 2u + half];
       if (!__all_sync(0xffffffffu, mbar_wait(bar_addr(bar_base, B_S_FULL + b), (n >> 1) & 1u, abort_flag))) break;
       tc_fence_after();
       uint32_t sraw[32];
       tmem_ld32(t_lane + T_S + b * TN + half * CPT, sraw);
       tmem_wait_ld();
-      if (!mask_range_full(mk, rv, k0, TN)) {
+      if (BITS) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          if (!((seen >> e) & 1u)) sraw[e] = 0xff800000u;
+      } else if (!mask_range_full(mk, rv, k0, TN)) {
 #pragma unroll
         for (int e = 0; e < 32; ++e)
           if (!mask_visible_row(mk, rv, k0 + half * CPT + e)) sraw[e] = 0xff800000u;  // -inf
@@ -181,7 +199,7 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
       const float neg_m = -m_eff;
       const uint64_t sc2 = pack_f32x2(sc, sc), nm2 = pack_f32x2(neg_m, neg_m);
       uint64_t ls2[2] = {0ull, 0ull};
-      uint32_t pk[16];
+      uint32_t pk[16], pl[16];
 #pragma unroll
       for (int e = 0; e < 32; e += 2) {
         float x0, x1;
@@ -189,6 +207,7 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
         const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
         ls2[(e >> 1) & 1] = add_f32x2(ls2[(e >> 1) & 1], pack_f32x2(p0, p1));
         pk[e >> 1] = pack_bf16x2(p0, p1);
+        if (BITS) pl[e >> 1] = pack_bf16x2(p0 - __uint_as_float(pk[e >> 1] << 16), p1 - __uint_as_float(pk[e >> 1] & 0xffff0000u));
       }
       {
         float s0, s1;
@@ -197,6 +216,7 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
       }
       // P column j = keys (2j, 2j+1): this thread's 32 keys are 16 columns
       tmem_st16(t_lane + T_S + b * TN + half * (CPT / 2), pk);
+      if (BITS) tmem_st16(t_lane + T_S + b * TN + TN / 2 + half * (CPT / 2), pl);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -205,9 +225,9 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
   } else if (warp == W_K) {
     // ---------------------------------------------------------------- K loader: 8 boxes {64 d, 64 keys}
     if (lane == 0) {
+      Walk walk(p, ts, live, v_begin);
       for (uint32_t n = 0; n < n_local; ++n) {
-        const uint32_t v = v_begin + n;
-        const uint32_t jt = v < ts.nA ? ts.a0 + v : ts.b0 + (v - ts.nA);
+        const uint32_t jt = walk.next();
         // K stage n & 1 is free once QK(n - 2) has completed
         const uint32_t st = n & 1u;
         if (n > 1 && !mbar_wait(bar_addr(bar_base, B_S_FULL + st), ((n - 2) >> 1) & 1u, abort_flag)) break;
@@ -222,9 +242,9 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
   } else if (warp == W_V) {
     // ---------------------------------------------------------------- V loader: this half's 4 boxes
     if (lane == 0) {
+      Walk walk(p, ts, live, v_begin);
       for (uint32_t n = 0; n < n_local; ++n) {
-        const uint32_t v = v_begin + n;
-        const uint32_t jt = v < ts.nA ? ts.a0 + v : ts.b0 + (v - ts.nA);
+        const uint32_t jt = walk.next();
         if (n > 0 && !mbar_wait(bar_addr(bar_base, B_V_EMPTY + ((n - 1) & 1u)), ((n - 1) >> 1) & 1u, abort_flag)) break;
         const uint32_t full = bar_addr(bar_base, B_V_FULL);
         mbar_expect_tx(full, 4 * KV_ATOM);
@@ -285,8 +305,10 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
         tc_fence_after();
         const uint32_t p_tmem = tmem + T_S + (n & 1u) * TN;
 #pragma unroll
-        for (uint32_t ks = 0; ks < TN / 16; ++ks)
+        for (uint32_t ks = 0; ks < TN / 16; ++ks) {
           umma_ts(tmem + T_O, p_tmem + ks * 8u, mkdesc(v_lo + ks * (2048u >> 4), HI), IDESC_PV, (n | ks) != 0u);
+          if (BITS) umma_ts(tmem + T_O, p_tmem + TN / 2 + ks * 8u, mkdesc(v_lo + ks * (2048u >> 4), HI), IDESC_PV, 1u);
+        }
         umma_commit(bar_addr(bar_base, B_V_EMPTY + (n & 1u)));  // PV done; the V tile is free
         if (n + 1 == n_local) umma_commit(bar_addr(bar_base, B_O_FINAL));
       }
@@ -327,7 +349,9 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
 }
 
 cudaError_t sm100_hd512_configure() {
-  return cudaFuncSetAttribute(dg_attn_sm100_hd512_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(h5::SMEM_REQ));
+  const cudaError_t e = cudaFuncSetAttribute(dg_attn_sm100_hd512_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(h5::SMEM_REQ));
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(dg_attn_sm100_hd512_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(h5::SMEM_REQ));
 }
 
 uint32_t sm100_hd512_key_tiles(const MaskParams& mk) {
@@ -349,7 +373,8 @@ cudaError_t launch_attn_sm100_hd512(const AttnParams& p, const CUtensorMap& tm_k
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, dg_attn_sm100_hd512_kernel, p, tm_k, tm_v);
+  return p.bits != nullptr ? cudaLaunchKernelEx(&cfg, dg_attn_sm100_hd512_kernel<true>, p, tm_k, tm_v)
+                           : cudaLaunchKernelEx(&cfg, dg_attn_sm100_hd512_kernel<false>, p, tm_k, tm_v);
 }
 
 }  // namespace dg

@@ -152,7 +152,10 @@ struct AttnParams {
   const float2* rope_table;      // [C][rot_half]; only read when q_prenormed == 0
   const __nv_bfloat16* cache_k;  // K[Hkv][cap][D]
   const __nv_bfloat16* cache_v;
-  const uint8_t* attend;         // optional bitmap [C][kv_len+C] (general kernel only)
+  const uint8_t* attend;         // optional bitmap [C][kv_len+C] (general kernel)
+  const uint4* bits;             // the same bitmap packed: [C][n_bits] tiles of 128 keys (tensor kernels), or null
+  const uint8_t* bits_live;      // [n_live_rows][n_bits]: 1 where any of a run of canvas rows sees a key of the tile
+  uint32_t n_bits, n_live_rows;
   __nv_bfloat16* out;            // [C][Hq][D] or null when partial output is requested
   float* out_o;                  // partial: [C][Hq][D] fp32 un-normalised
   float* out_m;                  // partial: [C][Hq]

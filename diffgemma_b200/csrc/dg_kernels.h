@@ -9,6 +9,9 @@ namespace dg {
 
 void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st, bool early = false);
 void launch_attn_general(const AttnParams& p, cudaStream_t st);
+// decoder bitmap [C][T] -> bits [C][ceil(T / 128)], live [pack_attend_runs(C)][ceil(T / 128)]
+uint32_t pack_attend_runs(uint32_t C);
+cudaError_t launch_pack_attend(const uint8_t* attend, uint32_t C, uint32_t T, uint4* bits, uint8_t* live, cudaStream_t st);
 void launch_merge_local(uint32_t n_parts, uint32_t rows, uint32_t D, const float* o, const float* m,
                         const float* l, __nv_bfloat16* out, cudaStream_t st);
 void launch_merge_pack(uint32_t rows, uint32_t D, const float* o, const float* m_local, const float* m_global,

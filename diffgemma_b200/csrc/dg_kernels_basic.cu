@@ -323,6 +323,47 @@ __global__ void __launch_bounds__(GEN_WARPS * 32) dg_attn_general_kernel(const A
   }
 }
 
+// Decoder bitmap uint8 [C][T] -> one bit per key, 128-key tiles [C][n_bits] of uint4, plus for every run of PACK_ROWS
+// canvas rows and every tile whether any of the rows sees a key of it.  A CTA packs PACK_ROWS rows of one tile: four
+// 32-byte reads per row and tile, all independent.
+constexpr uint32_t PACK_ROWS = 32;
+__global__ void __launch_bounds__(256) dg_pack_attend_kernel(const uint8_t* __restrict__ attend, uint32_t C, uint32_t T,
+                                                             uint4* __restrict__ bits, uint8_t* __restrict__ live) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // the kernels ahead may still read the previous call's bits
+  const uint32_t j = blockIdx.x, n_bits = gridDim.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  uint32_t any = 0u;
+#pragma unroll
+  for (uint32_t k = 0; k < PACK_ROWS / 8u; ++k) {
+    const uint32_t row = blockIdx.y * PACK_ROWS + k * 8u + warp;
+    if (row >= C) continue;   // warp-uniform
+    uint32_t w[4];
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+      const uint32_t t = j * 128u + e * 32u + lane;
+      w[e] = __ballot_sync(0xffffffffu, t < T && attend[size_t(row) * T + t] != 0);
+      any |= w[e];
+    }
+    if (lane == 0) bits[size_t(row) * n_bits + j] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  any = __syncthreads_or(any != 0u);
+  if (threadIdx.x == 0) live[size_t(blockIdx.y) * n_bits + j] = any ? 1 : 0;
+}
+
+uint32_t pack_attend_runs(uint32_t C) { return (C + PACK_ROWS - 1u) / PACK_ROWS; }
+cudaError_t launch_pack_attend(const uint8_t* attend, uint32_t C, uint32_t T, uint4* bits, uint8_t* live, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((T + 127u) / 128u, pack_attend_runs(C));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, dg_pack_attend_kernel, attend, C, T, bits, live);
+}
+
 void launch_attn_general(const AttnParams& p, cudaStream_t st) {
   dg_attn_general_kernel<<<dim3(p.C, p.Hq), GEN_WARPS * 32, 0, st>>>(p);
 }

@@ -847,3 +847,56 @@ def test_in_launch_append_matches_the_two_kernel_step(ctx, P, Hkv, W, mode, weig
                 assert torch.equal(a, b), f"in-launch append, output differs (stable={stable}, splits={splits})"
             assert torch.equal(got[1], base[1]) and torch.equal(got[2], base[2]), "cache contents differ"
     assert ctx.device_status()[0] == 0
+
+
+# ------------------------------------------------------------------------------------------
+# decoder bitmap on the tensor kernels
+# ------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("hd,P,Hq,Hkv,canvas,kind", [
+    (256, 0, 4, 2, 1, "random"),              # one row, one partial tile
+    (256, 127, 16, 8, 100, "random"),         # ragged everywhere, canvas across a tile edge
+    (256, 2049, 16, 2, 256, "padded"),        # dead tiles in front, splits meet in the workspace
+    (256, 700, 16, 2, 64, "blind"),           # rows and whole tiles that see nothing
+    (256, 131400, 2, 1, 3, "sparse"),         # more tiles than the live-tile words hold
+    (512, 63, 4, 2, 5, "random"),
+    (512, 1000, 16, 2, 200, "padded"),        # an odd number of 64-key halves ahead of the canvas
+    (512, 500, 8, 8, 33, "blind"),
+])
+def test_bitmap_tensor_path(ctx, hd, P, Hq, Hkv, canvas, kind):
+    """Against the oracle, and against the CUDA-core kernel: both keep P to at least 16 bits and sum in fp32, so their
+    bf16 outputs are the same value or neighbours (one step is 2^-7 of a value at most), plus what the order of the fp32
+    sums and a rounding of Q to the other side leave near zero (2e-3 of outputs below 4 in magnitude)."""
+    layer = AttnLayer(n_q_heads=Hq, n_kv_heads=Hkv, head_dim=hd, canvas=canvas, rope_theta=1e6, v_norm=int(hd == 512),
+                      rotary_dim=128 if hd == 512 else 256,
+                      rope_pairing=capi.ROPE_PROPORTIONAL if hd == 512 else capi.ROPE_SPLIT_HALF)
+    case = util.make_case(layer, P, seed=P + hd + canvas, weights=True)
+    T = P + canvas
+    rng = np.random.default_rng(P + hd)
+    if kind == "padded":
+        seen = np.broadcast_to(np.arange(T) >= P // 3, (canvas, T)).copy()
+    else:
+        seen = rng.random((canvas, T)) < (0.01 if kind == "sparse" else 0.6)
+    if kind == "blind":
+        seen[::7] = False
+        seen[:, 128:256] = False
+    kv, att = util.gpu_setup(ctx, case)
+    args = (util.dev(case, "q"), util.dev(case, "kc"), util.dev(case, "vc"), torch.from_numpy(seen.astype(np.uint8)).to(DEV),
+            util.dev(case, "qw"), util.dev(case, "kw"))
+    try:
+        ctx.force_general(True)
+        general = util.t2f(att.denoise_bitmap(kv, P, *args))
+        ctx.force_general(False)
+        for splits in (0, 1, 2, 5):
+            ctx.set_splits(splits)
+            outs = [util.t2f(att.denoise_bitmap(kv, P, *args)) for _ in range(2)]
+            assert np.array_equal(*outs)
+            np.testing.assert_allclose(outs[0], general, rtol=2.0 ** -7, atol=2e-3)
+            if kind == "blind":
+                assert (outs[0][::7] == 0).all()
+    finally:
+        ctx.force_general(False)
+        ctx.set_splits(0)
+    assert ctx.device_status()[0] == 0
+    if kind != "sparse":
+        util.assert_close(outs[0], util.run_oracle(case, attend=seen), f"bitmap {kind}")
+    kv.close()
