@@ -617,6 +617,38 @@ static SlotRuns slot_runs(const dg_kv* kv, uint64_t pos0, uint64_t n) {
   return r;
 }
 
+// One kernel for K, V and all heads where both tensors are this device's own memory (8,192 tokens of 2 x 512: a strided
+// copy per head, tensor and run of slots otherwise).  Host and peer memory, and tensors off 16-byte boundaries, stay
+// with the copies.  *done says whether the kernel was launched.
+static int32_t kv_copy_device(dg_kv* kv, void* k, void* v, uint64_t pos0, uint64_t n, bool to_cache, bool* done) {
+  *done = false;
+  const uint64_t chunks = n * kv->Hkv * (kv->D / 8);
+  if (chunks >= (1ull << 31) || !aligned16(k) || !aligned16(v)) return DG_OK;
+  for (const void* p : {k, v}) {
+    cudaPointerAttributes at = {};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      return DG_OK;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != kv->ctx->device) return DG_OK;
+  }
+  KvCopyParams p = {};
+  p.k = k;
+  p.v = v;
+  p.cache_k = kv->k;
+  p.cache_v = kv->v;
+  p.cap = kv->cap;
+  p.n_chunks = uint32_t(chunks);
+  p.row_chunks = kv->D / 8;
+  p.Hkv = kv->Hkv;
+  p.ring_mask = kv->ring_mask ? kv->ring_mask : 0xffffffffu;
+  p.slot0 = kv->ring_mask ? uint32_t(pos0 & kv->ring_mask) : uint32_t(pos0 - kv->pos_base);
+  p.to_cache = to_cache ? 1u : 0u;
+  DG_CUDA(launch_kv_copy(p, kv->ctx->stream));
+  *done = true;
+  return DG_OK;
+}
+
 extern "C" int32_t dg_kv_load_prefix(dg_kv* kv, const void* k, const void* v, uint64_t pos0, uint64_t n) {
   if (!kv || !k || !v) return fail(DG_ERR_INVALID_ARG, "NULL argument");
   if (kv->ring_mask == 0 && (pos0 < kv->pos_base || pos0 + n > kv->pos_base + kv->cap))
@@ -626,6 +658,13 @@ extern "C" int32_t dg_kv_load_prefix(dg_kv* kv, const void* k, const void* v, ui
   const size_t row = size_t(kv->D) * 2, spitch = size_t(kv->Hkv) * row;
   const SlotRuns runs = slot_runs(kv, pos0, n);
   uint64_t done = runs.skip;
+  {
+    bool copied = false;
+    const size_t skip = size_t(runs.skip) * spitch;
+    const int32_t r = kv_copy_device(kv, static_cast<uint8_t*>(const_cast<void*>(k)) + skip,
+                                     static_cast<uint8_t*>(const_cast<void*>(v)) + skip, pos0 + runs.skip, n - runs.skip, true, &copied);
+    if (r != DG_OK || copied) return r;
+  }
   for (int s = 0; s < 2; ++s) {
     if (runs.len[s] == 0) continue;
     for (uint32_t h = 0; h < kv->Hkv; ++h) {
@@ -649,7 +688,10 @@ extern "C" int32_t dg_kv_read(dg_kv* kv, void* k_out, void* v_out, uint64_t pos0
   const size_t row = size_t(kv->D) * 2, dpitch = size_t(kv->Hkv) * row;
   const SlotRuns runs = slot_runs(kv, pos0, n);
   uint64_t done = 0;
-  for (int s = 0; s < 2; ++s) {
+  bool copied = false;
+  const int32_t r = n == 0 ? DG_OK : kv_copy_device(kv, k_out, v_out, pos0, n, false, &copied);
+  if (r != DG_OK) return r;
+  for (int s = 0; s < 2 && !copied; ++s) {
     if (runs.len[s] == 0) continue;
     for (uint32_t h = 0; h < kv->Hkv; ++h) {
       DG_CUDA(cudaMemcpy2DAsync(static_cast<uint8_t*>(k_out) + done * dpitch + h * row, dpitch,

@@ -145,6 +145,20 @@ struct AppendParams {
   uint32_t pos_base;           // first position the cache holds (a shard of a long prefix; 0 otherwise)
 };
 
+// session copy: rows of a token-major [n][Hkv][D] tensor to or from the cache
+struct KvCopyParams {
+  void* k;                     // [n][Hkv][D]
+  void* v;
+  __nv_bfloat16* cache_k;      // K[Hkv][cap][D]
+  __nv_bfloat16* cache_v;
+  uint64_t cap;
+  uint32_t n_chunks;           // n * Hkv * row_chunks, 16 bytes each
+  uint32_t row_chunks;         // D / 8
+  uint32_t Hkv;
+  uint32_t slot0, ring_mask;   // cache slot of token i = (slot0 + i) & ring_mask
+  uint32_t to_cache;
+};
+
 // attention kernels (general and sm100)
 struct AttnParams {
   const __nv_bfloat16* q;        // [C][Hq][D]

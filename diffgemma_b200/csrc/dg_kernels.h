@@ -8,6 +8,8 @@
 namespace dg {
 
 void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st, bool early = false);
+// device memory to or from the cache (n_chunks < 2^31, 16-byte aligned tensors)
+cudaError_t launch_kv_copy(const KvCopyParams& p, cudaStream_t st);
 void launch_attn_general(const AttnParams& p, cudaStream_t st);
 // decoder bitmap [C][T] -> bits [C][ceil(T / 128)], live [pack_attend_runs(C)][ceil(T / 128)]
 uint32_t pack_attend_runs(uint32_t C);

@@ -141,6 +141,160 @@ __global__ void __launch_bounds__(256) dg_append_table_kernel(const AppendParams
   append_table_vector(a, w, lane);
 }
 
+// ------------------------------------------------------------------------------------------
+// The same stage for head_dim 256 and 512 with rotary runs of whole 16-byte chunks: a CTA takes one or a few tokens,
+// computes their (cos, sin) pairs once into shared memory, and a warp handles two head vectors at a time, lane c the
+// 16-byte chunks c and c + 32 together with the chunks that hold their rotation partners.
+// Bound: latency at canvas size, memory on long appends.  The kernel above issues a warp per CTA, 2-byte accesses and
+// a sincos per (vector, pair): a head_dim-512 step took 5 us longer with it (32k keys 295.8 -> 290.8 us, 150 keys
+// 23.4 -> 21.9 us).  Order of operations (chunk-wise sums of squares, butterfly, rotation through
+// rope_rotate / rope_norm_rotate) as above: both write the same bits.
+// ------------------------------------------------------------------------------------------
+constexpr uint32_t kRowsMaxTok = 4, kRowsMaxWarps = 10, kRowsUnit = 2;
+
+template <uint32_t NS>   // 16-byte chunks of a vector per lane: head_dim 256 -> 1, 512 -> 2
+__global__ void __launch_bounds__(kRowsMaxWarps * 32) dg_append_rows_kernel(const AppendParams p, const RopeParams rp, uint32_t tok_per_cta) {
+  __shared__ float2 cs[kRowsMaxTok * kMaxRotHalf];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // see dg_append_kernel
+  constexpr uint32_t D = NS * 256u, U = kRowsUnit;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+  const uint32_t tok0 = blockIdx.x * tok_per_cta;
+  const uint32_t nt = p.n - tok0 < tok_per_cta ? p.n - tok0 : tok_per_cta;
+  const uint32_t nq = p.q_in ? p.Hq : 0u, slots = nq + 2u * p.Hkv, n_vec = nt * slots;
+  const uint32_t rot_chunks = rp.rot_half / 8u, off_chunks = rp.pair_off / 8u;
+
+  // chunk of this lane in slot j, the chunk of its rotation partner (itself when not rotated), its first pair index
+  uint32_t chunk[NS], partner[NS], pair0[NS];
+  bool rot[NS], low[NS];
+#pragma unroll
+  for (uint32_t j = 0; j < NS; ++j) {
+    const uint32_t c = lane + 32u * j;
+    chunk[j] = c;
+    low[j] = c < rot_chunks;
+    rot[j] = low[j] || (c >= off_chunks && c < off_chunks + rot_chunks);
+    partner[j] = !rot[j] ? c : low[j] ? c + off_chunks : c - off_chunks;
+    pair0[j] = (low[j] ? c : c - off_chunks) * 8u;
+  }
+  uint4 x[U][NS], xp[U][NS];
+  auto load = [&](uint32_t v0) {
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint32_t v = v0 + u * n_warps;
+      if (v >= n_vec) break;
+      const uint32_t tok = tok0 + v / slots, slot = v % slots;
+      const bool is_q = slot < nq, is_k = !is_q && slot < nq + p.Hkv;
+      const uint32_t H = is_q ? p.Hq : p.Hkv, h = is_q ? slot : (slot - nq) % p.Hkv;
+      const uint4* src = reinterpret_cast<const uint4*>((is_q ? p.q_in : is_k ? p.k_in : p.v_in) + (size_t(tok) * H + h) * D);
+#pragma unroll
+      for (uint32_t j = 0; j < NS; ++j) {
+        x[u][j] = src[chunk[j]];
+        if ((is_q || is_k) && rot[j]) xp[u][j] = src[partner[j]];
+      }
+    }
+  };
+  load(warp);
+  // (cos, sin) of the tokens' positions, while the first vectors are on their way
+  for (uint32_t e = threadIdx.x; e < nt * rp.rot_half; e += blockDim.x) {
+    const uint32_t t = e / rp.rot_half, i = e - t * rp.rot_half;
+    const float a = float(p.pos0 + tok0 + t) * rp.inv_freq[i];
+    const float2 v = make_float2(cosf(a), sinf(a));
+    cs[t * rp.rot_half + i] = v;
+    if (p.rope_table) p.rope_table[size_t(tok0 + t) * rp.rot_half + i] = v;
+  }
+  __syncthreads();
+  auto lo16 = [](uint32_t w) { return __uint_as_float(w << 16); };
+  auto hi16 = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
+  for (uint32_t v0 = warp; v0 < n_vec; v0 += U * n_warps) {
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint32_t v = v0 + u * n_warps;
+      if (v >= n_vec) break;                              // warp-uniform
+      const uint32_t t = v / slots, tok = tok0 + t, slot = v % slots, pos = p.pos0 + tok;
+      const bool is_q = slot < nq, is_k = !is_q && slot < nq + p.Hkv;
+      const uint32_t H = is_q ? p.Hq : p.Hkv, h = is_q ? slot : (slot - nq) % p.Hkv;
+      uint4 y[NS];
+      if (is_q || is_k || p.v_norm) {
+        float ss = 0.f;
+#pragma unroll
+        for (uint32_t j = 0; j < NS; ++j) {
+          const uint32_t w[4] = {x[u][j].x, x[u][j].y, x[u][j].z, x[u][j].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            ss = __fmaf_rn(lo16(w[e]), lo16(w[e]), ss);
+            ss = __fmaf_rn(hi16(w[e]), hi16(w[e]), ss);
+          }
+        }
+        ss = warp_sum(ss);
+        const float inv = 1.0f / sqrtf(ss / float(D) + p.eps);
+        const __nv_bfloat16* wt = is_q ? p.qw : is_k ? p.kw : nullptr;
+        const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+#pragma unroll
+        for (uint32_t j = 0; j < NS; ++j) {
+          const uint32_t m[4] = {x[u][j].x, x[u][j].y, x[u][j].z, x[u][j].w};
+          const uint4 w4 = wt ? reinterpret_cast<const uint4*>(wt)[chunk[j]] : ones;
+          const uint32_t wm[4] = {w4.x, w4.y, w4.z, w4.w};
+          float r[8];
+          if ((is_q || is_k) && rot[j]) {
+            const uint32_t q[4] = {xp[u][j].x, xp[u][j].y, xp[u][j].z, xp[u][j].w};
+            const uint4 p4 = wt ? reinterpret_cast<const uint4*>(wt)[partner[j]] : ones;
+            const uint32_t wq[4] = {p4.x, p4.y, p4.z, p4.w};
+            const float4* tab = reinterpret_cast<const float4*>(cs + t * rp.rot_half + pair0[j]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float4 c2 = tab[e];
+#pragma unroll
+              for (int o = 0; o < 2; ++o) {
+                const float c = o ? c2.z : c2.x, s = o ? c2.w : c2.y;
+                const float xm = o ? hi16(m[e]) : lo16(m[e]), xq = o ? hi16(q[e]) : lo16(q[e]);
+                const float wo = o ? hi16(wm[e]) : lo16(wm[e]), wp = o ? hi16(wq[e]) : lo16(wq[e]);
+                if (is_k) {
+                  r[2 * e + o] = rope_norm_rotate(xm, xq, rope_coef_a(wo, c), rope_coef_b(wp, s, low[j]), inv);
+                } else {
+                  const float a = __fmul_rn(xm, __fmul_rn(inv, wo)), b = __fmul_rn(xq, __fmul_rn(inv, wp));
+                  r[2 * e + o] = low[j] ? rope_rotate_lo(a, b, c, s) : rope_rotate_hi(b, a, c, s);
+                }
+              }
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              r[2 * e] = __fmul_rn(lo16(m[e]), __fmul_rn(inv, lo16(wm[e])));
+              r[2 * e + 1] = __fmul_rn(hi16(m[e]), __fmul_rn(inv, hi16(wm[e])));
+            }
+          }
+          __nv_bfloat162 b[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) b[e] = __floats2bfloat162_rn(r[2 * e], r[2 * e + 1]);
+          y[j] = make_uint4(*reinterpret_cast<uint32_t*>(&b[0]), *reinterpret_cast<uint32_t*>(&b[1]),
+                            *reinterpret_cast<uint32_t*>(&b[2]), *reinterpret_cast<uint32_t*>(&b[3]));
+        }
+      } else {
+#pragma unroll
+        for (uint32_t j = 0; j < NS; ++j) y[j] = x[u][j];
+      }
+      __nv_bfloat16* wb = is_q ? p.q_out : is_k ? p.k_out : p.v_out;
+      const bool stored = !is_q && pos < p.write_end && pos >= p.pos_base;
+      __nv_bfloat16* cache = (is_k ? p.cache_k : p.cache_v) + (size_t(h) * p.cap + ((pos - p.pos_base) & p.ring_mask)) * D;
+      __syncwarp();   // the output may be the input: every lane has read its partner's chunk
+#pragma unroll
+      for (uint32_t j = 0; j < NS; ++j) {
+        if (wb) reinterpret_cast<uint4*>(wb + (size_t(tok) * H + h) * D)[chunk[j]] = y[j];
+        if (stored) reinterpret_cast<uint4*>(cache)[chunk[j]] = y[j];
+      }
+    }
+    if (v0 + U * n_warps < n_vec) load(v0 + U * n_warps);
+  }
+}
+
+static bool append_rows_ok(const AppendParams& p, const RopeParams& rp) {
+  if ((p.D != 256 && p.D != 512) || rp.rot_half % 8 != 0 || rp.pair_off % 8 != 0) return false;
+  const void* ptrs[] = {p.q_in, p.q_out, p.k_in, p.k_out, p.v_in, p.v_out, p.qw, p.kw};
+  for (const void* q : ptrs)
+    if (reinterpret_cast<uintptr_t>(q) & 15u) return false;   // the general kernel reads element by element
+  return true;
+}
+
 void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st, bool early) {
   if (p.n == 0) return;
   // `early`: the kernel may be scheduled while its predecessor on the stream is still draining (it
@@ -160,10 +314,67 @@ void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st,
     cudaLaunchKernelEx(&cfg, dg_append_table_kernel, p);
     return;
   }
+  if (append_rows_ok(p, rp)) {
+    // as many tokens per CTA as give its warps about two vectors each: one where Q or many KV heads come along
+    const uint32_t slots = (p.q_in ? p.Hq : 0u) + 2u * p.Hkv;
+    const uint32_t tok = slots >= 16u ? 1u : (16u / slots < kRowsMaxTok ? 16u / slots : kRowsMaxTok);
+    const uint32_t warps = (tok * slots + kRowsUnit - 1u) / kRowsUnit;
+    cfg.gridDim = dim3((p.n + tok - 1u) / tok);
+    cfg.blockDim = dim3(32u * (warps < kRowsMaxWarps ? warps : kRowsMaxWarps));
+    if (p.D == 256) cudaLaunchKernelEx(&cfg, dg_append_rows_kernel<1>, p, rp, tok);
+    else cudaLaunchKernelEx(&cfg, dg_append_rows_kernel<2>, p, rp, tok);
+    return;
+  }
   const uint32_t slots = (p.q_in ? p.Hq : 0u) + 2u * p.Hkv + (p.rope_table ? 1u : 0u);
   cfg.gridDim = dim3(p.n, slots);
   cfg.blockDim = dim3(32);
   cudaLaunchKernelEx(&cfg, dg_append_kernel, p, rp);
+}
+
+// ------------------------------------------------------------------------------------------
+// Saved sessions: rows of a token-major [n][Hkv][D] tensor to or from the head-major cache, K and V in one launch
+// (blockIdx.y), 16 bytes per access, four in flight per thread.  Bound: memory.  8,192 tokens of 2 x 512 loaded, 2,000
+// appended and all read back: 131.3 us with a strided copy per head, tensor and direction, 45.7 us with this and
+// dg_append_rows_kernel (84 MB, 12.8 us at copy bandwidth; the rest is launches and the wait of the read).
+// ------------------------------------------------------------------------------------------
+constexpr uint32_t kCopyChunks = 4;
+
+__global__ void __launch_bounds__(256) dg_kv_copy_kernel(const KvCopyParams p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // see dg_append_kernel
+  uint4* flat = reinterpret_cast<uint4*>(blockIdx.y ? p.v : p.k);
+  uint4* cache = reinterpret_cast<uint4*>(blockIdx.y ? p.cache_v : p.cache_k);
+  const uint32_t first = blockIdx.x * (256u * kCopyChunks) + threadIdx.x;
+  uint4 x[kCopyChunks];
+  uint4* slot[kCopyChunks];
+#pragma unroll
+  for (uint32_t j = 0; j < kCopyChunks; ++j) {
+    const uint32_t e = first + j * 256u;                   // chunk of the token-major tensor
+    if (e >= p.n_chunks) break;
+    const uint32_t row = e / p.row_chunks, c = e - row * p.row_chunks, tok = row / p.Hkv, h = row - tok * p.Hkv;
+    slot[j] = cache + (size_t(h) * p.cap + ((p.slot0 + tok) & p.ring_mask)) * p.row_chunks + c;
+    x[j] = p.to_cache ? flat[e] : *slot[j];
+  }
+#pragma unroll
+  for (uint32_t j = 0; j < kCopyChunks; ++j) {
+    const uint32_t e = first + j * 256u;
+    if (e >= p.n_chunks) break;
+    if (p.to_cache) *slot[j] = x[j];
+    else flat[e] = x[j];
+  }
+}
+
+cudaError_t launch_kv_copy(const KvCopyParams& p, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((p.n_chunks + 256u * kCopyChunks - 1u) / (256u * kCopyChunks), 2);
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, dg_kv_copy_kernel, p);
 }
 
 // ------------------------------------------------------------------------------------------
