@@ -73,8 +73,8 @@ struct dg_ctx {
   __nv_bfloat16* blk_v = nullptr;
   __nv_bfloat16* blk_o = nullptr;
   float* blk_part = nullptr;           // fp32 partial planes of the output projection, [4][rows][hidden]
-  uint16_t* topk_scores = nullptr;     // dg_attn_denoise_topk: bf16 score plane [Hkv][canvas * G][ld]
-  size_t topk_elems = 0;
+  void* topk_plane = nullptr;          // dg_attn_denoise_topk: fp32 scores of a pass and their group maxima
+  size_t topk_bytes = 0;
   uint4* bits = nullptr;               // dg_attn_denoise_bitmap: the packed bitmap [canvas][tiles] and its live-tile flags
   uint8_t* bits_live = nullptr;
   size_t bits_tiles = 0;               // capacity in 128-key tiles, for kMaxCanvas rows
@@ -344,6 +344,7 @@ extern "C" int32_t dg_ctx_create(int32_t device, dg_ctx** out) {
   if (e == cudaSuccess) e = sm100_hd512x_configure();
   if (e == cudaSuccess) e = sm100_hd512q_configure();
   if (e == cudaSuccess) e = sm100_gemm_configure();
+  if (e == cudaSuccess) e = sm100_topk_configure();
   if (e != cudaSuccess) {
     dg_ctx_destroy(c);
     return fail_cuda(e, "dg_ctx_create");
@@ -373,7 +374,7 @@ extern "C" int32_t dg_ctx_destroy(dg_ctx* c) {
   cudaFree(c->blk_v);
   cudaFree(c->blk_o);
   cudaFree(c->blk_part);
-  cudaFree(c->topk_scores);
+  cudaFree(c->topk_plane);
   cudaFree(c->bits);
   cudaFree(c->bits_live);
   for (cudaEvent_t e : c->ev) cudaEventDestroy(e);
@@ -2259,6 +2260,8 @@ extern "C" int32_t dg_attn_block(dg_ctx* c, const dg_layer_desc* d, const dg_blo
 // top-k sparse attention of the reference's full layers (src/shaders/attn/attention_topk/, enc.rs:2125-2135):
 // stage 1 -> score GEMM per KV head -> selection + gathered PV
 // ------------------------------------------------------------------------------------------
+constexpr size_t kTopkPlaneBytes = size_t(288) << 20;
+
 extern "C" int32_t dg_attn_denoise_topk(dg_ctx* c, const dg_layer_desc* d, dg_kv* kv, uint32_t kv_len, const void* q,
                                         const void* k, const void* v, const void* qw, const void* kw, const dg_topk_cfg* cfg,
                                         void* out) {
@@ -2281,57 +2284,47 @@ extern "C" int32_t dg_attn_denoise_topk(dg_ctx* c, const dg_layer_desc* d, dg_kv
   const size_t qe = size_t(C) * d->n_q_heads * D;
   r = ensure_stage(c, qe, 0);
   if (r != DG_OK) return r;
-  // the score plane: keys padded to whole tiles of the score GEMM (128 keys at head_dim 256, 64 at 512)
-  const uint32_t bn = D == 256 ? 128u : 64u;
-  const uint32_t T = kv_len + C, ld = (T + bn - 1) / bn * bn;
-  const size_t rows = size_t(C) * G, need = size_t(d->n_kv_heads) * ((rows + 127) / 128 * 128) * ld;
-  if (need > c->topk_elems) {
+  // The score plane is fp32 and covers whole row pairs (256 stacked rows) and key tiles (256 keys).  It is kept to
+  // kTopkPlaneBytes where that leaves at least one row pair: the row pairs then go through it in several passes.
+  const uint32_t T = kv_len + C, n_groups = (T + 255u) / 256u * 16u;
+  const uint32_t rows = C * G, rp_per_head = (rows + 255u) / 256u, n_rp = rp_per_head * d->n_kv_heads;
+  const size_t rp_scores = size_t(n_groups) * 16 * 256, rp_gmax = size_t(n_groups) * 256;   // elements of one row pair
+  uint32_t per_pass = uint32_t(kTopkPlaneBytes / (rp_scores * 4));
+  per_pass = per_pass < 1 ? 1 : per_pass > n_rp ? n_rp : per_pass;
+  const uint32_t passes = (n_rp + per_pass - 1) / per_pass;
+  per_pass = (n_rp + passes - 1) / passes;
+  const size_t need = per_pass * (rp_scores * 4 + rp_gmax * 2);
+  if (need > c->topk_bytes) {
     DG_CUDA(cudaStreamSynchronize(c->stream));
-    cudaFree(c->topk_scores);
-    c->topk_scores = nullptr;
-    c->topk_elems = 0;
-    DG_CUDA(cudaMalloc(&c->topk_scores, need * 2));
-    c->topk_elems = need;
+    cudaFree(c->topk_plane);
+    c->topk_plane = nullptr;
+    c->topk_bytes = 0;
+    DG_CUDA(cudaMalloc(&c->topk_plane, need));
+    c->topk_bytes = need;
   }
   cudaStream_t st = launch_stream(c);
   // 1. stage 1: Q normed + roped into the staging tensor, canvas K/V into the cache
   r = do_append(c, *d, kv, kv_len, C, q, c->stage_q, k, nullptr, v, nullptr, qw, kw, nullptr);
   if (r != DG_OK) return r;
-  // 2. scores of every (row, key) of one KV head: rows (i, g) of the staged Q against the cache's K
+  // 2. scores of every (row, key) and their group maxima; 3. selection + softmax over the kept keys + gathered PV
   CUtensorMap tm_q;
   {
     PFN_encodeTiled enc = get_encode_fn();
     if (!enc) return fail(DG_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-    for (uint32_t h = 0; h < d->n_kv_heads; ++h) {
-      const cuuint64_t dims[3] = {D, G, C};
-      const cuuint64_t strides[2] = {cuuint64_t(D) * 2, cuuint64_t(d->n_q_heads) * D * 2};
-      const cuuint32_t box[3] = {64, G, 128 / G};
-      const cuuint32_t estr[3] = {1, 1, 1};
-      const CUresult cr = enc(&tm_q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, c->stage_q + size_t(h) * G * D, dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (cr != CUDA_SUCCESS) return fail(DG_ERR_CUDA, "cuTensorMapEncodeTiled failed for the staged Q");
-      GemmParams g = {};
-      g.M = uint32_t(rows);
-      g.N = ld;
-      g.K = D;
-      g.n_seg = 1;
-      g.seg[0] = GemmSeg{c->topk_scores + size_t(h) * ((rows + 127) / 128 * 128) * ld, 0u, ld};
-      g.a_inner = G;
-      g.w_z = h;
-      g.status = c->d_status;
-      const cudaError_t e = launch_gemm_sm100(g, tm_q, kv->tm_k, bn, st);
-      if (e != cudaSuccess) return fail_cuda(e, "launch_gemm_sm100 (scores)");
-      c->last_launches += 1;
-    }
+    const cuuint64_t dims[3] = {D, d->n_q_heads, C};
+    const cuuint64_t strides[2] = {cuuint64_t(D) * 2, cuuint64_t(d->n_q_heads) * D * 2};
+    const cuuint32_t box[3] = {64, G, 128 / G};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult cr = enc(&tm_q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, c->stage_q, dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) return fail(DG_ERR_CUDA, "cuTensorMapEncodeTiled failed for the staged Q");
   }
-  // 3. selection + softmax over the kept keys + gathered PV
   TopkParams tp = {};
-  tp.scores = c->topk_scores;
-  tp.ld = ld;
-  tp.head_rows = uint32_t((rows + 127) / 128 * 128);
-  tp.q = c->stage_q;
-  tp.k = kv->k;
+  tp.scores = static_cast<float*>(c->topk_plane);
+  tp.gmax = reinterpret_cast<uint16_t*>(tp.scores + size_t(per_pass) * rp_scores);
+  tp.n_groups = n_groups;
+  tp.rp_per_head = rp_per_head;
   tp.v = kv->v;
   tp.out = static_cast<__nv_bfloat16*>(out);
   tp.C = C;
@@ -2345,8 +2338,15 @@ extern "C" int32_t dg_attn_denoise_topk(dg_ctx* c, const dg_layer_desc* d, dg_kv
   tp.k_min = cfg->k_min;
   tp.k_max = cfg->k_max;
   tp.scale_log2 = d->softmax_scale * 1.4426950408889634f;
-  const cudaError_t e = launch_topk_select_pv(tp, st);
-  if (e != cudaSuccess) return fail_cuda(e, "launch_topk_select_pv");
-  c->last_launches += 1;
+  tp.status = c->d_status;
+  for (uint32_t rp = 0; rp < n_rp; rp += per_pass) {
+    tp.rp0 = rp;
+    tp.rp1 = rp + per_pass < n_rp ? rp + per_pass : n_rp;
+    cudaError_t e = launch_topk_scores(tp, tm_q, kv->tm_k, c->num_sms, st);
+    if (e != cudaSuccess) return fail_cuda(e, "launch_topk_scores");
+    e = launch_topk_select_pv(tp, st);
+    if (e != cudaSuccess) return fail_cuda(e, "launch_topk_select_pv");
+    c->last_launches += 2;
+  }
   return DG_OK;
 }

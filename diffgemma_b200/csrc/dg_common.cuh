@@ -110,7 +110,7 @@ __device__ inline void dev_status_set(DevStatus* s, uint32_t code, uint32_t kern
   }
 }
 
-enum : uint32_t { KID_APPEND = 1, KID_GENERAL = 2, KID_SM100 = 3, KID_MERGE = 4, KID_VIS = 5, KID_SELFTEST = 6, KID_GEMM = 7 };
+enum : uint32_t { KID_APPEND = 1, KID_GENERAL = 2, KID_SM100 = 3, KID_MERGE = 4, KID_VIS = 5, KID_SELFTEST = 6, KID_GEMM = 7, KID_SCORES = 8 };
 
 // ----------------------------------------------------------------------------------------
 // Launch parameter blocks
@@ -256,25 +256,34 @@ struct GemmParams {
   float* rowsq;        // optional [M][N / tile width]: sum of squares of each row's rounded outputs per tile
   float* part;         // split-K: fp32 partial sums [k_slices][M][N] instead of the bf16 output
   uint32_t k_slices;
-  uint32_t a_inner;    // 0: A is a {K, M} map.  G > 0: A is a {K, G, M / G} map (rows (i, g) of one KV head of a
-                       // [C][Hq][D] tensor) with boxes {64, G, 128 / G}
-  uint32_t w_z;        // third coordinate of the W map (the KV head of a cache map), else 0
   DevStatus* status;
 };
 
-// top-k selection + gathered PV over a plane of 16-bit scores (csrc/dg_topk.cu)
+// Order-preserving key of an fp32 score: larger key = larger score; the two zeros are equal (a tie goes by index), NaN
+// sorts above +inf.
+__device__ __forceinline__ uint32_t score_order_key(float x) {
+  const uint32_t u = __float_as_uint(x + 0.0f);
+  return u ^ (uint32_t(int32_t(u) >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float score_from_key(uint32_t k) {
+  return __uint_as_float(k ^ ((k & 0x80000000u) ? 0x80000000u : 0xffffffffu));
+}
+
+// top-k attention: score plane (csrc/dg_topk_scores.cu), selection + gathered PV (csrc/dg_topk.cu).  A launch covers the
+// row pairs [rp0, rp1): row pair rp = 256 GQA-stacked rows (i, g) of KV head rp / rp_per_head.
 struct TopkParams {
-  const uint16_t* scores;        // bf16 [Hkv][head_rows][ld]: row i * G + g of KV head h, key t
-  uint32_t ld, head_rows;        // head_rows = C * G rounded up to whole 128-row tiles
-  const __nv_bfloat16* q;        // normed + roped Q [C][Hq][D]
-  const __nv_bfloat16* k;        // caches [Hkv][cap][D]
-  const __nv_bfloat16* v;
+  float* scores;                 // [row pair][8][n_groups][2][32][8]: 32-row block, group of 16 keys, its halves, row, key
+  uint16_t* gmax;                // [row pair][256][n_groups]: the larger half of the order key of each group's maximum
+  uint32_t n_groups;             // groups of 16 keys: whole tiles of 256 keys
+  uint32_t rp0, rp1, rp_per_head;
+  const __nv_bfloat16* v;        // cache [Hkv][cap][D]
   __nv_bfloat16* out;            // [C][Hq][D]
   uint32_t C, Hq, G, D;
   uint64_t cap;
   MaskParams mask;
   uint32_t k_fixed, k_div, k_min, k_max;   // k = k_div ? clamp(n_visible / k_div, k_min, k_max) : k_fixed, at most n_visible
   float scale_log2;
+  DevStatus* status;
 };
 
 }  // namespace dg

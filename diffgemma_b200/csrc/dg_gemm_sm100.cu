@@ -27,9 +27,8 @@ namespace gm {
 constexpr uint32_t GM = 128, BK = 64;   // rows of a tile, contraction elements per stage
 constexpr uint32_t THREADS = 192;
 constexpr uint32_t A_STAGE = GM * BK * 2;   // 16 KB
-// stages of the ring: deep for the projections (44-128 contraction blocks per CTA); two for the score GEMM of the
-// top-k path, whose contraction is four or eight blocks, so that three CTAs share an SM and one's epilogue overlaps
-// another's loads
+// stages of the ring: deep for the projections (44-128 contraction blocks per CTA); two where the contraction is at most
+// eight blocks, so that three CTAs share an SM and one's epilogue overlaps another's loads
 __host__ __device__ constexpr uint32_t stages(uint32_t bn, bool shallow) { return shallow ? 2u : bn >= 128 ? 6u : 8u; }
 __host__ __device__ constexpr uint32_t smem_bytes(uint32_t bn, bool shallow) {
   return stages(bn, shallow) * (A_STAGE + bn * BK * 2) + 256 + 1024;
@@ -110,15 +109,13 @@ dg_gemm_sm100_kernel(const GemmParams g, const __grid_constant__ CUtensorMap tm_
           if (is_leader) mbar_expect_tx(bar_addr(bar_base, B_FULL + s), 2 * STAGE);
           const uint32_t full = lead_bar(B_FULL + s);
           tma_load_3d_pair(smem_base + s * STAGE, &tm_a, full, int32_t((kb0 + kb) * BK), int32_t(m0), 0);
-          tma_load_3d_pair(smem_base + s * STAGE + A_STAGE, &tm_w, full, int32_t((kb0 + kb) * BK), int32_t(n0 + xi * (BN / 2)),
-                           int32_t(g.w_z));
+          tma_load_3d_pair(smem_base + s * STAGE + A_STAGE, &tm_w, full, int32_t((kb0 + kb) * BK), int32_t(n0 + xi * (BN / 2)), 0);
           continue;
         }
         const uint32_t full = bar_addr(bar_base, B_FULL + s);
         mbar_expect_tx(full, STAGE);
-        if (g.a_inner == 0u) tma_load_3d(smem_base + s * STAGE, &tm_a, full, int32_t((kb0 + kb) * BK), int32_t(m0), 0);
-        else tma_load_3d(smem_base + s * STAGE, &tm_a, full, int32_t((kb0 + kb) * BK), 0, int32_t(m0 / g.a_inner));
-        tma_load_3d(smem_base + s * STAGE + A_STAGE, &tm_w, full, int32_t((kb0 + kb) * BK), int32_t(n0), int32_t(g.w_z));
+        tma_load_3d(smem_base + s * STAGE, &tm_a, full, int32_t((kb0 + kb) * BK), int32_t(m0), 0);
+        tma_load_3d(smem_base + s * STAGE + A_STAGE, &tm_w, full, int32_t((kb0 + kb) * BK), int32_t(n0), 0);
       }
     }
   } else if (warp == 1) {

@@ -66,7 +66,10 @@ uint32_t sm100_key_tiles(const MaskParams& mk);                     // upper bou
 cudaError_t sm100_gemm_configure();
 cudaError_t launch_gemm_sm100(const GemmParams& g, const CUtensorMap& tm_a, const CUtensorMap& tm_w, uint32_t bn,
                               cudaStream_t st);
-// top-k selection + gathered PV (csrc/dg_topk.cu)
+// top-k attention: fp32 scores with their group maxima (csrc/dg_topk_scores.cu; tm_q a {D, Hq, C} map of the normed Q with
+// boxes {64, G, 128 / G}, tm_k the cache's map), then selection + gathered PV (csrc/dg_topk.cu), for row pairs [rp0, rp1)
+cudaError_t sm100_topk_configure();
+cudaError_t launch_topk_scores(const TopkParams& p, const CUtensorMap& tm_q, const CUtensorMap& tm_k, int num_sms, cudaStream_t st);
 cudaError_t launch_topk_select_pv(const TopkParams& p, cudaStream_t st);
 cudaError_t launch_gemm_sm100_pair(const GemmParams& g, const CUtensorMap& tm_a, const CUtensorMap& tm_w, cudaStream_t st);
 cudaError_t launch_rmsnorm_rows(const void* x, const void* w, void* y, uint32_t rows, uint32_t dim, cudaStream_t st);

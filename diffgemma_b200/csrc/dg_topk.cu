@@ -2,15 +2,20 @@
 // oracle src/shaders/attn/attention_topk/cpu.rs:39-120), the selection and gathered-PV half.
 //
 // Per (canvas row, query head): only the k highest-scoring visible keys are kept (ties: lower index first), the
-// softmax is renormalised over them and O = sum_j p_j V[idx_j].  The scores of all keys come from a tensor-core GEMM
-// (dg_gemm_sm100_kernel: S[h][row][T] = Qn . K^T as bf16); this kernel
-//   1. finds the k-th largest 16-bit score with two 256-bin radix histograms (the reference's two levels on its u16
-//      key plane, attention_topk.metal:186-262), reading the row of the plane from L2;
-//   2. keeps every key above that value and, of the keys that share it, the best by EXACT fp32 score (recomputed
-//      from Q and K; ties by index) - or, when more than CAND_CAP keys share it (degenerate inputs: identical
-//      scores), the lowest indices;
-//   3. recomputes the exact fp32 scores of the k winners, softmax, and gathers V.
-// One CTA of 256 threads per (row, head).
+// softmax is renormalised over them and O = sum_j p_j V[idx_j].  dg_topk_scores.cu has written the fp32 scores of all
+// keys (masked ones as -inf) and, per group of 16 consecutive keys, the larger half of the order key of its maximum.
+// This kernel, one CTA of 256 threads per (row, head),
+//   1. finds the k-th largest of the group maxima, to 16 bits, rounded down: at least k keys reach that bound, and every
+//      key that does lies in a group whose maximum does.  On scores without structure about 1.03 k groups with
+//      1.07 k such keys are left of T / 16 groups (k = T / 128);
+//   2. reads those groups only, one in eight, and lists the keys at or above the bound in index order;
+//   3. finds the k-th largest of them exactly (radix over the 32-bit order keys) and keeps what lies above it and the
+//      lowest indices among what equals it;
+//   4. softmax over the kept scores, and the gather of V, a warp per kept key.
+// Lists that outgrow shared memory (many equal scores, clustered ones) take the same steps over the groups in memory.
+// Bound: the gather (4,096 rows x 258 keys x 1 KB = 1.08 GB out of L2 at head_dim 512): 180 us of 372 for the whole call at
+// 33,024 keys.  With bf16 scores, two histograms over all of a row and the exact scores of the kept keys computed again
+// from K (another 1.08 GB gathered) the call took 900 us.
 #include <cuda.h>
 
 #include "dg_common.cuh"
@@ -20,101 +25,81 @@
 namespace dg {
 
 namespace tk {
-constexpr uint32_t THREADS = 256;
+constexpr uint32_t THREADS = 256, WARPS = THREADS / 32;
 constexpr uint32_t K_CAP = 1024;      // most keys kept per row (the reference's largest slot capacity)
-constexpr uint32_t CAND_CAP = 1024;   // keys sharing the threshold value that are still ranked by exact score
+constexpr uint32_t G_CAP = 2048;      // groups listed in shared memory
+constexpr uint32_t C_CAP = 256;       // keys listed per warp
 }  // namespace tk
 
-// larger key = larger bf16 value; -0 and +0 differ, NaN sorts above +inf and is never produced by finite inputs
-__device__ __forceinline__ uint32_t bf16_order_key(uint16_t b) {
-  return (b & 0x8000u) ? (~uint32_t(b) & 0xffffu) : (uint32_t(b) | 0x8000u);
-}
-
-__device__ __forceinline__ float dot_row_bf16(const __nv_bfloat16* a, const __nv_bfloat16* b, uint32_t D, uint32_t lane) {
-  // one warp, 16-byte loads; D is a multiple of 256 or the tail is handled by the stride loop
-  float acc = 0.f;
-  for (uint32_t c = lane; c < D / 8; c += 32) {
-    const uint4 x = reinterpret_cast<const uint4*>(a)[c], y = reinterpret_cast<const uint4*>(b)[c];
-    const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+// Shared state of the radix steps: bin counts, per-warp sums, and the outcome {bin, keys above it, keys in it}.
+struct TopkRadix {
+  uint32_t hist[256];
+  uint32_t wsum[tk::WARPS];
+  uint32_t out[3];
+};
+// The bin, from the top, in which the running count reaches `need` (1 <= need <= total).  All threads, after a barrier
+// that follows the counting; ends with a barrier.
+__device__ __forceinline__ void topk_find_bin(TopkRadix& r, uint32_t need) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, bin = 255u - threadIdx.x;
+  const uint32_t own = r.hist[bin];
+  uint32_t incl = own;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      acc = fmaf(__uint_as_float(xs[e] << 16), __uint_as_float(ys[e] << 16), acc);
-      acc = fmaf(__uint_as_float(xs[e] & 0xffff0000u), __uint_as_float(ys[e] & 0xffff0000u), acc);
-    }
+  for (uint32_t o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
   }
+  if (lane == 31) r.wsum[warp] = incl;
+  __syncthreads();
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  return acc;
+  for (uint32_t w = 0; w < tk::WARPS; ++w)
+    if (w < warp) incl += r.wsum[w];
+  // fewer than `need` in all (scores of -inf or NaN among the visible ones): the last bin, all of it
+  if (incl - own < need && (incl >= need || bin == 0u)) {
+    r.out[0] = bin;
+    r.out[1] = incl - own;
+    r.out[2] = own;
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ uint32_t warp_excl_sum(uint32_t v, uint32_t lane, uint32_t& total) {
+  uint32_t incl = v;
+#pragma unroll
+  for (uint32_t o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  total = __shfl_sync(0xffffffffu, incl, 31);
+  return incl - v;
 }
 
-__global__ void __launch_bounds__(tk::THREADS) dg_topk_select_pv_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(tk::THREADS, 4) dg_topk_select_pv_kernel(const TopkParams p) {
   using namespace tk;
-  __shared__ uint32_t hist[256];
-  __shared__ uint32_t whist[THREADS / 32][256];   // one histogram per warp, added up into hist
-  __shared__ float o_part[THREADS / 32][512];     // the warps' partial output rows
-  __shared__ uint32_t s_idx[K_CAP];      // winners
-  __shared__ float s_sc[K_CAP];          // their exact scores, then their probabilities
-  __shared__ uint32_t c_idx[CAND_CAP];   // keys that share the threshold value
-  __shared__ float c_sc[CAND_CAP];
-  __shared__ uint32_t sh[8];             // 0 winners, 1 candidates, 2 bin, 3 need, 4 above, 5 n_valid
-  __shared__ float red[8];
-  __shared__ uint32_t scan[THREADS];
+  __shared__ TopkRadix rad;
+  // listed groups, then the winners in index order with their scores (later probabilities)
+  __shared__ __align__(16) uint32_t lists[2 * K_CAP];
+  uint32_t* glist = lists;                                        // [G_CAP]
+  uint32_t* s_idx = lists;                                        // [K_CAP]
+  float* s_sc = reinterpret_cast<float*>(lists + K_CAP);          // [K_CAP]
+  static_assert(G_CAP <= 2 * K_CAP, "group list");
+  // listed keys and their positions per warp, then the warps' partial output rows
+  __shared__ __align__(16) uint32_t cands[2 * WARPS * C_CAP];
+  uint32_t(*c_key)[C_CAP] = reinterpret_cast<uint32_t(*)[C_CAP]>(cands);
+  uint32_t(*c_idx)[C_CAP] = reinterpret_cast<uint32_t(*)[C_CAP]>(cands + WARPS * C_CAP);
+  float(*s_part)[512] = reinterpret_cast<float(*)[512]>(cands);
+  static_assert(2 * C_CAP >= 512, "partial rows");
+  __shared__ uint32_t c_n[WARPS], w_cnt[WARPS], w_eq[WARPS];
+  __shared__ uint32_t sh_bulk;
+  __shared__ float red[WARPS];
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t i = blockIdx.x, h = blockIdx.y;           // canvas row, query head
-  const uint32_t kvh = h / p.G, g = h % p.G;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const uint16_t* srow = p.scores + (size_t(kvh) * p.head_rows + size_t(i) * p.G + g) * p.ld;
+  // blockIdx.x: row of the pass = (row pair, stacked row)
+  const uint32_t rp = p.rp0 + blockIdx.x / 256u, R = (rp % p.rp_per_head) * 256u + blockIdx.x % 256u;
+  if (R >= p.C * p.G) return;
+  const uint32_t kvh = rp / p.rp_per_head, i = R / p.G, h = kvh * p.G + R % p.G;
   const MaskParams mk = p.mask;
   const RowVis rv = mask_row(mk, i);
   const uint32_t T = mk.can_hi;
-  const bool all_vis = mask_range_full(mk, rv, 0u, T);       // every key below T is visible to this row
-  auto visible = [&](uint32_t t) { return all_vis || mask_visible_row(mk, rv, t); };
-  // every visible key of the row, eight per 16-byte load (the row of the plane starts on a 16-byte boundary and is
-  // padded to whole tiles), two loads in flight per thread: f(t, key)
-  const uint4* row4 = reinterpret_cast<const uint4*>(srow);
-  const uint32_t n8 = (T + 7u) / 8u;
-  auto for_keys = [&](auto f) {
-#pragma unroll 2
-    for (uint32_t c = tid; c < n8; c += THREADS) {
-      const uint4 x = row4[c];
-      const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
-      const uint32_t base = c * 8u;
-      const bool whole = all_vis && base + 8u <= T;      // no key of the chunk needs a bounds or mask test
-#pragma unroll
-      for (uint32_t w = 0; w < 4; ++w) {
-        // both order-preserving keys of the word at once: a negative value is complemented, a positive one gets
-        // its sign bit set
-        const uint32_t sg = (xs[w] >> 15) & 0x00010001u;
-        const uint32_t k2 = xs[w] ^ ((sg * 0xffffu) | 0x80008000u);
-        const uint32_t t = base + 2u * w;
-        if (whole || (t < T && visible(t))) f(t, k2 & 0xffffu);
-        if (whole || (t + 1u < T && visible(t + 1u))) f(t + 1u, k2 >> 16);
-      }
-    }
-  };
-  auto zero_whist = [&]() {
-    for (uint32_t b = tid; b < (THREADS / 32) * 256; b += THREADS) (&whist[0][0])[b] = 0u;
-  };
-  auto fold_whist = [&]() {
-    for (uint32_t b = tid; b < 256; b += THREADS) {
-      uint32_t c = 0;
-#pragma unroll
-      for (uint32_t w = 0; w < THREADS / 32; ++w) c += whist[w][b];
-      hist[b] = c;
-    }
-  };
-
-  // ---- visible keys and k
-  uint32_t nv = 0;
-  if (!all_vis)
-    for (uint32_t t = tid; t < T; t += THREADS) nv += visible(t) ? 1u : 0u;
-  if (tid < 8) sh[tid] = 0u;
-  zero_whist();
-  __syncthreads();
-  if (!all_vis) atomicAdd(&sh[5], nv);
-  __syncthreads();
-  const uint32_t n_valid = all_vis ? T : sh[5];
+  const uint32_t n_valid = (mk.pre_hi > rv.lo ? mk.pre_hi - rv.lo : 0u) + (rv.can_hi > rv.can_lo ? rv.can_hi - rv.can_lo : 0u);
   uint32_t k_req = p.k_fixed;
   if (p.k_div != 0u) {
     k_req = n_valid / p.k_div;
@@ -123,146 +108,259 @@ __global__ void __launch_bounds__(tk::THREADS) dg_topk_select_pv_kernel(const To
   }
   uint32_t k = k_req < n_valid ? k_req : n_valid;
   if (k > K_CAP) k = K_CAP;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __nv_bfloat16* orow = p.out + (size_t(i) * p.Hq + h) * p.D;
   if (k == 0u) {
     for (uint32_t d = tid; d < p.D; d += THREADS) orow[d] = __float2bfloat16(0.f);
     return;
   }
+  const uint32_t n_groups = p.n_groups;
+  const uint4* gmax = reinterpret_cast<const uint4*>(p.gmax + size_t(blockIdx.x) * n_groups);       // eight groups per load
+  // 16 keys of group g of this row: float4 (g * 128 + (q >> 1) * 64 + (q & 1)), q = 0..3
+  const uint4* row = reinterpret_cast<const uint4*>(p.scores) + (size_t(blockIdx.x / 32u) * n_groups * 512u + (blockIdx.x % 32u) * 8u) / 4u;
+  auto quad = [&](uint32_t g, uint32_t q) { return row[size_t(g) * 128u + (q >> 1) * 64u + (q & 1u)]; };
+  auto okey = [](uint32_t bits) { return score_order_key(__uint_as_float(bits)); };
+  const uint32_t n_g8 = n_groups / 8u;
 
-  // ---- level 1: top byte of the key
-  // (one histogram per warp: scores cluster on a few exponent values, a single one would serialise on a few bins)
-  for_keys([&](uint32_t, uint32_t key) { atomicAdd(&whist[warp][key >> 8], 1u); });
-  __syncthreads();
-  fold_whist();
-  __syncthreads();
-  if (tid == 0) {
-    uint32_t cum = 0, b1 = 0;
-    for (int b = 255; b >= 0; --b) {
-      if (cum + hist[b] >= k) {
-        b1 = uint32_t(b);
-        break;
+  // ---- 1. bound: the k-th largest group maximum (16 bits of it)
+  uint32_t bound16 = 0u;
+  if (n_groups > k) {
+    uint32_t need = k;
+#pragma unroll 1
+    for (uint32_t level = 0; level < 2; ++level) {
+      rad.hist[tid] = 0u;
+      __syncthreads();
+      for (uint32_t c = tid; c < n_g8; c += THREADS) {
+        const uint4 x = gmax[c];
+        const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (uint32_t w = 0; w < 4; ++w)
+#pragma unroll
+          for (uint32_t o = 0; o < 2; ++o) {
+            const uint32_t key = (xs[w] >> (16 * o)) & 0xffffu;
+            if (level == 0) atomicAdd(&rad.hist[key >> 8], 1u);
+            else if ((key >> 8) == bound16) atomicAdd(&rad.hist[key & 0xffu], 1u);
+          }
       }
-      cum += hist[b];
+      __syncthreads();
+      topk_find_bin(rad, need);
+      need -= rad.out[1];
+      bound16 = (bound16 << 8) | rad.out[0];
+      __syncthreads();
     }
-    sh[2] = b1;
-    sh[4] = cum;          // keys whose top byte is larger
   }
-  __syncthreads();
-  const uint32_t bin1 = sh[2];
-  uint32_t above = sh[4];
-  __syncthreads();
-  zero_whist();
-  __syncthreads();
-  // ---- level 2: low byte inside that bin
-  for_keys([&](uint32_t, uint32_t key) {
-    if ((key >> 8) == bin1) atomicAdd(&whist[warp][key & 0xffu], 1u);
-  });
-  __syncthreads();
-  fold_whist();
-  __syncthreads();
-  if (tid == 0) {
-    uint32_t cum = above, b2 = 0;
-    for (int b = 255; b >= 0; --b) {
-      if (cum + hist[b] >= k) {
-        b2 = uint32_t(b);
-        break;
-      }
-      cum += hist[b];
-    }
-    sh[2] = (bin1 << 8) | b2;     // the k-th largest 16-bit key
-    sh[4] = cum;                  // keys strictly above it: all kept
-    sh[3] = k - cum;              // still to take from the keys that share it
-    sh[1] = hist[b2];             // how many share it
-  }
-  __syncthreads();
-  const uint32_t thr = sh[2], need = sh[3], n_cand = sh[1];
-  above = sh[4];
-  const bool ranked = n_cand <= CAND_CAP;
-  __syncthreads();
-  if (tid == 0) sh[1] = 0u;
-  __syncthreads();
+  // masked keys are -inf (0x007f...): with fewer groups in sight than k the bound is what lies just above them
+  if (bound16 < 0x80u) bound16 = 0x80u;
 
-  // ---- emit the keys above the threshold; collect (or count) the ones that share it
-  uint32_t my_cand = 0;
-  const uint32_t per = (T + THREADS - 1) / THREADS;          // contiguous index ranges, for the index-ordered path
-  if (ranked) {
-    for_keys([&](uint32_t t, uint32_t key) {
-      if (key > thr) s_idx[atomicAdd(&sh[0], 1u)] = t;
-      else if (key == thr) c_idx[atomicAdd(&sh[1], 1u)] = t;
-    });
-  } else {
-    const uint32_t t_lo = tid * per, t_hi = (t_lo + per < T) ? t_lo + per : T;
-    for (uint32_t t = t_lo; t < t_hi; ++t) {
-      if (!visible(t)) continue;
-      const uint32_t key = bf16_order_key(srow[t]);
-      if (key > thr) s_idx[atomicAdd(&sh[0], 1u)] = t;
-      else if (key == thr) ++my_cand;
+  // ---- 2. groups that reach the bound, in index order: each warp looks through a contiguous run
+  const uint32_t per_w = (n_g8 + WARPS - 1u) / WARPS;
+  const uint32_t g8_lo = warp * per_w < n_g8 ? warp * per_w : n_g8, g8_hi = g8_lo + per_w < n_g8 ? g8_lo + per_w : n_g8;
+  auto reach = [&](const uint4 x) {      // bit e: group e of the eight reaches the bound
+    const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+    uint32_t m = 0u;
+#pragma unroll
+    for (uint32_t w = 0; w < 4; ++w) {
+      if ((xs[w] & 0xffffu) >= bound16) m |= 1u << (2 * w);
+      if ((xs[w] >> 16) >= bound16) m |= 2u << (2 * w);
     }
-  }
+    return m;
+  };
+  uint32_t mine = 0u;
+  for (uint32_t c = g8_lo + lane; c < g8_hi; c += 32u) mine += __popc(reach(gmax[c]));
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (lane == 0) w_cnt[warp] = mine;
+  if (tid == 0) sh_bulk = 0u;
   __syncthreads();
-  const __nv_bfloat16* qrow = p.q + (size_t(i) * p.Hq + h) * p.D;
-  const __nv_bfloat16* kbase = p.k + size_t(kvh) * p.cap * p.D;
-  const __nv_bfloat16* vbase = p.v + size_t(kvh) * p.cap * p.D;
-  if (ranked) {
-    // exact scores of the candidates; a candidate is kept when fewer than `need` others beat it (score, then index)
-    for (uint32_t c = warp; c < n_cand; c += THREADS / 32) {
-      const float s = dot_row_bf16(qrow, kbase + size_t(c_idx[c]) * p.D, p.D, lane);
-      if (lane == 0) c_sc[c] = s;
+  uint32_t g_off = 0u, n_list = 0u;
+#pragma unroll
+  for (uint32_t w = 0; w < WARPS; ++w) {
+    if (w < warp) g_off += w_cnt[w];
+    n_list += w_cnt[w];
+  }
+  if (n_list <= G_CAP) {
+    for (uint32_t c0 = g8_lo; c0 < g8_hi; c0 += 32u) {
+      const uint32_t c = c0 + lane;
+      uint32_t m = c < g8_hi ? reach(gmax[c]) : 0u, total;
+      uint32_t at = g_off + warp_excl_sum(__popc(m), lane, total);
+      for (; m != 0u; m &= m - 1u) glist[at++] = c * 8u + (__ffs(m) - 1u);
+      g_off += total;
     }
     __syncthreads();
-    for (uint32_t c = tid; c < n_cand; c += THREADS) {
-      const float s = c_sc[c];
-      const uint32_t t = c_idx[c];
-      uint32_t better = 0;
-      for (uint32_t o = 0; o < n_cand; ++o) {
-        const float so = c_sc[o];
-        better += (so > s || (so == s && c_idx[o] < t)) ? 1u : 0u;
-      }
-      if (better < need) s_idx[atomicAdd(&sh[0], 1u)] = t;
-    }
-  } else {
-    // identical scores in bulk: the lowest indices, by an exclusive scan over the threads' index ranges
-    scan[tid] = my_cand;
-    __syncthreads();
-    if (tid == 0) {
-      uint32_t run = 0;
-      for (uint32_t j = 0; j < THREADS; ++j) {
-        const uint32_t c = scan[j];
-        scan[j] = run;
-        run += c;
-      }
-    }
-    __syncthreads();
-    uint32_t before = scan[tid];
-    const uint32_t t_lo = tid * per, t_hi = (t_lo + per < T) ? t_lo + per : T;
-    for (uint32_t t = t_lo; t < t_hi && before < need; ++t) {
-      if (!visible(t)) continue;
-      if (bf16_order_key(srow[t]) == thr) {
-        s_idx[atomicAdd(&sh[0], 1u)] = t;
-        ++before;
-      }
-    }
-  }
-  __syncthreads();
-  // sh[0] == k now.  The winners were appended in the order the threads got to them: sort them by index, so that
-  // every sum below is taken in the same order in every run.
-  for (uint32_t j = tid; j < k; j += THREADS) {
-    const uint32_t t = s_idx[j];
-    uint32_t rank = 0;
-    for (uint32_t o = 0; o < k; ++o) rank += s_idx[o] < t ? 1u : 0u;
-    c_idx[rank] = t;
-  }
-  __syncthreads();
-  for (uint32_t j = tid; j < k; j += THREADS) s_idx[j] = c_idx[j];
-  __syncthreads();
-
-  // ---- exact scores of the winners, softmax over them
+    // ---- keys at or above the bound: four lanes per group, eight groups at a time, in index order
+    const uint32_t bound = bound16 << 16;
+    const uint32_t l_lo = n_list * warp / WARPS, l_hi = n_list * (warp + 1u) / WARPS;
+    uint32_t n = 0u;
 #pragma unroll 2
-  for (uint32_t j = warp; j < k; j += THREADS / 32) {
-    const float s = dot_row_bf16(qrow, kbase + size_t(s_idx[j]) * p.D, p.D, lane);
-    if (lane == 0) s_sc[j] = s * p.scale_log2;
+    for (uint32_t l0 = l_lo; l0 < l_hi; l0 += 8u) {
+      const uint32_t l = l0 + (lane >> 2), q = lane & 3u;
+      uint32_t t0 = 0u, m = 0u, key[4] = {0u, 0u, 0u, 0u};
+      if (l < l_hi) {
+        const uint32_t g = glist[l];
+        const uint4 x = quad(g, q);
+        const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+        t0 = g * 16u + q * 4u;
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+          key[e] = okey(xs[e]);
+          if (key[e] >= bound && t0 + e < T) m |= 1u << e;
+        }
+      }
+      uint32_t total;
+      uint32_t at = n + warp_excl_sum(__popc(m), lane, total);
+      n += total;
+      if (n > C_CAP) break;                  // warp-uniform
+#pragma unroll
+      for (uint32_t e = 0; e < 4; ++e)
+        if ((m >> e) & 1u) {
+          c_key[warp][at] = key[e];
+          c_idx[warp][at] = t0 + e;
+          ++at;
+        }
+    }
+    if (lane == 0) {
+      c_n[warp] = n;
+      if (n > C_CAP) sh_bulk = 1u;
+    }
+  } else if (tid == 0) {
+    sh_bulk = 1u;
   }
   __syncthreads();
+
+  // ---- 3. the k-th largest key, exactly, and the winners in index order
+  const bool bulk = sh_bulk != 0u;
+  uint32_t n_cand = 0u;
+  if (!bulk) {
+#pragma unroll
+    for (uint32_t w = 0; w < WARPS; ++w) n_cand += c_n[w];
+  }
+  // keys of the groups that reach the bound, straight from memory: f(t, order key); thread tid takes a contiguous run
+  const uint32_t per_t = (n_groups + THREADS - 1u) / THREADS;
+  const uint32_t gt_lo = tid * per_t < n_groups ? tid * per_t : n_groups, gt_hi = gt_lo + per_t < n_groups ? gt_lo + per_t : n_groups;
+  auto for_bulk = [&](auto f) {
+    const uint16_t* g16 = reinterpret_cast<const uint16_t*>(gmax);
+    for (uint32_t g = gt_lo; g < gt_hi; ++g) {
+      if (g16[g] < bound16) continue;
+      for (uint32_t q = 0; q < 4; ++q) {
+        const uint4 x = quad(g, q);
+        const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e)
+          if (g * 16u + q * 4u + e < T) f(g * 16u + q * 4u + e, okey(xs[e]));
+      }
+    }
+  };
+  auto for_listed = [&](auto f) {
+    for (uint32_t j = lane; j < c_n[warp]; j += 32u) f(c_idx[warp][j], c_key[warp][j]);
+  };
+  uint32_t thr = 0u, need = k;              // kept: keys above thr, and the first `need` of those equal to it
+  if (bulk || n_cand > k) {
+    uint32_t mask = 0u;
+#pragma unroll 1
+    for (int shift = 24; shift >= 0; shift -= 8) {
+      rad.hist[tid] = 0u;
+      __syncthreads();
+      auto count = [&](uint32_t, uint32_t key) {
+        if ((key & mask) == thr) atomicAdd(&rad.hist[(key >> shift) & 0xffu], 1u);
+      };
+      if (bulk) for_bulk(count);
+      else for_listed(count);
+      __syncthreads();
+      topk_find_bin(rad, need);
+      need -= rad.out[1];
+      thr |= rad.out[0] << shift;
+      mask |= 0xffu << shift;
+      const bool done = rad.out[2] == need;   // all of the bin is kept: nothing below matters
+      __syncthreads();
+      if (done) {
+        // every key with this prefix is kept: "above thr - 1"
+        need = 0u;
+        thr = thr != 0u ? thr - 1u : 0u;
+        break;
+      }
+    }
+  }
+  uint32_t n_kept;
+  if (!bulk) {
+    uint32_t gt = 0u, eq = 0u;
+    const uint32_t n = c_n[warp];
+    for (uint32_t j = lane; j < n; j += 32u) {
+      const uint32_t key = c_key[warp][j];
+      gt += key > thr ? 1u : 0u;
+      eq += key == thr ? 1u : 0u;
+    }
+    gt = __reduce_add_sync(0xffffffffu, gt);
+    eq = __reduce_add_sync(0xffffffffu, eq);
+    if (lane == 0) {
+      w_cnt[warp] = gt;
+      w_eq[warp] = eq;
+    }
+    __syncthreads();
+    uint32_t at = 0u, eq_before = 0u, all_gt = 0u, all_eq = 0u;
+#pragma unroll
+    for (uint32_t w = 0; w < WARPS; ++w) {
+      if (w < warp) {
+        at += w_cnt[w];
+        eq_before += w_eq[w];
+      }
+      all_gt += w_cnt[w];
+      all_eq += w_eq[w];
+    }
+    at += eq_before < need ? eq_before : need;
+    n_kept = all_gt + (all_eq < need ? all_eq : need);
+    for (uint32_t j0 = 0; j0 < n; j0 += 32u) {
+      const uint32_t j = j0 + lane;
+      const uint32_t key = j < n ? c_key[warp][j] : 0u;
+      const bool is_eq = j < n && key == thr;
+      const uint32_t eq_mask = __ballot_sync(0xffffffffu, is_eq), below = (1u << lane) - 1u;
+      const bool take = (j < n && key > thr) || (is_eq && eq_before + __popc(eq_mask & below) < need);
+      const uint32_t take_mask = __ballot_sync(0xffffffffu, take);
+      if (take) {
+        const uint32_t o = at + __popc(take_mask & below);
+        s_idx[o] = c_idx[warp][j];
+        s_sc[o] = score_from_key(key);
+      }
+      at += __popc(take_mask);
+      eq_before += __popc(eq_mask);
+    }
+  } else {
+    uint32_t gt = 0u, eq = 0u;
+    for_bulk([&](uint32_t, uint32_t key) {
+      gt += key > thr ? 1u : 0u;
+      eq += key == thr ? 1u : 0u;
+    });
+    uint32_t gt_w, eq_w;
+    const uint32_t gt_x = warp_excl_sum(gt, lane, gt_w), eq_x = warp_excl_sum(eq, lane, eq_w);
+    if (lane == 0) {
+      w_cnt[warp] = gt_w;
+      w_eq[warp] = eq_w;
+    }
+    __syncthreads();
+    uint32_t gt_before = gt_x, eq_before = eq_x, all_gt = 0u, all_eq = 0u;
+#pragma unroll
+    for (uint32_t w = 0; w < WARPS; ++w) {
+      if (w < warp) {
+        gt_before += w_cnt[w];
+        eq_before += w_eq[w];
+      }
+      all_gt += w_cnt[w];
+      all_eq += w_eq[w];
+    }
+    n_kept = all_gt + (all_eq < need ? all_eq : need);
+    uint32_t at = gt_before + (eq_before < need ? eq_before : need);
+    for_bulk([&](uint32_t t, uint32_t key) {
+      const bool take = key > thr || (key == thr && eq_before < need);
+      if (key == thr) ++eq_before;
+      if (take) {
+        s_idx[at] = t;
+        s_sc[at] = score_from_key(key);
+        ++at;
+      }
+    });
+  }
+  k = n_kept < k ? n_kept : k;
+  __syncthreads();
+
+  // ---- 4. softmax over the winners
   float mx = -INFINITY;
   for (uint32_t j = tid; j < k; j += THREADS) mx = fmaxf(mx, s_sc[j]);
 #pragma unroll
@@ -271,11 +369,12 @@ __global__ void __launch_bounds__(tk::THREADS) dg_topk_select_pv_kernel(const To
   __syncthreads();
   mx = red[0];
 #pragma unroll
-  for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red[w]);
+  for (uint32_t w = 1; w < WARPS; ++w) mx = fmaxf(mx, red[w]);
+  mx *= p.scale_log2;
   __syncthreads();
   float l = 0.f;
   for (uint32_t j = tid; j < k; j += THREADS) {
-    const float pj = fast_exp2(s_sc[j] - mx);
+    const float pj = fast_exp2(s_sc[j] * p.scale_log2 - mx);
     s_sc[j] = pj;
     l += pj;
   }
@@ -285,45 +384,53 @@ __global__ void __launch_bounds__(tk::THREADS) dg_topk_select_pv_kernel(const To
   __syncthreads();
   l = 0.f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) l += red[w];
+  for (uint32_t w = 0; w < WARPS; ++w) l += red[w];
   const float inv_l = l > 0.f ? 1.0f / l : 0.f;
 
   // ---- O = sum_j p_j V[idx_j]: a warp takes every eighth kept key, its lanes cover the value row with 16-byte
-  // loads (several rows in flight), and the eight partial rows meet in shared memory
-  __syncthreads();
+  // loads (several rows in flight), packed fp32 pairs, and the eight partial rows meet in shared memory
+  const __nv_bfloat16* vbase = p.v + size_t(kvh) * p.cap * p.D;
   const uint32_t n_chunk = p.D / 256;            // 16-byte chunks per lane: 1 at head_dim 256, 2 at 512
-  float acc[16];
+  uint64_t acc[8];
 #pragma unroll
-  for (int e = 0; e < 16; ++e) acc[e] = 0.f;
+  for (int e = 0; e < 8; ++e) acc[e] = 0ull;
+  auto add_row = [&](float pj, uint32_t c, const uint4 x) {
+    const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+    const uint64_t p2 = pack_f32x2(pj, pj);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[c * 4 + e] = fma_f32x2(p2, bf16x2_to_f32x2(xs[e]), acc[c * 4 + e]);
+  };
+  if (n_chunk == 2u) {
 #pragma unroll 4
-  for (uint32_t j = warp; j < k; j += THREADS / 32) {
-    const uint4* vr = reinterpret_cast<const uint4*>(vbase + size_t(s_idx[j]) * p.D);
-    const float pj = s_sc[j];
-#pragma unroll
-    for (uint32_t c = 0; c < 2; ++c) {
-      if (c >= n_chunk) break;
-      const uint4 x = vr[c * 32u + lane];
-      const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        acc[c * 8 + 2 * e] = fmaf(pj, __uint_as_float(xs[e] << 16), acc[c * 8 + 2 * e]);
-        acc[c * 8 + 2 * e + 1] = fmaf(pj, __uint_as_float(xs[e] & 0xffff0000u), acc[c * 8 + 2 * e + 1]);
-      }
+    for (uint32_t j = warp; j < k; j += WARPS) {
+      const uint4* vr = reinterpret_cast<const uint4*>(vbase + size_t(s_idx[j]) * 512u) + lane;
+      const uint4 a = vr[0], b = vr[32];
+      add_row(s_sc[j], 0, a);
+      add_row(s_sc[j], 1, b);
     }
+  } else {
+#pragma unroll 8
+    for (uint32_t j = warp; j < k; j += WARPS)
+      add_row(s_sc[j], 0, reinterpret_cast<const uint4*>(vbase + size_t(s_idx[j]) * 256u)[lane]);
   }
 #pragma unroll
   for (uint32_t c = 0; c < 2; ++c) {
     if (c >= n_chunk) break;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o_part[warp][(c * 32u + lane) * 8u + e] = acc[c * 8 + e];
+    for (int e = 0; e < 4; ++e) {
+      float a0, a1;
+      unpack_f32x2(acc[c * 4 + e], a0, a1);
+      s_part[warp][(c * 32u + lane) * 8u + 2 * e] = a0;
+      s_part[warp][(c * 32u + lane) * 8u + 2 * e + 1] = a1;
+    }
   }
   __syncthreads();
   for (uint32_t d2 = tid; d2 < p.D / 2; d2 += THREADS) {
     float a0 = 0.f, a1 = 0.f;
 #pragma unroll
-    for (uint32_t w = 0; w < THREADS / 32; ++w) {      // fixed order: same bits every run
-      a0 += o_part[w][2 * d2];
-      a1 += o_part[w][2 * d2 + 1];
+    for (uint32_t w = 0; w < WARPS; ++w) {      // fixed order: same bits every run
+      a0 += s_part[w][2 * d2];
+      a1 += s_part[w][2 * d2 + 1];
     }
     reinterpret_cast<uint32_t*>(orow)[d2] = pack_bf16x2(a0 * inv_l, a1 * inv_l);
   }
@@ -331,7 +438,7 @@ __global__ void __launch_bounds__(tk::THREADS) dg_topk_select_pv_kernel(const To
 
 cudaError_t launch_topk_select_pv(const TopkParams& p, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.C, p.Hq);
+  cfg.gridDim = dim3((p.rp1 - p.rp0) * 256u);
   cfg.blockDim = dim3(tk::THREADS);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
