@@ -2141,6 +2141,11 @@ static int32_t ensure_block_ws(dg_ctx* c, size_t rows, size_t hidden, size_t qe,
   DG_CUDA(cudaMalloc(&c->blk_part, kBlockMaxSlices * Rp * H * sizeof(float)));
   DG_CUDA(cudaMemset(c->blk_xn, 0, Rp * H * 2));
   DG_CUDA(cudaMemset(c->blk_o, 0, Rp * Q * 2));
+  // maps of the two activations the projections read, over whole 128-row tiles: made anew with every allocation (a
+  // buffer may come back at its old address while another one moved)
+  int32_t r = make_kv_tmap(&c->blk_tm_xn, c->blk_xn, Rp, 1, 128, uint32_t(H));
+  if (r == DG_OK) r = make_kv_tmap(&c->blk_tm_o, c->blk_o, Rp, 1, 128, uint32_t(Q));
+  if (r != DG_OK) return r;
   c->blk_rows = R;
   c->blk_hidden = H;
   c->blk_qe = Q;
@@ -2179,18 +2184,9 @@ extern "C" int32_t dg_attn_block(dg_ctx* c, const dg_layer_desc* d, const dg_blo
   if (H == 0 || H % 64 != 0 || H > 8192 || nq % 128 != 0 || nk % 128 != 0)
     return fail(DG_ERR_UNSUPPORTED, "dg_attn_block: hidden must be a multiple of 64 up to 8192, n_heads * head_dim a multiple of 128");
   DG_CUDA(cudaSetDevice(c->device));
-  const size_t old_rows = c->blk_rows, old_h = c->blk_hidden, old_q = c->blk_qe;
-  const __nv_bfloat16* old_xn = c->blk_xn;
   r = ensure_block_ws(c, C, H, nq, nk);
   if (r != DG_OK) return r;
-  if (c->blk_xn != old_xn || old_rows != c->blk_rows || old_h != c->blk_hidden || old_q != c->blk_qe || old_xn == nullptr) {
-    // maps of the two activations the projections read, over whole 128-row tiles
-    const size_t Rp = (c->blk_rows + 127) / 128 * 128;
-    r = make_kv_tmap(&c->blk_tm_xn, c->blk_xn, Rp, 1, 128, uint32_t(c->blk_hidden));
-    if (r == DG_OK) r = make_kv_tmap(&c->blk_tm_o, c->blk_o, Rp, 1, 128, uint32_t(c->blk_qe));
-    if (r != DG_OK) return r;
-  }
-  // the maps above span the buffers' full width: this call's width must be the buffers'
+  // the activations' maps span the buffers' full width: this call's width must be the buffers'
   if (H != c->blk_hidden || nq != c->blk_qe)
     return fail(DG_ERR_UNSUPPORTED, "dg_attn_block: one context serves one (hidden, n_q_heads * head_dim) geometry");
   const CUtensorMap *tm_wqkv = nullptr, *tm_wo = nullptr;
