@@ -231,115 +231,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   float m_used = -INFINITY, l_run = 0.f;
 
   if (warp < SM_WARPS) {
-    // ---------------------------------------------------------------- Q prologue (one warp per row)
-    // A warp takes eight rows of the tile; lane c owns the 16-byte chunk c of a row, so every global
-    // access is one contiguous 512-byte row.  The raw rows are copied asynchronously straight into
-    // their final (swizzled) place; each lane then reads back its own chunk and its RoPE partner,
-    // chunk c ^ 16, and overwrites its own chunk with
-    //     rsqrt(mean(x^2) + eps) * (x * (w cos) -/+ partner * (w_partner sin)),
-    // in packed fp32 pairs.  The prologue is bound by instruction issue (sixteen warps on four
-    // schedulers), so the per-row work is kept to the reads, one butterfly and four packed products.
-    // Consecutive stacked rows share their canvas row, hence their table entries, G at a time.
-    {
-      constexpr uint32_t RPW = BM / SM_WARPS;
-      const bool do_norm = !p.q_prenormed;
-      const uint32_t c = lane, c16 = lane & 15u;
-      const uint32_t R0 = mt * BM + warp * RPW;
-      const uint32_t i0 = R0 / p.G, g0 = R0 % p.G;
-      // byte offset of (row it of this warp, chunk c): (c ^ 16) has the same low three bits, so the
-      // partner sits at the same place two swizzle atoms away
-      uint8_t* q_own = smem + OFF_Q + (c >> 3) * ATOM_BYTES + warp * RPW * 128u;
-      uint8_t* q_par = smem + OFF_Q + ((c ^ 16u) >> 3) * ATOM_BYTES + warp * RPW * 128u;
-      if (!p.early_q) issue_q_rows();
-      if (do_norm) {
-        uint4 w4 = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u), wp4 = w4;   // bf16 1.0
-        if (p.qw) {
-          w4 = reinterpret_cast<const uint4*>(p.qw)[c];
-          wp4 = reinterpret_cast<const uint4*>(p.qw)[c ^ 16u];
-        }
-        // low half of a row: x cos - partner sin; high half: x cos + partner sin
-        const float sgn = lane < 16u ? -1.0f : 1.0f;
-        const uint64_t sgn2 = pack_f32x2(sgn, sgn);
-        const uint32_t wm[4] = {w4.x, w4.y, w4.z, w4.w};
-        const uint32_t wq[4] = {wp4.x, wp4.y, wp4.z, wp4.w};
-        uint64_t wm2[4], wq2[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          wm2[e] = bf16x2_to_f32x2(wm[e]);
-          wq2[e] = mul_f32x2(bf16x2_to_f32x2(wq[e]), sgn2);
-        }
-        uint64_t A[4], B[4];   // w cos and -/+ w_partner sin of this lane's eight pairs
-        float4 raw[4];         // the table entries of the NEXT canvas row, requested one canvas row ahead
-        auto fetch_table = [&](uint32_t i) {
-          // (cos, sin) of the pairs 8 c16 .. 8 c16 + 7 of canvas row i
-          const float4* tab = reinterpret_cast<const float4*>(p.rope_table + size_t(i < p.C ? i : p.C - 1u) * 128 + c16 * 8u);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) raw[e] = tab[e];
-        };
-        auto use_table = [&]() {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            A[e] = mul_f32x2(wm2[e], pack_f32x2(raw[e].x, raw[e].z));
-            B[e] = mul_f32x2(wq2[e], pack_f32x2(raw[e].y, raw[e].w));
-          }
-        };
-        if (R0 < rows_per_head) fetch_table(i0);
-        cp_async_wait_all();
-        __syncwarp();
-        uint32_t i = i0, g = g0;
-        if (R0 < rows_per_head) {
-          use_table();
-          fetch_table(i0 + 1u);   // in flight while the rows of canvas row i0 are worked on
-        }
-#pragma unroll
-        for (uint32_t it = 0; it < RPW; ++it) {
-          if (R0 + it >= rows_per_head) break;   // warp-uniform
-          if (it != 0 && g == 0) {
-            use_table();
-            fetch_table(i + 1u);
-          }
-          const uint32_t off = it * 128u + (((c & 7u) ^ it) << 4);
-          const uint4 xm = *reinterpret_cast<const uint4*>(q_own + off);
-          const uint4 xq = *reinterpret_cast<const uint4*>(q_par + off);
-          const uint32_t m[4] = {xm.x, xm.y, xm.z, xm.w};
-          const uint32_t q[4] = {xq.x, xq.y, xq.z, xq.w};
-          uint64_t m2[4];
-          uint64_t acc = 0ull;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            m2[e] = bf16x2_to_f32x2(m[e]);
-            acc = fma_f32x2(m2[e], m2[e], acc);
-          }
-          float s0, s1;
-          unpack_f32x2(acc, s0, s1);
-          float ss = s0 + s1;
-#pragma unroll
-          for (uint32_t o = 16; o >= 1; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);   // identical in every lane
-          const float inv = rsqrtf(ss * (1.0f / float(HD)) + p.eps);
-          const uint64_t inv2 = pack_f32x2(inv, inv);
-          uint32_t y[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint64_t t = fma_f32x2(m2[e], A[e], mul_f32x2(bf16x2_to_f32x2(q[e]), B[e]));
-            float y0, y1;
-            unpack_f32x2(mul_f32x2(t, inv2), y0, y1);
-            y[e] = pack_bf16x2(y0, y1);
-          }
-          __syncwarp();   // the partner has read this chunk
-          *reinterpret_cast<uint4*>(q_own + off) = make_uint4(y[0], y[1], y[2], y[3]);
-          if (++g == p.G) { g = 0; ++i; }
-        }
-      } else {
-        cp_async_wait_all();
-      }
-    }
-    if (PAIR) fence_proxy_async_all(); else fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-      if (PAIR) mbar_arrive_cluster(lead_bar(B_Q)); else mbar_arrive(bar_addr(bar_base, B_Q));
-    }
-    stamp(p, 2);
-
+    // Two things stand between the set-up and the first score tile: this CTA's Q rows and its share of the canvas
+    // append.  The append goes first, while the raw Q rows are on their way: other CTAs wait for it (those whose splits
+    // hold the canvas keys, before their loads), nobody else waits for this CTA's Q.
     // ---------------------------------------------------------------- canvas append inside the launch
     // The 2 C Hkv head vectors of canvas K / V are cut into units of up to four heads of one token's K or V (the
     // token's rotation is prepared once per unit) and the units into shares of one unit per softmax warp.  Every CTA
@@ -347,10 +241,12 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     // that are running - also when part of the grid has not been scheduled yet (more clusters than fit) - and
     // none of them needs anything from anybody to finish its shares.  Whoever waits for the append (the
     // loaders, before a key tile that holds canvas positions) therefore never waits for a CTA that has not
-    // started.  The window between "Q is ready" and the first score tile is otherwise idle for these warps.
-    // The last CTA to leave the kernel puts the counters back to zero.
+    // started.  The last CTA to leave the kernel puts the counters back to zero.
     if (p.ap_vectors != 0u) {
       if (p.early_q) asm volatile("griddepcontrol.wait;" ::: "memory");   // the cache may still be in use ahead of us
+      uint32_t ticket = 0;
+      if (tid == 0) ticket = atomicAdd(p.ap_ctl, 1u);   // in flight while the rows are asked for
+      if (!p.early_q) issue_q_rows();
       AppendVecArgs av;
       av.k_in = p.ap_k;
       av.v_in = p.ap_v;
@@ -366,18 +262,20 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       av.write_end = p.ap_write_end;
       av.pos_base = p.pos_base;
       av.eps = p.eps;
-      // a share = one unit (up to four heads of one token's K or V) for every softmax warp
-      const uint32_t n_units = append_unit_count(p.ap_vectors / (2u * p.Hkv), p.Hkv);
-      const uint32_t n_shares = (n_units + SM_WARPS - 1u) / SM_WARPS;
+      // a share = one unit (up to ap_unit_heads heads of one token's K or V) for every softmax warp
+      const uint32_t groups = append_unit_groups(p.Hkv, p.ap_unit_heads);
+      const uint32_t n_units = p.ap_vectors / p.Hkv * groups;
+      const uint32_t n_shares = append_share_count(p.ap_vectors / (2u * p.Hkv), p.Hkv, p.ap_unit_heads);
+      static_assert(SM_WARPS == kAppendShareUnits, "one unit per softmax warp");
       uint4 kw_own, kw_partner;
       append_norm_weight(av, lane, kw_own, kw_partner);
       // In a share the K units (norm, rotation) and the V units (a copy unless V is normed) of a token alternate
       // in runs of `groups`; odd shares shift the warps by one run, so that no warp gets the K units every time.
-      const uint32_t groups = (p.Hkv + APPEND_UNIT_HEADS - 1u) / APPEND_UNIT_HEADS;
       uint32_t mine = 0;
       // the next share number is asked for before the work on this one starts: its round trip through the counter
       // (about 500 cycles) then runs beside the work
-      if (tid == 0) ctl[3u] = atomicAdd(p.ap_ctl, 1u);
+      if (tid == 0) ctl[3u] = ticket;
+#pragma unroll 1
       for (uint32_t it = 0;; ++it) {
         // two slots in turn: a slot is rewritten only after the barrier that follows everybody's read of it
         asm volatile("bar.sync 5, %0;" ::"n"(SM_WARPS * 32) : "memory");
@@ -386,7 +284,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
         uint32_t next = 0;
         if (tid == 0) next = atomicAdd(p.ap_ctl, 1u);
         const uint32_t u = share * SM_WARPS + ((warp + (share & 1u) * groups) % SM_WARPS);
-        if (u < n_units) mine += append_table_unit(av, u, lane, kw_own, kw_partner);
+        if (u < n_units) mine += append_table_unit(av, u, lane, p.ap_unit_heads, groups, kw_own, kw_partner);
         if (tid == 0) ctl[3u + ((it + 1u) & 1u)] = next;
       }
       if (mine != 0u) {
@@ -394,7 +292,97 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
         __syncwarp();
         if (lane == 0) atomicAdd(p.ap_ctl + 1, mine);
       }
+    } else if (!p.early_q) {
+      issue_q_rows();
     }
+    stamp(p, 15);
+
+    // ---------------------------------------------------------------- Q prologue (half a warp per row)
+    // A warp takes eight rows of the tile, two at a time; lane c of a half owns the 16-byte chunks c and c + 16 of a row,
+    // which are each other's RoPE partners: for every pair
+    //     rsqrt(mean(x^2) + eps) * (x * (w cos) -/+ partner * (w_partner sin)),
+    // in packed fp32 pairs, both chunks rewritten in their final (swizzled) place.  The code runs once per launch, so what
+    // bounds it is fetching its instructions: the loop is kept rolled, and its body small.
+    {
+      constexpr uint32_t RPW = BM / SM_WARPS;
+      const uint32_t c = lane & 15u, half = lane >> 4;
+      uint8_t* q_own = smem + OFF_Q + (c >> 3) * ATOM_BYTES + warp * RPW * 128u;   // chunk c; chunk c + 16: two atoms on
+      if (!p.q_prenormed) {
+        uint4 w_lo = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u), w_hi = w_lo;   // bf16 1.0
+        if (p.qw) {
+          w_lo = reinterpret_cast<const uint4*>(p.qw)[c];
+          w_hi = reinterpret_cast<const uint4*>(p.qw)[c + 16u];
+        }
+        const uint32_t wl[4] = {w_lo.x, w_lo.y, w_lo.z, w_lo.w}, wh[4] = {w_hi.x, w_hi.y, w_hi.z, w_hi.w};
+        // canvas row of this half's row; consecutive stacked rows share it, and its table entries, G at a time
+        uint32_t R = mt * BM + warp * RPW + half, i = R / p.G, g = R % p.G;
+        float4 raw[4];         // (cos, sin) of the pairs 8 c .. 8 c + 7 of canvas row i
+        auto fetch_table = [&]() {
+          const float4* tab = reinterpret_cast<const float4*>(p.rope_table + size_t(i < p.C ? i : p.C - 1u) * 128 + c * 8u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) raw[e] = tab[e];
+        };
+        fetch_table();
+        cp_async_wait_all();
+        __syncwarp();
+        const uint64_t neg2 = pack_f32x2(-1.0f, -1.0f);
+#pragma unroll 1
+        for (uint32_t r8 = half; r8 < RPW; r8 += 2u, R += 2u) {
+          uint8_t* at = q_own + r8 * 128u + (((c & 7u) ^ r8) << 4);
+          const uint4 xl = *reinterpret_cast<const uint4*>(at), xh = *reinterpret_cast<const uint4*>(at + 2u * ATOM_BYTES);
+          const uint32_t lo[4] = {xl.x, xl.y, xl.z, xl.w}, hi[4] = {xh.x, xh.y, xh.z, xh.w};
+          uint64_t l2[4], h2[4], acc_l = 0ull, acc_h = 0ull;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            l2[e] = bf16x2_to_f32x2(lo[e]);
+            h2[e] = bf16x2_to_f32x2(hi[e]);
+            acc_l = fma_f32x2(l2[e], l2[e], acc_l);
+            acc_h = fma_f32x2(h2[e], h2[e], acc_h);
+          }
+          float s0, s1, s2, s3;
+          unpack_f32x2(acc_l, s0, s1);
+          unpack_f32x2(acc_h, s2, s3);
+          float ss = (s0 + s1) + (s2 + s3);
+#pragma unroll
+          for (uint32_t o = 8; o >= 1; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);   // identical in the half warp
+          const float inv = rsqrtf(ss * (1.0f / float(HD)) + p.eps);
+          const uint64_t inv2 = pack_f32x2(inv, inv);
+          uint32_t yl[4], yh[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint64_t cs = pack_f32x2(raw[e].x, raw[e].z), sn = pack_f32x2(raw[e].y, raw[e].w);
+            const uint64_t w2l = bf16x2_to_f32x2(wl[e]), w2h = bf16x2_to_f32x2(wh[e]);
+            const uint64_t tl = fma_f32x2(l2[e], mul_f32x2(w2l, cs), mul_f32x2(h2[e], mul_f32x2(mul_f32x2(w2h, neg2), sn)));
+            const uint64_t th = fma_f32x2(h2[e], mul_f32x2(w2h, cs), mul_f32x2(l2[e], mul_f32x2(w2l, sn)));
+            float y0, y1;
+            unpack_f32x2(mul_f32x2(tl, inv2), y0, y1);
+            yl[e] = pack_bf16x2(y0, y1);
+            unpack_f32x2(mul_f32x2(th, inv2), y0, y1);
+            yh[e] = pack_bf16x2(y0, y1);
+          }
+          // canvas row of the next two rows; its table entries fly during their first half
+          const uint32_t i_now = i;
+          g += 2u;
+          while (g >= p.G) {
+            g -= p.G;
+            ++i;
+          }
+          if (i != i_now) fetch_table();
+          if (R < rows_per_head) {     // rows past the last one keep the zeros that were copied in
+            *reinterpret_cast<uint4*>(at) = make_uint4(yl[0], yl[1], yl[2], yl[3]);
+            *reinterpret_cast<uint4*>(at + 2u * ATOM_BYTES) = make_uint4(yh[0], yh[1], yh[2], yh[3]);
+          }
+        }
+      } else {
+        cp_async_wait_all();
+      }
+    }
+    if (PAIR) fence_proxy_async_all(); else fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      if (PAIR) mbar_arrive_cluster(lead_bar(B_Q)); else mbar_arrive(bar_addr(bar_base, B_Q));
+    }
+    stamp(p, 2);
 
     // ---------------------------------------------------------------- softmax main loop
     const uint32_t R = mt * BM + r;
@@ -433,9 +421,10 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
         for (int e = 0; e < 32; ++e)
           if (!((seen >> e) & 1u)) sraw[e] = 0xff800000u;
       } else if (!mask_range_full(mk, rv, k0, BN)) {
+        const uint32_t seen = mask_bits16(mk, rv, k0 + qd * (CPT / 2)) | (mask_bits16(mk, rv, k0 + 64u + qd * (CPT / 2)) << 16);
 #pragma unroll
         for (int e = 0; e < 32; ++e)
-          if (!mask_visible_row(mk, rv, k0 + (e < 16 ? 0u : 48u) + qd * (CPT / 2) + e)) sraw[e] = 0xff800000u;  // -inf
+          if (!((seen >> e) & 1u)) sraw[e] = 0xff800000u;  // -inf
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -787,11 +776,46 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     } else {
     const bool to_bf16 = direct && p.out != nullptr;
     const float inv_l = l_tot > 0.f ? 1.0f / l_tot : 0.f;
-    const float mul = to_bf16 ? inv_l : 1.0f;
+    const float mul = inv_l;
     float* dst_o = direct ? p.out_o : p.ws_o + size_t(split) * rows_total * HD;
+    if (to_bf16) {
+      // Final rows: a thread rounds its quarter of a row into shared memory (the Q and K tiles are dead; rows of
+      // HBUF_LD halves, free of bank conflicts both ways), then a warp stores eight whole 512-byte rows.
+      uint8_t* rows16 = smem + OFF_Q;
+#pragma unroll
+      for (uint32_t c = 0; c < OPT / 32; ++c) {
+        uint32_t o[32];
+        if (have_o) {
+          tmem_ld32(t_lane + TM_O + qd * OPT + c * 32u, o);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = 0u;
+        }
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            w[e] = pack_bf16x2(__uint_as_float(o[q4 * 8 + 2 * e]) * mul, __uint_as_float(o[q4 * 8 + 2 * e + 1]) * mul);
+          *reinterpret_cast<uint4*>(rows16 + (r * HBUF_LD + qd * OPT + c * 32u + q4 * 8u) * 2u) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      row_group_sync(smw);
+      const uint32_t r0 = smw * 32u + qd * 8u, Rw = mt * BM + r0;
+      uint32_t i = Rw / p.G, g = Rw % p.G;
+#pragma unroll
+      for (uint32_t k = 0; k < 8; ++k) {
+        if (Rw + k < rows_per_head) {
+          const uint4 w = *reinterpret_cast<const uint4*>(rows16 + ((r0 + k) * HBUF_LD + lane * 8u) * 2u);
+          *reinterpret_cast<uint4*>(p.out + (size_t(i) * p.Hq + kvh * p.G + g) * HD + lane * 8u) = w;
+        }
+        if (++g == p.G) { g = 0; ++i; }
+      }
+    } else {
     // Each thread owns a quarter of one row in TMEM, but rows are 1 KB apart in memory.  A 32 x 32
     // chunk goes through a padded per-warp tile in shared memory (the Q tile is dead by now) so that
-    // every store instruction of the warp writes four full 128-byte lines (64-byte for bf16).
+    // every store instruction of the warp writes four full 128-byte lines.
     float* tile = reinterpret_cast<float*>(smem + OFF_Q) + warp * (32 * 36);
     size_t orow_k[8];
     bool valid_k[8];
@@ -816,24 +840,17 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
 #pragma unroll
       for (int q4 = 0; q4 < 8; ++q4)
         *reinterpret_cast<float4*>(tile + lane * 36 + q4 * 4) =
-            make_float4(__uint_as_float(o[q4 * 4]) * mul, __uint_as_float(o[q4 * 4 + 1]) * mul,
-                        __uint_as_float(o[q4 * 4 + 2]) * mul, __uint_as_float(o[q4 * 4 + 3]) * mul);
+            make_float4(__uint_as_float(o[q4 * 4]), __uint_as_float(o[q4 * 4 + 1]), __uint_as_float(o[q4 * 4 + 2]),
+                        __uint_as_float(o[q4 * 4 + 3]));
       __syncwarp();
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const float4 v4 = *reinterpret_cast<const float4*>(tile + (k * 4 + (lane >> 3)) * 36 + (lane & 7) * 4);
-        if (!valid_k[k]) continue;
-        if (to_bf16) {
-          uint2 w2;
-          w2.x = pack_bf16x2(v4.x, v4.y);
-          w2.y = pack_bf16x2(v4.z, v4.w);
-          *reinterpret_cast<uint2*>(p.out + orow_k[k] * HD + col0 + (lane & 7) * 4) = w2;
-        } else {
-          *reinterpret_cast<float4*>(dst_o + orow_k[k] * HD + col0 + (lane & 7) * 4) = v4;
-        }
+        if (valid_k[k]) *reinterpret_cast<float4*>(dst_o + orow_k[k] * HD + col0 + (lane & 7) * 4) = v4;
       }
       __syncwarp();
     }
+    }   // !to_bf16
     if (valid && !to_bf16 && qd == 0) {
       if (direct) {
         p.out_m[orow] = m_used * 0.6931471805599453f;   // log2 units -> natural units

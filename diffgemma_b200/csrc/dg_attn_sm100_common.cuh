@@ -133,7 +133,7 @@ __device__ __forceinline__ uint32_t bar_addr(uint32_t bar_base, uint32_t idx) { 
 // 6 MMA issuer on K tiles, 7 on V tiles, 8 on P (softmax output), 9 its whole loop,
 // 10 softmax thread 0 on S (scores), 11 softmax thread 0 on the rescale barrier.
 // Slots 12-14 are time stamps inside the tail: 12 the last PV has completed, 13 the cluster's CTAs have all
-// finished their MMAs (cluster merge only), 14 the partial rows of the cluster have all arrived.
+// finished their MMAs (cluster merge only), 14 the partial rows of the cluster have all arrived.  15: this CTA's part of the in-launch append is done.
 constexpr uint32_t STAMP_SLOTS = 16;
 __device__ __forceinline__ void stamp(const AttnParams& p, uint32_t slot) {
   if (p.stamps != nullptr && threadIdx.x == 0) {

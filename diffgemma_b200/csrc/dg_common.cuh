@@ -83,6 +83,15 @@ __host__ __device__ inline bool mask_visible_row(const MaskParams& m, const RowV
 __host__ __device__ inline bool mask_visible(const MaskParams& m, uint32_t row, uint32_t t) {
   return mask_visible_row(m, mask_row(m, row), t);
 }
+// bit e: is key k0 + e visible to the row, e < 16 (positions stay below 2^31)
+__host__ __device__ inline uint32_t mask_run16(uint32_t lo, uint32_t hi, uint32_t k0) {
+  const int32_t a = int32_t(lo) - int32_t(k0), b = int32_t(hi) - int32_t(k0);
+  const uint32_t from = a <= 0 ? 0u : a >= 16 ? 16u : uint32_t(a), to = b <= 0 ? 0u : b >= 16 ? 16u : uint32_t(b);
+  return to > from ? ((1u << to) - 1u) & ~((1u << from) - 1u) : 0u;
+}
+__host__ __device__ inline uint32_t mask_bits16(const MaskParams& m, const RowVis& v, uint32_t k0) {
+  return mask_run16(v.lo, m.pre_hi, k0) | mask_run16(v.can_lo, v.can_hi, k0);
+}
 // whole key range [k0, k0 + n) visible to the row
 __host__ __device__ inline bool mask_range_full(const MaskParams& m, const RowVis& v, uint32_t k0, uint32_t n) {
   const bool joined = m.pre_hi == m.kv_len && v.can_lo == m.kv_len && v.can_hi > m.kv_len;
@@ -202,9 +211,17 @@ struct AttnParams {
   __nv_bfloat16* ap_cache_v;
   uint32_t* ap_ctl;              // {next share, vectors done, CTAs finished}: zero between launches
   uint32_t ap_vectors;
+  uint32_t ap_unit_heads;        // heads of one token's K or V that a warp takes at a time (1, 2 or 4)
   uint32_t ap_v_norm;
   uint32_t ap_write_end;         // positions >= this are not stored (0xffffffff: none)
 };
+
+// Shares of the in-launch append: one unit (unit_heads heads of one token's K or V) for each of a CTA's 16 softmax warps.
+constexpr uint32_t kAppendShareUnits = 16;
+__host__ __device__ inline uint32_t append_unit_groups(uint32_t Hkv, uint32_t unit_heads) { return (Hkv + unit_heads - 1u) / unit_heads; }
+__host__ __device__ inline uint32_t append_share_count(uint32_t n_tok, uint32_t Hkv, uint32_t unit_heads) {
+  return (n_tok * 2u * append_unit_groups(Hkv, unit_heads) + kAppendShareUnits - 1u) / kAppendShareUnits;
+}
 
 // Up to kMaxBatchLaunch independent canvases served by ONE launch of the head_dim-256 tensor kernel
 // (blockIdx.z = canvas): the kernel's whole parameter block, tensor maps first (64-byte aligned).
