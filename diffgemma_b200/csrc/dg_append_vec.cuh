@@ -134,16 +134,16 @@ __device__ __forceinline__ void append_table_vector(const AppendVecArgs& p, uint
 
 // The same work cut into units of up to unit_heads (at most APPEND_UNIT_HEADS) heads of one token's K or V: a warp loads
 // the vectors of its unit together and prepares the token's rotation once.  Unit u = (tok * 2 + kv) * groups + grp with
-// groups = ceil(Hkv / unit_heads); returns how many vectors the unit stands for (written or not).
+// groups = ceil(Hkv / unit_heads).
 constexpr uint32_t APPEND_UNIT_HEADS = 4;
-__device__ __forceinline__ uint32_t append_table_unit(const AppendVecArgs& p, uint32_t u, uint32_t lane, uint32_t unit_heads,
+__device__ __forceinline__ void append_table_unit(const AppendVecArgs& p, uint32_t u, uint32_t lane, uint32_t unit_heads,
                                                       uint32_t groups, const uint4 kw_own, const uint4 kw_partner) {
   const uint32_t tok = u / (2u * groups), rem = u % (2u * groups);
   const bool is_k = rem < groups;
   const uint32_t h0 = (is_k ? rem : rem - groups) * unit_heads;
   const uint32_t nh = p.Hkv - h0 < unit_heads ? p.Hkv - h0 : unit_heads;
   const uint32_t pos = p.pos0 + tok;
-  if (pos >= p.write_end || pos < p.pos_base) return nh;
+  if (pos >= p.write_end || pos < p.pos_base) return;
   const uint4* src = reinterpret_cast<const uint4*>((is_k ? p.k_in : p.v_in) + (size_t(tok) * p.Hkv + h0) * 256u) + lane;
   uint4 x[APPEND_UNIT_HEADS];
 #pragma unroll
@@ -157,7 +157,6 @@ __device__ __forceinline__ uint32_t append_table_unit(const AppendVecArgs& p, ui
 #pragma unroll
     for (uint32_t e = 0; e + 1 < APPEND_UNIT_HEADS; ++e) x[e] = x[e + 1];
   }
-  return nh;
 }
 
 }  // namespace dg

@@ -70,7 +70,8 @@ enum : uint32_t {
   B_P_FULL = 11,   // +buffer: P of the tile's keys [0, 64)
   B_O_FINAL = 14,  // single phase: every PV of this CTA has completed
   B_P2_FULL = 15,  // +buffer: P of the tile's keys [64, 128)
-  B_COUNT = 17
+  B_RX = 17,       // cluster merge, single phase: the other splits' rows have landed (bytes counted)
+  B_COUNT = 18
 };
 }  // namespace one
 
@@ -138,7 +139,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   };
 
   static_assert(!(PAIR && BITS), "the bitmap form runs one CTA per query tile");
-  uint32_t* live = reinterpret_cast<uint32_t*>(smem + OFF_ML);   // BITS: tiles with a visible key (no cluster merge then)
+  uint32_t* live = reinterpret_cast<uint32_t*>(smem + OFF_LIVE);   // BITS: tiles with a visible key
   // both CTAs of a pair walk the same key tiles: schedule from the pair's first canvas row
   const uint32_t row_first = ((PAIR ? (mt & ~1u) : mt) * BM) / p.G;
   const uint32_t row_last = (((PAIR ? (mt | 1u) : mt) + 1u) * BM - 1u) / p.G;
@@ -184,6 +185,8 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       mbar_init(bar_addr(bar_base, B_P2_FULL + st), (PAIR ? 2u : 1u) * SM_WARPS);
     }
     mbar_init(bar_addr(bar_base, B_O_FINAL), 1);
+    mbar_init(bar_addr(bar_base, B_RX), 1);
+    if (cs > 1) mbar_expect_tx(bar_addr(bar_base, B_RX), (cs - 1u) * (BM / cs) * ROW_BYTES);
     ctl[1] = 0u;
     ctl[2] = 0u;
     fence_mbar_init();
@@ -230,6 +233,8 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   // per-row softmax state (identical in every thread of a row, except l_run which is per quarter)
   float m_used = -INFINITY, l_run = 0.f;
 
+  // opens a share of the append: the softmax warps and the MMA warp
+  auto append_sync = [&]() { asm volatile("bar.sync 5, %0;" ::"n"((SM_WARPS + 1u) * 32) : "memory"); };
   if (warp < SM_WARPS) {
     // Two things stand between the set-up and the first score tile: this CTA's Q rows and its share of the canvas
     // append.  The append goes first, while the raw Q rows are on their way: other CTAs wait for it (those whose splits
@@ -271,26 +276,20 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       append_norm_weight(av, lane, kw_own, kw_partner);
       // In a share the K units (norm, rotation) and the V units (a copy unless V is normed) of a token alternate
       // in runs of `groups`; odd shares shift the warps by one run, so that no warp gets the K units every time.
-      uint32_t mine = 0;
       // the next share number is asked for before the work on this one starts: its round trip through the counter
       // (about 500 cycles) then runs beside the work
       if (tid == 0) ctl[3u] = ticket;
 #pragma unroll 1
       for (uint32_t it = 0;; ++it) {
         // two slots in turn: a slot is rewritten only after the barrier that follows everybody's read of it
-        asm volatile("bar.sync 5, %0;" ::"n"(SM_WARPS * 32) : "memory");
+        append_sync();
         const uint32_t share = ctl[3u + (it & 1u)];
         if (share >= n_shares) break;
         uint32_t next = 0;
         if (tid == 0) next = atomicAdd(p.ap_ctl, 1u);
         const uint32_t u = share * SM_WARPS + ((warp + (share & 1u) * groups) % SM_WARPS);
-        if (u < n_units) mine += append_table_unit(av, u, lane, p.ap_unit_heads, groups, kw_own, kw_partner);
+        if (u < n_units) append_table_unit(av, u, lane, p.ap_unit_heads, groups, kw_own, kw_partner);
         if (tid == 0) ctl[3u + ((it + 1u) & 1u)] = next;
-      }
-      if (mine != 0u) {
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) atomicAdd(p.ap_ctl + 1, mine);
       }
     } else if (!p.early_q) {
       issue_q_rows();
@@ -565,6 +564,25 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     // The whole warp runs the loop and its waits; one lane, chosen by elect.sync, issues.  With the issuing
     // branch under elect.sync the instruction stream of an MMA is shorter than under a lane == 0 test
     // (measured on the head_dim-512 kernel: a quarter less time per step with the tensor pipe free-running).
+    if (p.ap_vectors != 0u) {
+      // This warp, idle until Q is there, publishes the softmax warps' shares of the append, so that none of them waits
+      // for its stores to reach L2: at the barrier that opens a share all stores of the one before have been issued.
+      const uint32_t groups = append_unit_groups(p.Hkv, p.ap_unit_heads), n_units = p.ap_vectors / p.Hkv * groups;
+      const uint32_t n_shares = append_share_count(p.ap_vectors / (2u * p.Hkv), p.Hkv, p.ap_unit_heads);
+      uint32_t done = 0;      // vectors of the share in hand
+      for (uint32_t it = 0;; ++it) {
+        append_sync();
+        const uint32_t share = ctl[3u + (it & 1u)];
+        if (it != 0u && lane == 0) {
+          __threadfence();
+          atomicAdd(p.ap_ctl + 1, done);
+        }
+        if (share >= n_shares) break;
+        const uint32_t u = share * SM_WARPS + lane, h0 = (u % groups) * p.ap_unit_heads;
+        const uint32_t nh = p.Hkv - h0 < p.ap_unit_heads ? p.Hkv - h0 : p.ap_unit_heads;
+        done = __reduce_add_sync(0xffffffffu, lane < SM_WARPS && u < n_units ? nh : 0u);
+      }
+    }
     if (n_local > 0 && is_leader) {
       auto uni = [&](bool ok1) -> bool { return __all_sync(0xffffffffu, ok1); };
       constexpr uint32_t IDESC_QK = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, 0);   // A, B K-major
@@ -687,11 +705,6 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     }
   }
   stamp(p, 12);
-  // Cluster merge: partial rows are pushed into the owner CTA's Q/K/V region, which must be dead
-  // in EVERY CTA of the cluster first - all of this CTA's MMAs are complete once its softmax
-  // warps have seen O_FINAL, and this barrier collects that from all CTAs.
-  if (cs > 1) cluster_sync_all();
-  stamp(p, 13);
   if (warp < SM_WARPS) {
     const uint32_t R = mt * BM + r;
     const bool valid = R < rows_per_head;
@@ -708,41 +721,22 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     const bool direct = (p.n_splits == 1);
     const bool via_dsmem = cs > 1;
     if (via_dsmem) {
-      // The partial stays on chip.  Row r of the query tile is merged by CTA r / (BM / S) of the
-      // cluster, so each thread pushes its columns of the un-normalised O row (and one thread the
-      // row's (m, l, 1 / scale)) straight into that CTA's receive buffer with remote shared-memory
-      // stores: recv[source CTA][row within the owner's share][HBUF_LD halves] in the dead Q/K/V
-      // region.  An SM moves only about 16 B/clk into another SM's shared memory, so the rows travel
-      // as fp16 with one power-of-two scale per row that puts the row's largest magnitude into
-      // [2^14, 2^15): 11 significant bits relative to the row maximum whatever the range of V, against
-      // the 8 bits of the bf16 output, and half the bytes.
-      const uint32_t rpc = BM / cs;
-      // split index of this CTA inside the cluster and cluster rank of the CTA that owns row r
-      // (pair form: the CTA with the same position in its pair)
-      const uint32_t src_rank = PAIR ? (crank >> 1) : crank;
-      const uint32_t owner_split = r / rpc, rl = r % rpc;
-      const uint32_t owner = PAIR ? ((owner_split << 1) | xi) : owner_split;
-      // rows this CTA owns itself stay in its own shared memory (plain stores): only the others' rows
-      // take the SM-to-SM path
-      const bool own = owner == crank;
-      const uint32_t row_local = smem_base + OFF_Q + ((src_rank * rpc + rl) * HBUF_LD) * 2u;
-      const uint32_t dst_row = own ? row_local : dsmem_addr(row_local, owner);
-      uint32_t oa[32], ob[32];
-      if (have_o) {
-        tmem_ld32(t_lane + TM_O + qd * OPT, oa);
-        tmem_ld32(t_lane + TM_O + qd * OPT + 32u, ob);
-        tmem_wait_ld();
-      } else {
-#pragma unroll
-        for (uint32_t e = 0; e < 32; ++e) oa[e] = ob[e] = 0u;
-      }
+      // The partial stays on chip.  Row r of the query tile is merged by CTA r / (BM / S) of the cluster.  Every CTA
+      // lays its un-normalised rows out in its own (dead) K/V region, [BM] rows of ROW_BYTES: the row as fp16 with
+      // one power-of-two scale that puts its largest magnitude into [2^14, 2^15) - 11 significant bits relative to the
+      // row maximum whatever the range of V, against the 8 bits of the bf16 output, and half the bytes -, then the
+      // row's (m, l, 1 / scale) in what would be padding.  One bulk copy per owner then moves BM / S rows at once.
+      uint8_t* row = smem + OFF_STAGE + r * ROW_BYTES;
       float amax = 0.f;
+#pragma unroll 1
+      for (uint32_t c = 0; c < OPT / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld32(t_lane + TM_O + qd * OPT + c * 32u, o);
+        tmem_wait_ld();
 #pragma unroll
-      for (uint32_t e = 0; e < 32; e += 2) {
-        amax = max3_f32(amax, fabsf(__uint_as_float(oa[e])), fabsf(__uint_as_float(oa[e + 1])));
-        amax = max3_f32(amax, fabsf(__uint_as_float(ob[e])), fabsf(__uint_as_float(ob[e + 1])));
+        for (uint32_t e = 0; e < 32; e += 2) amax = max3_f32(amax, fabsf(__uint_as_float(o[e])), fabsf(__uint_as_float(o[e + 1])));
       }
-      xch_misc[r * NTR + qd] = amax;
+      xch_misc[r * NTR + qd] = have_o ? amax : 0.f;
       row_group_sync(smw);
       float rmax = 0.f;
 #pragma unroll
@@ -752,27 +746,27 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       const bool scaled = eb >= 15u && eb < 255u;
       const float sc = scaled ? __uint_as_float((268u - eb) << 23) : 1.0f;       // 2^(14 - exponent)
       const float inv_sc = scaled ? __uint_as_float((eb - 14u) << 23) : 1.0f;
+#pragma unroll 1
+      for (uint32_t c = 0; c < OPT / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld32(t_lane + TM_O + qd * OPT + c * 32u, o);
+        tmem_wait_ld();
+        if (!have_o) {
 #pragma unroll
-      for (uint32_t q4 = 0; q4 < 4; ++q4) {
-        uint32_t ha[4], hb[4];
-#pragma unroll
-        for (uint32_t e = 0; e < 4; ++e) {
-          ha[e] = pack_f16x2(__uint_as_float(oa[q4 * 8 + 2 * e]) * sc, __uint_as_float(oa[q4 * 8 + 2 * e + 1]) * sc);
-          hb[e] = pack_f16x2(__uint_as_float(ob[q4 * 8 + 2 * e]) * sc, __uint_as_float(ob[q4 * 8 + 2 * e + 1]) * sc);
+          for (uint32_t e = 0; e < 32; ++e) o[e] = 0u;
         }
-        if (own) {
-          smem_st_u4(dst_row + (qd * OPT + q4 * 8u) * 2u, make_uint4(ha[0], ha[1], ha[2], ha[3]));
-          smem_st_u4(dst_row + (qd * OPT + 32u + q4 * 8u) * 2u, make_uint4(hb[0], hb[1], hb[2], hb[3]));
-        } else {
-          dsmem_st_u4(dst_row + (qd * OPT + q4 * 8u) * 2u, make_uint4(ha[0], ha[1], ha[2], ha[3]));
-          dsmem_st_u4(dst_row + (qd * OPT + 32u + q4 * 8u) * 2u, make_uint4(hb[0], hb[1], hb[2], hb[3]));
+#pragma unroll
+        for (uint32_t q4 = 0; q4 < 4; ++q4) {
+          uint32_t w[4];
+#pragma unroll
+          for (uint32_t e = 0; e < 4; ++e)
+            w[e] = pack_f16x2(__uint_as_float(o[q4 * 8 + 2 * e]) * sc, __uint_as_float(o[q4 * 8 + 2 * e + 1]) * sc);
+          *reinterpret_cast<uint4*>(row + (qd * OPT + c * 32u + q4 * 8u) * 2u) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
-      if (qd == 0) {
-        const uint32_t ml_local = smem_base + OFF_ML + (src_rank * rpc + rl) * 16u;
-        const uint4 rec = make_uint4(__float_as_uint(m_used), __float_as_uint(l_tot), __float_as_uint(inv_sc), 0u);
-        if (own) smem_st_u4(ml_local, rec); else dsmem_st_u4(dsmem_addr(ml_local, owner), rec);
-      }
+      if (qd == 0)
+        *reinterpret_cast<uint4*>(row + HD * 2u) = make_uint4(__float_as_uint(m_used), __float_as_uint(l_tot), __float_as_uint(inv_sc), 0u);
+      fence_proxy_async_smem();      // ordinary stores, read by the bulk copies
     } else {
     const bool to_bf16 = direct && p.out != nullptr;
     const float inv_l = l_tot > 0.f ? 1.0f / l_tot : 0.f;
@@ -864,6 +858,20 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     }   // !via_dsmem
   }
 
+  // Rows are copied into the owner CTA's Q/K region, which must be dead in EVERY CTA of the cluster first: all of this
+  // CTA's MMAs are complete once its softmax warps have seen O_FINAL, and this barrier collects that, and the staged
+  // rows of this CTA, from everybody.
+  stamp(p, 13);
+  if (cs > 1) {
+    cluster_sync_all();
+    const uint32_t rank = PAIR ? (crank >> 1) : crank, rpc = BM / cs;
+    if (tid < cs && tid != rank) {
+      // rows owned by split `tid` of the cluster (pair form: by the CTA with the same position in its pair)
+      const uint32_t owner = PAIR ? ((tid << 1) | xi) : tid;
+      bulk_copy_dsmem(dsmem_addr(smem_base + OFF_Q + rank * rpc * ROW_BYTES, owner), smem_base + OFF_STAGE + tid * rpc * ROW_BYTES,
+                      rpc * ROW_BYTES, dsmem_addr(bar_addr(bar_base, B_RX), owner));
+    }
+  }
   stamp(p, 4);
   // ------------------------------------------------------------------ teardown
   if (*abort_flag) {
@@ -878,9 +886,8 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   __syncthreads();
   if (PAIR) {
     // Neither CTA of the pair may free tensor memory or leave while the other can still be the
-    // target of a pair-wide MMA or commit; in cluster-merge mode this barrier also closes the
-    // exchange of partial rows.
-    cluster_sync_all();
+    // target of a pair-wide MMA or commit (in cluster-merge mode the barrier above has seen to that).
+    if (cs == 1) cluster_sync_all();
     if (warp == W_MMA) tmem_dealloc_pair(tmem, TMEM_COLS);
   } else if (warp == W_MMA) {
     tmem_dealloc(tmem, TMEM_COLS);
@@ -889,16 +896,15 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   // ------------------------------------------------------------------ split merge, level 1: inside the cluster
   if (cs > 1) {
     // The cs CTAs that hold consecutive splits of this query tile are one thread-block cluster
-    // (cluster dims (1, cs, 1), pair form (2, cs, 1)).  Every CTA has pushed each partial row to the
-    // CTA that owns it; after the cluster barrier CTA k holds all cs partials of rows
-    // [k*BM/cs, (k+1)*BM/cs) in its own shared memory and merges them.  Nothing touches remote
-    // shared memory after the barrier, so no second barrier is needed.
-    if (!PAIR) cluster_sync_all();
+    // (cluster dims (1, cs, 1), pair form (2, cs, 1)).  CTA k merges rows [k*BM/cs, (k+1)*BM/cs): its own partial where
+    // it was staged, the others' where their copies land.
+    __all_sync(0xffffffffu, mbar_wait_cluster(bar_addr(bar_base, B_RX), 0u, abort_flag));
     stamp(p, 14);
     const uint32_t rank = PAIR ? (crank >> 1) : crank;
     const uint32_t rpc = BM / cs;
-    const __half* recv = reinterpret_cast<const __half*>(smem + OFF_Q);      // [cs][rpc][HBUF_LD], scaled
-    const float4* recv_ml = reinterpret_cast<const float4*>(smem + OFF_ML);  // [cs][rpc]: m, l, 1 / scale
+    const uint8_t* recv = smem + OFF_Q;                                      // [cs][rpc] rows; this CTA's own place stays empty
+    const uint8_t* own_rows = smem + OFF_STAGE + rank * rpc * ROW_BYTES;     // [rpc] rows
+    auto part = [&](uint32_t s2, uint32_t rl) { return (s2 == rank ? own_rows : recv + s2 * rpc * ROW_BYTES) + rl * ROW_BYTES; };
     // A warp merges four rows at a time (lane = eight columns), every lane reading the cs (m, l)
     // pairs itself: no shuffles and four independent chains, because this pass is bound by latency
     constexpr uint32_t RK1 = 4;
@@ -908,7 +914,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       for (uint32_t k = 0; k < RK1; ++k) {
         const uint32_t rl = rl0 + k < rpc ? rl0 + k : rpc - 1;
         mg[k] = -INFINITY;
-        for (uint32_t s2 = 0; s2 < cs; ++s2) mg[k] = fmaxf(mg[k], recv_ml[s2 * rpc + rl].x);
+        for (uint32_t s2 = 0; s2 < cs; ++s2) mg[k] = fmaxf(mg[k], *reinterpret_cast<const float*>(part(s2, rl) + HD * 2u));
         lg[k] = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[k][e] = 0.f;
@@ -917,11 +923,11 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
 #pragma unroll
         for (uint32_t k = 0; k < RK1; ++k) {
           const uint32_t rl = rl0 + k < rpc ? rl0 + k : rpc - 1;
-          const float4 ml = recv_ml[s2 * rpc + rl];
+          const float4 ml = *reinterpret_cast<const float4*>(part(s2, rl) + HD * 2u);
           const float w = (ml.x == -INFINITY) ? 0.f : fast_exp2(ml.x - mg[k]);
           lg[k] += w * ml.y;
           const float ws = w * ml.z;   // the row's scale folded into its weight
-          const uint4 x = *reinterpret_cast<const uint4*>(recv + (s2 * rpc + rl) * HBUF_LD + lane * 8);
+          const uint4 x = *reinterpret_cast<const uint4*>(part(s2, rl) + lane * 16u);
           const float2 x0 = unpack_f16x2(x.x), x1 = unpack_f16x2(x.y), x2 = unpack_f16x2(x.z), x3 = unpack_f16x2(x.w);
           acc[k][0] += ws * x0.x; acc[k][1] += ws * x0.y; acc[k][2] += ws * x1.x; acc[k][3] += ws * x1.y;
           acc[k][4] += ws * x2.x; acc[k][5] += ws * x2.y; acc[k][6] += ws * x3.x; acc[k][7] += ws * x3.y;
@@ -1194,6 +1200,8 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     }
   }
   stamp(p, 5);
+  // the copies out of this CTA's shared memory have all landed once every CTA of the cluster is through its merge
+  if (cs > 1) cluster_sync_all();
   if (p.ap_vectors != 0u && tid == 0) {
     // every CTA is past its own share taking and its waits on the append counters by now; the last one to
     // get here puts the share counter and the done counter back to zero for the next launch

@@ -20,9 +20,12 @@ constexpr uint32_t OFF_K = TILE_BYTES;
 constexpr uint32_t OFF_V = 2 * TILE_BYTES;
 constexpr uint32_t OFF_BAR = 3 * TILE_BYTES;
 constexpr uint32_t OFF_XCH = OFF_BAR + 256;             // row-group exchange scratch (8 KB)
-constexpr uint32_t OFF_ML = OFF_XCH + 8192;             // (m, l, 1 / scale, -) of the on-chip partial rows, [BM] float4
-constexpr uint32_t HBUF_LD = 264;                       // halves per row of the on-chip partial (padded 256)
-constexpr uint32_t SMEM_BYTES = OFF_ML + 2048 + 1024;   // + alignment slack
+constexpr uint32_t OFF_LIVE = OFF_XCH + 8192;           // bitmap form: live-tile words
+constexpr uint32_t HBUF_LD = 264;                       // halves of a staged row: 256 and 16 bytes (padding, or m, l, 1 / scale)
+constexpr uint32_t ROW_BYTES = HBUF_LD * 2;
+constexpr uint32_t OFF_STAGE = 72 * 1024;               // partial rows on their way out; what comes in lies at OFF_Q
+static_assert(BM * ROW_BYTES <= OFF_STAGE && OFF_STAGE + BM * ROW_BYTES <= OFF_BAR, "exchange buffers");
+constexpr uint32_t SMEM_BYTES = OFF_LIVE + 2048 + 1024;   // + alignment slack
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t TM_S = 0;            // two S buffers of 128 columns
 constexpr uint32_t TM_O = 256;          // O accumulator, 256 columns
@@ -132,8 +135,8 @@ __device__ __forceinline__ uint32_t bar_addr(uint32_t bar_base, uint32_t idx) { 
 // Slots 6-11 hold SM-clock cycles that single threads spent waiting inside the key loop:
 // 6 MMA issuer on K tiles, 7 on V tiles, 8 on P (softmax output), 9 its whole loop,
 // 10 softmax thread 0 on S (scores), 11 softmax thread 0 on the rescale barrier.
-// Slots 12-14 are time stamps inside the tail: 12 the last PV has completed, 13 the cluster's CTAs have all
-// finished their MMAs (cluster merge only), 14 the partial rows of the cluster have all arrived.  15: this CTA's part of the in-launch append is done.
+// Slots 12-14 are time stamps inside the tail: 12 the last PV has completed, 13 this CTA's partial rows are staged
+// (cluster merge only), 14 the other splits' rows have arrived.  15: this CTA's part of the in-launch append is done.
 constexpr uint32_t STAMP_SLOTS = 16;
 __device__ __forceinline__ void stamp(const AttnParams& p, uint32_t slot) {
   if (p.stamps != nullptr && threadIdx.x == 0) {

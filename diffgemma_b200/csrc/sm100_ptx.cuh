@@ -126,30 +126,6 @@ __device__ __forceinline__ uint32_t dsmem_addr(uint32_t local_saddr, uint32_t ra
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_saddr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ float4 dsmem_ld_f4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr)
-               : "memory");
-  return v;
-}
-// plain store to this CTA's own shared memory (shared::cta address)
-__device__ __forceinline__ void smem_st_u4(uint32_t addr, uint4 v) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-__device__ __forceinline__ void dsmem_st_u4(uint32_t addr, uint4 v) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
-               : "memory");
-}
-__device__ __forceinline__ void dsmem_st_f2(uint32_t addr, float2 v) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
-}
-__device__ __forceinline__ float2 dsmem_ld_f2(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-  return v;
-}
 
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA / UMMA reads)
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -352,6 +328,13 @@ __device__ __forceinline__ void dsmem_st_async_f32(uint32_t addr, float v, uint3
 __device__ __forceinline__ void dsmem_st_async_u4(uint32_t addr, uint4 v, uint32_t cluster_bar) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
                "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(cluster_bar)
+               : "memory");
+}
+// asynchronous copy of `bytes` (a multiple of 16) from this CTA's shared memory to 16-byte aligned shared memory of a CTA
+// of the cluster, counted on a barrier of that CTA; no multicast
+__device__ __forceinline__ void bulk_copy_dsmem(uint32_t cluster_dst, uint32_t src, uint32_t bytes, uint32_t cluster_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(cluster_dst),
+               "r"(src), "r"(bytes), "r"(cluster_bar)
                : "memory");
 }
 // tiled load into this CTA's shared memory whose bytes are counted on a barrier of the pair's

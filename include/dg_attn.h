@@ -433,7 +433,7 @@ int32_t dg_ctx_kernel_timing(dg_ctx* ctx, int32_t on, uint32_t max_launches);
  * 2 Q prologue done, 3 key loop done, 4 epilogue done, 5 merge done; slots 6-11 hold SM-clock
  * cycles single threads spent waiting inside the key loop (6 MMA issuer on K, 7 on V, 8 on P,
  * 9 the issuer's whole loop, 10 softmax thread 0 on S, 11 on the rescale barrier); slots 12-14 are
- * stamps inside the tail (12 last PV complete, 13 cluster's MMAs complete, 14 cluster's rows arrived).  The
+ * stamps inside the tail (12 last PV complete, 13 own rows staged, 14 cluster's rows arrived).  The
  * stamps cost time; NULL switches them off.                                                             */
 int32_t dg_ctx_phase_stamps(dg_ctx* ctx, void* device_buffer);
 int32_t dg_ctx_kernel_time(dg_ctx* ctx, double* total_ms, uint32_t* launches);
