@@ -999,12 +999,10 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     p.ws_counters = c->counters;
   }
   if (p.ap_vectors != 0u) {
-    // In-launch append: as many heads per unit of work as share a token's rotation, fewer where that would leave CTAs
-    // of this canvas without a share (32 query tiles x 4 splits of a layer with 8 KV heads: 64 shares of four heads,
-    // 128 of two)
-    const uint32_t ctas = q_tiles * p.n_splits;
-    uint32_t u = p.Hkv >= 4u ? 4u : p.Hkv >= 2u ? 2u : 1u;
-    while (u > 1u && append_share_count(p.C, p.Hkv, u) * 2u <= ctas) u /= 2u;
+    // In-launch append: K and V of one head per unit of work, of more heads (they share the token's rotation) where that
+    // would be more shares than this canvas has CTAs: a second share costs a CTA another round trip and load latency
+    uint32_t u = 1u;
+    while (u < kAppendUnitHeads && u < p.Hkv && append_share_count(p.C, p.Hkv, u) > q_tiles * p.n_splits) u *= 2u;
     p.ap_unit_heads = u;
   }
   if (a.defer != nullptr) {

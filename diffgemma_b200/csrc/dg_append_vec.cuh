@@ -132,30 +132,38 @@ __device__ __forceinline__ void append_table_vector(const AppendVecArgs& p, uint
   append_vector_finish(p, is_k, h, pos, lane, x, rot);
 }
 
-// The same work cut into units of up to unit_heads (at most APPEND_UNIT_HEADS) heads of one token's K or V: a warp loads
-// the vectors of its unit together and prepares the token's rotation once.  Unit u = (tok * 2 + kv) * groups + grp with
+// The same work cut into units, K and V of up to unit_heads (at most APPEND_UNIT_HEADS) heads of one token: a warp loads
+// the unit's vectors together and prepares the token's rotation once.  Unit u = tok * groups + grp with
 // groups = ceil(Hkv / unit_heads).
-constexpr uint32_t APPEND_UNIT_HEADS = 4;
+constexpr uint32_t APPEND_UNIT_HEADS = kAppendUnitHeads;
 __device__ __forceinline__ void append_table_unit(const AppendVecArgs& p, uint32_t u, uint32_t lane, uint32_t unit_heads,
-                                                      uint32_t groups, const uint4 kw_own, const uint4 kw_partner) {
-  const uint32_t tok = u / (2u * groups), rem = u % (2u * groups);
-  const bool is_k = rem < groups;
-  const uint32_t h0 = (is_k ? rem : rem - groups) * unit_heads;
+                                                  uint32_t groups, const uint4 kw_own, const uint4 kw_partner) {
+  const uint32_t tok = u / groups, h0 = (u % groups) * unit_heads;
   const uint32_t nh = p.Hkv - h0 < unit_heads ? p.Hkv - h0 : unit_heads;
   const uint32_t pos = p.pos0 + tok;
   if (pos >= p.write_end || pos < p.pos_base) return;
-  const uint4* src = reinterpret_cast<const uint4*>((is_k ? p.k_in : p.v_in) + (size_t(tok) * p.Hkv + h0) * 256u) + lane;
-  uint4 x[APPEND_UNIT_HEADS];
+  const size_t first = (size_t(tok) * p.Hkv + h0) * 32u + lane;
+  const uint4* ks = reinterpret_cast<const uint4*>(p.k_in) + first;
+  const uint4* vs = reinterpret_cast<const uint4*>(p.v_in) + first;
+  uint4 xk[APPEND_UNIT_HEADS], xv[APPEND_UNIT_HEADS];
 #pragma unroll
-  for (uint32_t j = 0; j < APPEND_UNIT_HEADS; ++j) x[j] = j < nh ? src[j * 32u] : make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t j = 0; j < APPEND_UNIT_HEADS; ++j)
+    if (j < nh) {
+      xk[j] = ks[j * 32u];
+      xv[j] = vs[j * 32u];
+    }
   AppendRot rot;
-  if (is_k) append_token_rot(p, tok, lane, kw_own, kw_partner, rot);
-  // one body for all vectors (the next one moves up): the code runs a few times per launch and is bound by its fetch
+  append_token_rot(p, tok, lane, kw_own, kw_partner, rot);
+  // one body for all vectors (the next ones move up): the code runs a few times per launch and is bound by its fetch
 #pragma unroll 1
   for (uint32_t j = 0; j < nh; ++j) {
-    append_vector_finish(p, is_k, h0 + j, pos, lane, x[0], rot);
+    append_vector_finish(p, true, h0 + j, pos, lane, xk[0], rot);
+    append_vector_finish(p, false, h0 + j, pos, lane, xv[0], rot);
 #pragma unroll
-    for (uint32_t e = 0; e + 1 < APPEND_UNIT_HEADS; ++e) x[e] = x[e + 1];
+    for (uint32_t e = 0; e + 1 < APPEND_UNIT_HEADS; ++e) {
+      xk[e] = xk[e + 1];
+      xv[e] = xv[e + 1];
+    }
   }
 }
 

@@ -233,21 +233,27 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   // per-row softmax state (identical in every thread of a row, except l_run which is per quarter)
   float m_used = -INFINITY, l_run = 0.f;
 
-  // opens a share of the append: the softmax warps and the MMA warp
+  // barrier of the in-launch append: the softmax warps and the MMA warp
   auto append_sync = [&]() { asm volatile("bar.sync 5, %0;" ::"n"((SM_WARPS + 1u) * 32) : "memory"); };
+  // The 2 C Hkv head vectors of canvas K / V are cut into units, K and V of up to four heads of one token (whose rotation
+  // is prepared once), and the units into shares of one unit per softmax warp.
+  const uint32_t ap_groups = p.ap_vectors != 0u ? append_unit_groups(p.Hkv, p.ap_unit_heads) : 1u;
+  const uint32_t ap_units = p.ap_vectors != 0u ? p.ap_vectors / (2u * p.Hkv) * ap_groups : 0u;
+  const uint32_t ap_shares = (ap_units + SM_WARPS - 1u) / SM_WARPS;
+  static_assert(SM_WARPS == kAppendShareUnits, "one unit per softmax warp");
   if (warp < SM_WARPS) {
-    // Two things stand between the set-up and the first score tile: this CTA's Q rows and its share of the canvas
-    // append.  The append goes first, while the raw Q rows are on their way: other CTAs wait for it (those whose splits
-    // hold the canvas keys, before their loads), nobody else waits for this CTA's Q.
+    // Two things stand between the set-up and the first score tile: this CTA's Q rows and its shares of the canvas append.
+    // The append goes first, while the raw Q rows are on their way: other CTAs wait for it (those whose splits hold the
+    // canvas keys, before their loads), nobody else waits for this CTA's Q.
     // ---------------------------------------------------------------- canvas append inside the launch
-    // The 2 C Hkv head vectors of canvas K / V are cut into units of up to four heads of one token's K or V (the
-    // token's rotation is prepared once per unit) and the units into shares of one unit per softmax warp.  Every CTA
-    // that gets here keeps taking shares from a counter until none is left, so all shares are taken by CTAs
+    // Every CTA that gets here keeps taking shares from a counter until none is left, so all shares are taken by CTAs
     // that are running - also when part of the grid has not been scheduled yet (more clusters than fit) - and
     // none of them needs anything from anybody to finish its shares.  Whoever waits for the append (the
     // loaders, before a key tile that holds canvas positions) therefore never waits for a CTA that has not
     // started.  The last CTA to leave the kernel puts the counters back to zero.
-    if (p.ap_vectors != 0u) {
+    // What a share costs is latency: the counter's round trip, then its vectors'.  The launch therefore cuts the work so
+    // that, where possible, a CTA has one share; a unit's loads are all issued together.
+    if (ap_shares != 0u) {
       if (p.early_q) asm volatile("griddepcontrol.wait;" ::: "memory");   // the cache may still be in use ahead of us
       uint32_t ticket = 0;
       if (tid == 0) ticket = atomicAdd(p.ap_ctl, 1u);   // in flight while the rows are asked for
@@ -267,29 +273,18 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       av.write_end = p.ap_write_end;
       av.pos_base = p.pos_base;
       av.eps = p.eps;
-      // a share = one unit (up to ap_unit_heads heads of one token's K or V) for every softmax warp
-      const uint32_t groups = append_unit_groups(p.Hkv, p.ap_unit_heads);
-      const uint32_t n_units = p.ap_vectors / p.Hkv * groups;
-      const uint32_t n_shares = append_share_count(p.ap_vectors / (2u * p.Hkv), p.Hkv, p.ap_unit_heads);
-      static_assert(SM_WARPS == kAppendShareUnits, "one unit per softmax warp");
       uint4 kw_own, kw_partner;
       append_norm_weight(av, lane, kw_own, kw_partner);
-      // In a share the K units (norm, rotation) and the V units (a copy unless V is normed) of a token alternate
-      // in runs of `groups`; odd shares shift the warps by one run, so that no warp gets the K units every time.
-      // the next share number is asked for before the work on this one starts: its round trip through the counter
-      // (about 500 cycles) then runs beside the work
-      if (tid == 0) ctl[3u] = ticket;
 #pragma unroll 1
       for (uint32_t it = 0;; ++it) {
         // two slots in turn: a slot is rewritten only after the barrier that follows everybody's read of it
+        if (tid == 0) ctl[3u + (it & 1u)] = ticket;
         append_sync();
         const uint32_t share = ctl[3u + (it & 1u)];
-        if (share >= n_shares) break;
-        uint32_t next = 0;
-        if (tid == 0) next = atomicAdd(p.ap_ctl, 1u);
-        const uint32_t u = share * SM_WARPS + ((warp + (share & 1u) * groups) % SM_WARPS);
-        if (u < n_units) append_table_unit(av, u, lane, p.ap_unit_heads, groups, kw_own, kw_partner);
-        if (tid == 0) ctl[3u + ((it + 1u) & 1u)] = next;
+        if (share >= ap_shares) break;
+        if (tid == 0) ticket = atomicAdd(p.ap_ctl, 1u);   // its round trip runs beside the work on this share
+        const uint32_t u = share * SM_WARPS + warp;
+        if (u < ap_units) append_table_unit(av, u, lane, p.ap_unit_heads, ap_groups, kw_own, kw_partner);
       }
     } else if (!p.early_q) {
       issue_q_rows();
@@ -299,9 +294,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     // ---------------------------------------------------------------- Q prologue (half a warp per row)
     // A warp takes eight rows of the tile, two at a time; lane c of a half owns the 16-byte chunks c and c + 16 of a row,
     // which are each other's RoPE partners: for every pair
-    //     rsqrt(mean(x^2) + eps) * (x * (w cos) -/+ partner * (w_partner sin)),
-    // in packed fp32 pairs, both chunks rewritten in their final (swizzled) place.  The code runs once per launch, so what
-    // bounds it is fetching its instructions: the loop is kept rolled, and its body small.
+    //     rsqrt(mean(x^2) + eps) * ((x w) cos -/+ (partner w_partner) sin),
+    // in packed fp32 pairs (x w is exact: two bf16), both chunks rewritten in their final (swizzled) place.  The code runs
+    // once per launch, and what bounds it is issuing, and at first fetching, its instructions: a rolled loop, a small body.
     {
       constexpr uint32_t RPW = BM / SM_WARPS;
       const uint32_t c = lane & 15u, half = lane >> 4;
@@ -324,7 +319,6 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
         fetch_table();
         cp_async_wait_all();
         __syncwarp();
-        const uint64_t neg2 = pack_f32x2(-1.0f, -1.0f);
 #pragma unroll 1
         for (uint32_t r8 = half; r8 < RPW; r8 += 2u, R += 2u) {
           uint8_t* at = q_own + r8 * 128u + (((c & 7u) ^ r8) << 4);
@@ -350,9 +344,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const uint64_t cs = pack_f32x2(raw[e].x, raw[e].z), sn = pack_f32x2(raw[e].y, raw[e].w);
-            const uint64_t w2l = bf16x2_to_f32x2(wl[e]), w2h = bf16x2_to_f32x2(wh[e]);
-            const uint64_t tl = fma_f32x2(l2[e], mul_f32x2(w2l, cs), mul_f32x2(h2[e], mul_f32x2(mul_f32x2(w2h, neg2), sn)));
-            const uint64_t th = fma_f32x2(h2[e], mul_f32x2(w2h, cs), mul_f32x2(l2[e], mul_f32x2(w2l, sn)));
+            const uint64_t nsn = pack_f32x2(-raw[e].y, -raw[e].w);
+            const uint64_t ul = mul_f32x2(l2[e], bf16x2_to_f32x2(wl[e])), uh = mul_f32x2(h2[e], bf16x2_to_f32x2(wh[e]));
+            const uint64_t tl = fma_f32x2(ul, cs, mul_f32x2(uh, nsn)), th = fma_f32x2(uh, cs, mul_f32x2(ul, sn));
             float y0, y1;
             unpack_f32x2(mul_f32x2(tl, inv2), y0, y1);
             yl[e] = pack_bf16x2(y0, y1);
@@ -565,10 +559,8 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     // branch under elect.sync the instruction stream of an MMA is shorter than under a lane == 0 test
     // (measured on the head_dim-512 kernel: a quarter less time per step with the tensor pipe free-running).
     if (p.ap_vectors != 0u) {
-      // This warp, idle until Q is there, publishes the softmax warps' shares of the append, so that none of them waits
+      // This warp, idle until Q is there, publishes the softmax warps' shares of the append, so that none of those waits
       // for its stores to reach L2: at the barrier that opens a share all stores of the one before have been issued.
-      const uint32_t groups = append_unit_groups(p.Hkv, p.ap_unit_heads), n_units = p.ap_vectors / p.Hkv * groups;
-      const uint32_t n_shares = append_share_count(p.ap_vectors / (2u * p.Hkv), p.Hkv, p.ap_unit_heads);
       uint32_t done = 0;      // vectors of the share in hand
       for (uint32_t it = 0;; ++it) {
         append_sync();
@@ -577,10 +569,10 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
           __threadfence();
           atomicAdd(p.ap_ctl + 1, done);
         }
-        if (share >= n_shares) break;
-        const uint32_t u = share * SM_WARPS + lane, h0 = (u % groups) * p.ap_unit_heads;
+        if (share >= ap_shares) break;
+        const uint32_t u = share * SM_WARPS + lane, h0 = (u % ap_groups) * p.ap_unit_heads;
         const uint32_t nh = p.Hkv - h0 < p.ap_unit_heads ? p.Hkv - h0 : p.ap_unit_heads;
-        done = __reduce_add_sync(0xffffffffu, lane < SM_WARPS && u < n_units ? nh : 0u);
+        done = __reduce_add_sync(0xffffffffu, lane < SM_WARPS && u < ap_units ? 2u * nh : 0u);
       }
     }
     if (n_local > 0 && is_leader) {
@@ -905,8 +897,60 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     const uint8_t* recv = smem + OFF_Q;                                      // [cs][rpc] rows; this CTA's own place stays empty
     const uint8_t* own_rows = smem + OFF_STAGE + rank * rpc * ROW_BYTES;     // [rpc] rows
     auto part = [&](uint32_t s2, uint32_t rl) { return (s2 == rank ? own_rows : recv + s2 * rpc * ROW_BYTES) + rl * ROW_BYTES; };
-    // A warp merges four rows at a time (lane = eight columns), every lane reading the cs (m, l)
-    // pairs itself: no shuffles and four independent chains, because this pass is bound by latency
+    if (n_groups == 1u) {
+      // The usual end: a warp takes two rows at a time (lane = eight columns), every lane reading the cs (m, l) pairs
+      // itself.  Small on purpose: the code runs once per launch.
+      const uint32_t n_warps = THREADS / 32;
+      for (uint32_t rl0 = warp * 2u; rl0 < rpc; rl0 += n_warps * 2u) {
+        float mg[2] = {-INFINITY, -INFINITY}, lg[2] = {0.f, 0.f};
+        uint64_t acc[2][4] = {};
+#pragma unroll 1
+        for (uint32_t s2 = 0; s2 < cs; ++s2)
+#pragma unroll
+          for (uint32_t k = 0; k < 2; ++k) mg[k] = fmaxf(mg[k], *reinterpret_cast<const float*>(part(s2, rl0 + k) + HD * 2u));
+#pragma unroll 1
+        for (uint32_t s2 = 0; s2 < cs; ++s2)
+#pragma unroll
+          for (uint32_t k = 0; k < 2; ++k) {
+            const float4 ml = *reinterpret_cast<const float4*>(part(s2, rl0 + k) + HD * 2u);
+            const uint4 x = *reinterpret_cast<const uint4*>(part(s2, rl0 + k) + lane * 16u);
+            const float w = (ml.x == -INFINITY) ? 0.f : fast_exp2(ml.x - mg[k]);
+            lg[k] += w * ml.y;
+            const uint64_t ws = pack_f32x2(w * ml.z, w * ml.z);   // the row's scale folded into its weight
+            const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 f = unpack_f16x2(xs[e]);
+              acc[k][e] = fma_f32x2(ws, pack_f32x2(f.x, f.y), acc[k][e]);
+            }
+          }
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+          const uint32_t R = mt * BM + rank * rpc + rl0 + k;
+          if (R >= rows_per_head) continue;
+          const size_t orow = size_t(R / p.G) * p.Hq + kvh * p.G + R % p.G;
+          float a[8];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) unpack_f32x2(acc[k][e], a[2 * e], a[2 * e + 1]);
+          if (p.out) {
+            const float inv = lg[k] > 0.f ? 1.0f / lg[k] : 0.f;
+            *reinterpret_cast<uint4*>(p.out + orow * HD + lane * 8) =
+                make_uint4(pack_bf16x2(a[0] * inv, a[1] * inv), pack_bf16x2(a[2] * inv, a[3] * inv), pack_bf16x2(a[4] * inv, a[5] * inv),
+                           pack_bf16x2(a[6] * inv, a[7] * inv));
+          } else {
+            float4* dst = reinterpret_cast<float4*>(p.out_o + orow * HD + lane * 8);
+            dst[0] = make_float4(a[0], a[1], a[2], a[3]);
+            dst[1] = make_float4(a[4], a[5], a[6], a[7]);
+            if (lane == 0) {
+              p.out_m[orow] = mg[k] * 0.6931471805599453f;
+              p.out_l[orow] = lg[k];
+            }
+          }
+        }
+      }
+    } else {
+    // With a second level a warp merges four rows at a time: no shuffles and four independent chains, because this pass
+    // is bound by latency
     constexpr uint32_t RK1 = 4;
     for (uint32_t rl0 = warp * RK1; rl0 < rpc; rl0 += (THREADS / 32) * RK1) {
       float mg[RK1], lg[RK1], acc[RK1][8];
@@ -942,7 +986,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
         const uint32_t Rc = live[k] ? R : mt * BM;
         orow[k] = size_t(Rc / p.G) * p.Hq + kvh * p.G + Rc % p.G;
       }
-      if (n_groups > 1) {
+      {
         // Level 2, per warp: the group's merged rows (un-normalised, relative to mg) go to the
         // workspace, the warp counts itself in on the arrival counter of these four rows, and the
         // warp of the LAST group to arrive folds the other groups' rows into the ones it still holds
@@ -1023,6 +1067,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
         }
       }
     }
+  }
   }
   if (n_groups > 1 && cs == 1) {
     // ---------------------------------------------------------------- splits without clusters

@@ -211,16 +211,16 @@ struct AttnParams {
   __nv_bfloat16* ap_cache_v;
   uint32_t* ap_ctl;              // {next share, vectors done, CTAs finished}: zero between launches
   uint32_t ap_vectors;
-  uint32_t ap_unit_heads;        // heads of one token's K or V that a warp takes at a time (1, 2 or 4)
+  uint32_t ap_unit_heads;        // heads of one token whose K and V a warp takes at a time (1, 2 or 4)
   uint32_t ap_v_norm;
   uint32_t ap_write_end;         // positions >= this are not stored (0xffffffff: none)
 };
 
-// Shares of the in-launch append: one unit (unit_heads heads of one token's K or V) for each of a CTA's 16 softmax warps.
-constexpr uint32_t kAppendShareUnits = 16;
+// Shares of the in-launch append: one unit (K and V of unit_heads heads of one token) for each of a CTA's 16 softmax warps.
+constexpr uint32_t kAppendShareUnits = 16, kAppendUnitHeads = 4;
 __host__ __device__ inline uint32_t append_unit_groups(uint32_t Hkv, uint32_t unit_heads) { return (Hkv + unit_heads - 1u) / unit_heads; }
 __host__ __device__ inline uint32_t append_share_count(uint32_t n_tok, uint32_t Hkv, uint32_t unit_heads) {
-  return (n_tok * 2u * append_unit_groups(Hkv, unit_heads) + kAppendShareUnits - 1u) / kAppendShareUnits;
+  return (n_tok * append_unit_groups(Hkv, unit_heads) + kAppendShareUnits - 1u) / kAppendShareUnits;
 }
 
 // Up to kMaxBatchLaunch independent canvases served by ONE launch of the head_dim-256 tensor kernel
