@@ -227,123 +227,113 @@ dg_gemm_sm100_kernel(const GemmParams g, const __grid_constant__ CUtensorMap tm_
   }
 }
 
-// Row-wise kernels: one block of 256 threads per row, a thread holds up to ROW_VEC 8-element vectors of the row in
-// registers, so the row crosses memory once.
-constexpr uint32_t ROW_VEC = 4;        // rows of up to 256 * 4 * 8 = 8192 elements
+// Row-wise kernels: one block per row, one 8-element vector per thread (rows of up to 8,192 elements): the row crosses
+// memory once, every load of the block is in flight at once, and there is no loop: at 256 rows these kernels last a few
+// microseconds, bound by one memory round trip and by fetching their code (a block of 256 threads with four unrolled
+// vectors each: 60.8 us for the attention block of a sliding layer, 58.4 us with these).
+constexpr uint32_t ROW_THREADS = 1024;
+static uint32_t row_block(uint32_t dim) { return (dim / 8u + 31u) / 32u * 32u; }
 
-__device__ __forceinline__ float block_sum_256(float acc, float* red) {
+// sum over the block, the same bits in every thread
+__device__ __forceinline__ float block_sum(float acc, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  const uint32_t lane = threadIdx.x & 31u, n_warps = blockDim.x >> 5;
+  if (lane == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  float t = 0.f;
+  float t = lane < n_warps ? red[lane] : 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) t += red[i];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   return t;
 }
+__device__ __forceinline__ float lo_f32(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi_f32(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // y[row] = bf16(x[row] * rsqrt(mean(x[row]^2) + 1e-6) * w)
 // (rms_norm_rows_tiled.metal:16-78: f32 sum of squares, v * inv, then * weight).
-__global__ void __launch_bounds__(256) dg_rmsnorm_rows_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y,
-                                                              uint32_t dim) {
-  __shared__ float red[8];
+__global__ void __launch_bounds__(ROW_THREADS) dg_rmsnorm_rows_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y,
+                                                                      uint32_t dim) {
+  __shared__ float red[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const uint32_t n_vec = dim / 8;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(blockIdx.x) * dim);
-  uint4 v[ROW_VEC];
+  const uint32_t i = threadIdx.x;
+  const bool live = i < dim / 8u;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const uint4 v = live ? reinterpret_cast<const uint4*>(x + size_t(blockIdx.x) * dim)[i] : zero;
+  const uint4 w4 = live && w != nullptr ? reinterpret_cast<const uint4*>(w)[i] : zero;
+  const uint32_t xs[4] = {v.x, v.y, v.z, v.w}, ws[4] = {w4.x, w4.y, w4.z, w4.w};
   float acc = 0.f;
 #pragma unroll
-  for (uint32_t j = 0; j < ROW_VEC; ++j) {
-    const uint32_t i = threadIdx.x + j * 256u;
-    v[j] = i < n_vec ? xr[i] : make_uint4(0u, 0u, 0u, 0u);
-    const uint32_t ws[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-#pragma unroll
-    for (uint32_t e = 0; e < 4; ++e) {
-      const float lo = __uint_as_float(ws[e] << 16), hi = __uint_as_float(ws[e] & 0xffff0000u);
-      acc = fmaf(lo, lo, acc);
-      acc = fmaf(hi, hi, acc);
-    }
+  for (uint32_t e = 0; e < 4; ++e) {
+    acc = fmaf(lo_f32(xs[e]), lo_f32(xs[e]), acc);
+    acc = fmaf(hi_f32(xs[e]), hi_f32(xs[e]), acc);
   }
-  const float inv = rsqrtf(block_sum_256(acc, red) / float(dim) + 1e-6f);
-  uint4* yr = reinterpret_cast<uint4*>(y + size_t(blockIdx.x) * dim);
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
+  const float inv = rsqrtf(block_sum(acc, red) / float(dim) + 1e-6f);
+  if (!live) return;
+  uint32_t o[4];
 #pragma unroll
-  for (uint32_t j = 0; j < ROW_VEC; ++j) {
-    const uint32_t i = threadIdx.x + j * 256u;
-    if (i >= n_vec) continue;
-    const uint4 w4 = w != nullptr ? wr[i] : make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
-    const uint32_t xs[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, ws[4] = {w4.x, w4.y, w4.z, w4.w};
-    uint32_t o[4];
-#pragma unroll
-    for (uint32_t e = 0; e < 4; ++e) {
-      float lo = __uint_as_float(xs[e] << 16) * inv, hi = __uint_as_float(xs[e] & 0xffff0000u) * inv;
-      if (w != nullptr) {
-        lo *= __uint_as_float(ws[e] << 16);
-        hi *= __uint_as_float(ws[e] & 0xffff0000u);
-      }
-      o[e] = pack_bf16x2(lo, hi);
+  for (uint32_t e = 0; e < 4; ++e) {
+    float lo = lo_f32(xs[e]) * inv, hi = hi_f32(xs[e]) * inv;
+    if (w != nullptr) {
+      lo *= lo_f32(ws[e]);
+      hi *= hi_f32(ws[e]);
     }
-    yr[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    o[e] = pack_bf16x2(lo, hi);
   }
+  reinterpret_cast<uint4*>(y + size_t(blockIdx.x) * dim)[i] = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // out[row] = bf16(hidden[row] + bf16(t[row] * inv * w)) with t[row] = bf16(sum over the n_part fp32 partial planes of
 // the output projection), inv = rsqrt(mean(t[row]^2) + 1e-6)
 // (enc.rs:888-911: the projection stored to the bf16 arena, its RMS norm in place, then the residual add).
 // The planes are added in a fixed order: same bits every run.
-__global__ void __launch_bounds__(256) dg_norm_residual_kernel(const float* part, uint32_t n_part, size_t plane,
-                                                               const __nv_bfloat16* w, const __nv_bfloat16* hidden,
-                                                               __nv_bfloat16* out, uint32_t dim) {
-  __shared__ float red[8];
+__global__ void __launch_bounds__(ROW_THREADS) dg_norm_residual_kernel(const float* part, uint32_t n_part, size_t plane,
+                                                                       const __nv_bfloat16* w, const __nv_bfloat16* hidden,
+                                                                       __nv_bfloat16* out, uint32_t dim) {
+  __shared__ float red[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const uint32_t n_vec = dim / 8;
-  float t[ROW_VEC][8];
+  const uint32_t i = threadIdx.x;
+  const bool live = i < dim / 8u;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const uint4 h4 = live ? reinterpret_cast<const uint4*>(hidden + size_t(blockIdx.x) * dim)[i] : zero;
+  const uint4 w4 = live && w != nullptr ? reinterpret_cast<const uint4*>(w)[i] : zero;
+  float4 a[4], b[4];          // the planes (at most four slices of the contraction), all requested together
+#pragma unroll
+  for (uint32_t s = 0; s < 4; ++s) {
+    const float4* pr = reinterpret_cast<const float4*>(part + s * plane + size_t(blockIdx.x) * dim) + 2 * i;
+    const bool has = live && s < n_part;
+    a[s] = has ? pr[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+    b[s] = has ? pr[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float t[8] = {a[0].x, a[0].y, a[0].z, a[0].w, b[0].x, b[0].y, b[0].z, b[0].w};
+#pragma unroll
+  for (uint32_t s = 1; s < 4; ++s) {
+    t[0] += a[s].x; t[1] += a[s].y; t[2] += a[s].z; t[3] += a[s].w;
+    t[4] += b[s].x; t[5] += b[s].y; t[6] += b[s].z; t[7] += b[s].w;
+  }
   float acc = 0.f;
 #pragma unroll
-  for (uint32_t j = 0; j < ROW_VEC; ++j) {
-    const uint32_t i = threadIdx.x + j * 256u;
-#pragma unroll
-    for (uint32_t e = 0; e < 8; ++e) t[j][e] = 0.f;
-    if (i >= n_vec) continue;
-    for (uint32_t s = 0; s < n_part; ++s) {
-      const float4* pr = reinterpret_cast<const float4*>(part + s * plane + size_t(blockIdx.x) * dim) + 2 * i;
-      const float4 a = pr[0], b = pr[1];
-      t[j][0] += a.x; t[j][1] += a.y; t[j][2] += a.z; t[j][3] += a.w;
-      t[j][4] += b.x; t[j][5] += b.y; t[j][6] += b.z; t[j][7] += b.w;
-    }
-#pragma unroll
-    for (uint32_t e = 0; e < 8; ++e) {
-      t[j][e] = __bfloat162float(__float2bfloat16(t[j][e]));      // the projection as stored
-      acc = fmaf(t[j][e], t[j][e], acc);
-    }
+  for (uint32_t e = 0; e < 8; ++e) {
+    t[e] = __bfloat162float(__float2bfloat16(t[e]));      // the projection as stored
+    acc = fmaf(t[e], t[e], acc);
   }
-  const float inv = rsqrtf(block_sum_256(acc, red) / float(dim) + 1e-6f);
-  const uint4* hr = reinterpret_cast<const uint4*>(hidden + size_t(blockIdx.x) * dim);
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
-  uint4* orow = reinterpret_cast<uint4*>(out + size_t(blockIdx.x) * dim);
+  const float inv = rsqrtf(block_sum(acc, red) / float(dim) + 1e-6f);
+  if (!live) return;
+  const uint32_t hs[4] = {h4.x, h4.y, h4.z, h4.w}, ws[4] = {w4.x, w4.y, w4.z, w4.w};
+  uint32_t o[4];
 #pragma unroll
-  for (uint32_t j = 0; j < ROW_VEC; ++j) {
-    const uint32_t i = threadIdx.x + j * 256u;
-    if (i >= n_vec) continue;
-    const uint4 h4 = hr[i];
-    const uint4 w4 = w != nullptr ? wr[i] : make_uint4(0u, 0u, 0u, 0u);
-    const uint32_t hs[4] = {h4.x, h4.y, h4.z, h4.w}, ws[4] = {w4.x, w4.y, w4.z, w4.w};
-    uint32_t o[4];
-#pragma unroll
-    for (uint32_t e = 0; e < 4; ++e) {
-      float lo = t[j][2 * e] * inv, hi = t[j][2 * e + 1] * inv;
-      if (w != nullptr) {
-        lo *= __uint_as_float(ws[e] << 16);
-        hi *= __uint_as_float(ws[e] & 0xffff0000u);
-      }
-      lo = __bfloat162float(__float2bfloat16(lo));               // the normed projection as stored
-      hi = __bfloat162float(__float2bfloat16(hi));
-      o[e] = pack_bf16x2(__uint_as_float(hs[e] << 16) + lo, __uint_as_float(hs[e] & 0xffff0000u) + hi);
+  for (uint32_t e = 0; e < 4; ++e) {
+    float lo = t[2 * e] * inv, hi = t[2 * e + 1] * inv;
+    if (w != nullptr) {
+      lo *= lo_f32(ws[e]);
+      hi *= hi_f32(ws[e]);
     }
-    orow[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    lo = __bfloat162float(__float2bfloat16(lo));               // the normed projection as stored
+    hi = __bfloat162float(__float2bfloat16(hi));
+    o[e] = pack_bf16x2(lo_f32(hs[e]) + lo, hi_f32(hs[e]) + hi);
   }
+  reinterpret_cast<uint4*>(out + size_t(blockIdx.x) * dim)[i] = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 cudaError_t sm100_gemm_configure() {
@@ -414,7 +404,7 @@ cudaError_t launch_gemm_sm100_pair(const GemmParams& g, const CUtensorMap& tm_a,
 cudaError_t launch_rmsnorm_rows(const void* x, const void* w, void* y, uint32_t rows, uint32_t dim, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  pdl_cfg(cfg, attr, dim3(rows), dim3(256), 0, st);
+  pdl_cfg(cfg, attr, dim3(rows), dim3(row_block(dim)), 0, st);
   return cudaLaunchKernelEx(&cfg, dg_rmsnorm_rows_kernel, static_cast<const __nv_bfloat16*>(x),
                             static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y), dim);
 }
@@ -423,7 +413,7 @@ cudaError_t launch_norm_residual(const float* part, uint32_t n_part, const void*
                                  uint32_t rows, uint32_t dim, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
-  pdl_cfg(cfg, attr, dim3(rows), dim3(256), 0, st);
+  pdl_cfg(cfg, attr, dim3(rows), dim3(row_block(dim)), 0, st);
   return cudaLaunchKernelEx(&cfg, dg_norm_residual_kernel, part, n_part, size_t(rows) * dim,
                             static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(hidden),
                             static_cast<__nv_bfloat16*>(out), dim);
