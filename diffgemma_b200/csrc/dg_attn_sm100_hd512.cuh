@@ -44,37 +44,45 @@ __host__ __device__ inline TileSched tile_sched64(const MaskParams& mk, uint32_t
 // Copies a query tile into the CTA: elements [0, 256) of every row into tensor memory (by the threads with
 // half == 0), elements [256, 512) into the K-major 128-byte-swizzled shared-memory atoms at q_smem (half == 1).
 // Thread (smw, lane) owns row r = smw * 32 + lane; the caller signals the barrier afterwards.
+// One memory round trip for the shared-memory half (every copy in flight, a warp per row), two for the other
+// (64 registers): with 4 or 8 loads in flight per thread the tile took 5 us.
 __device__ __forceinline__ void copy_q_tile(const AttnParams& p, uint8_t* q_smem, uint32_t tmem, uint32_t kvh, uint32_t mt,
                                             uint32_t smw, uint32_t lane, uint32_t half) {
-  const uint32_t r = smw * 32 + lane;
-  const uint32_t R = mt * BM + r;
-  const bool valid = R < p.C * p.G;
-  const uint32_t i = valid ? R / p.G : 0u;
-  const uint32_t h = kvh * p.G + (valid ? R % p.G : 0u);
-  const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t(i) * p.Hq + h) * HDQ);
+  const uint32_t rows_per_head = p.C * p.G;
   if (half == 0) {
+    const uint32_t R = mt * BM + smw * 32 + lane;
+    const bool valid = R < rows_per_head;
+    const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t(valid ? R / p.G : 0u) * p.Hq + kvh * p.G + (valid ? R % p.G : 0u)) * HDQ);
     // 16-byte chunk c = columns [4c, 4c + 4) of lane r, so that the 16 elements of contraction step kk sit in
     // columns [8 kk, 8 kk + 8) (the layout P uses)
     const uint32_t t_row = tmem + ((smw * 32u) << 16) + T_Q;
 #pragma unroll 1
-    for (uint32_t g8 = 0; g8 < 4; ++g8) {
-      uint32_t w[32];
+    for (uint32_t g16 = 0; g16 < 2; ++g16) {
+      uint32_t w[2][32];
 #pragma unroll
-      for (uint32_t j = 0; j < 8; ++j) {
-        const uint4 v4 = valid ? src[g8 * 8 + j] : make_uint4(0u, 0u, 0u, 0u);
-        w[4 * j] = v4.x; w[4 * j + 1] = v4.y; w[4 * j + 2] = v4.z; w[4 * j + 3] = v4.w;
+      for (uint32_t j = 0; j < 16; ++j) {
+        const uint4 v4 = valid ? src[g16 * 16 + j] : make_uint4(0u, 0u, 0u, 0u);
+        uint32_t* d = &w[j >> 3][4 * (j & 7u)];
+        d[0] = v4.x; d[1] = v4.y; d[2] = v4.z; d[3] = v4.w;
       }
-      tmem_st32(t_row + g8 * 32u, w);
+      tmem_st32(t_row + g16 * 64u, w[0]);
+      tmem_st32(t_row + g16 * 64u + 32u, w[1]);
     }
     tmem_wait_st();
     tc_fence_before();
   } else {
-    // atom = 64-element column block, 16-byte chunk index XOR (row & 7)
+    // lane = 16-byte chunk of the row's second half; atom = 64-element column block, chunk index XOR (row & 7)
+    const uint32_t R0 = mt * BM + smw * 32;
+    uint32_t i = R0 / p.G, g = R0 % p.G;
+    uint8_t* dst = q_smem + (lane >> 3) * Q_ATOM + smw * 32u * 128u;
 #pragma unroll 4
-    for (uint32_t j = 0; j < 32; ++j) {
-      const uint4 v4 = valid ? src[32 + j] : make_uint4(0u, 0u, 0u, 0u);
-      *reinterpret_cast<uint4*>(q_smem + (j >> 3) * Q_ATOM + r * 128u + (((j & 7u) ^ (r & 7u)) << 4)) = v4;
+    for (uint32_t k = 0; k < 32; ++k) {
+      const bool valid = R0 + k < rows_per_head;   // warp-uniform; rows past the end are zero-filled
+      const __nv_bfloat16* src = valid ? p.q + (size_t(i) * p.Hq + kvh * p.G + g) * HDQ + 256u + lane * 8u : p.q;
+      cp_async_16(smem_u32(dst + k * 128u + (((lane & 7u) ^ (k & 7u)) << 4)), src, valid ? 16u : 0u);
+      if (++g == p.G) { g = 0; ++i; }
     }
+    cp_async_wait_all();
     fence_proxy_async_smem();
   }
 }
@@ -176,46 +184,75 @@ __device__ __forceinline__ void merge_splits_last(const AttnParams& p, volatile 
   __syncthreads();
   if (!*is_last) return;
   __threadfence();
+  // A warp merges four rows at a time: what bounds this tail is the round trip to L2, so the (m, l) pairs of the four
+  // rows are requested together, then their partial rows of every split pair after pair.
   const float2* ml_all = reinterpret_cast<const float2*>(p.ws_ml);
-  for (uint32_t rr = warp; rr < BM; rr += n_threads / 32) {
-    const uint32_t R = mt * BM + rr;
-    if (R >= rows_per_head) break;
-    const size_t orow = size_t(R / p.G) * p.Hq + kvh * p.G + R % p.G;
-    float2 ml = make_float2(-INFINITY, 0.f);
-    if (lane < S) ml = ml_all[(size_t(lane) * 2 + dh) * rows_total + orow];
-    float mg = ml.x;
+  constexpr uint32_t RK = 4;
+  for (uint32_t r0 = warp * RK; r0 < BM; r0 += n_threads / 32 * RK) {
+    size_t orow[RK];
+    bool live[RK];
+    float2 ml[RK];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-    const float w_mine = (ml.x == -INFINITY) ? 0.f : fast_exp2(ml.x - mg);
-    float lg = w_mine * ml.y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
-    float acc[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-    for (uint32_t s = 0; s < S; ++s) {
-      const float w = __shfl_sync(0xffffffffu, w_mine, int(s));
-      const float4* src = reinterpret_cast<const float4*>(p.ws_o + (size_t(s) * rows_total + orow) * HDQ + dh * HDV + lane * 8);
-      const float4 a = src[0], bq = src[1];
-      acc[0] += w * a.x; acc[1] += w * a.y; acc[2] += w * a.z; acc[3] += w * a.w;
-      acc[4] += w * bq.x; acc[5] += w * bq.y; acc[6] += w * bq.z; acc[7] += w * bq.w;
+    for (uint32_t k = 0; k < RK; ++k) {
+      const uint32_t R = mt * BM + r0 + k;
+      live[k] = R < rows_per_head;
+      const uint32_t Rc = live[k] ? R : mt * BM;
+      orow[k] = size_t(Rc / p.G) * p.Hq + kvh * p.G + Rc % p.G;
+      ml[k] = lane < S ? ml_all[(size_t(lane) * 2 + dh) * rows_total + orow[k]] : make_float2(-INFINITY, 0.f);
     }
-    const size_t off = orow * HDQ + dh * HDV + lane * 8;
-    if (p.out) {
-      const float inv = lg > 0.f ? 1.0f / lg : 0.f;
-      uint4 w4;
-      w4.x = pack_bf16x2(acc[0] * inv, acc[1] * inv);
-      w4.y = pack_bf16x2(acc[2] * inv, acc[3] * inv);
-      w4.z = pack_bf16x2(acc[4] * inv, acc[5] * inv);
-      w4.w = pack_bf16x2(acc[6] * inv, acc[7] * inv);
-      *reinterpret_cast<uint4*>(p.out + off) = w4;
-    } else {
-      float4* dst = reinterpret_cast<float4*>(p.out_o + off);
-      dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-      dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-      if (lane == 0 && dh == 0) {
-        p.out_m[orow] = mg * 0.6931471805599453f;
-        p.out_l[orow] = lg;
+    float w_mine[RK], mg[RK], lg[RK], acc[RK][8];
+#pragma unroll
+    for (uint32_t k = 0; k < RK; ++k) {
+      mg[k] = ml[k].x;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mg[k] = fmaxf(mg[k], __shfl_xor_sync(0xffffffffu, mg[k], o));
+      w_mine[k] = (ml[k].x == -INFINITY) ? 0.f : fast_exp2(ml[k].x - mg[k]);
+      lg[k] = w_mine[k] * ml[k].y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) lg[k] += __shfl_xor_sync(0xffffffffu, lg[k], o);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[k][e] = 0.f;
+    }
+    for (uint32_t s0 = 0; s0 < S; s0 += 2) {
+      float4 a[RK][2], bq[RK][2];
+#pragma unroll
+      for (uint32_t k = 0; k < RK; ++k)
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j) {
+          const uint32_t s = s0 + j < S ? s0 + j : S - 1u;   // clamped; its weight is zeroed below
+          const float4* src = reinterpret_cast<const float4*>(p.ws_o + (size_t(s) * rows_total + orow[k]) * HDQ + dh * HDV + lane * 8);
+          a[k][j] = src[0];
+          bq[k][j] = src[1];
+        }
+#pragma unroll
+      for (uint32_t j = 0; j < 2; ++j)
+#pragma unroll
+        for (uint32_t k = 0; k < RK; ++k) {
+          const float w = s0 + j < S ? __shfl_sync(0xffffffffu, w_mine[k], int(s0 + j)) : 0.f;
+          acc[k][0] += w * a[k][j].x; acc[k][1] += w * a[k][j].y; acc[k][2] += w * a[k][j].z; acc[k][3] += w * a[k][j].w;
+          acc[k][4] += w * bq[k][j].x; acc[k][5] += w * bq[k][j].y; acc[k][6] += w * bq[k][j].z; acc[k][7] += w * bq[k][j].w;
+        }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < RK; ++k) {
+      if (!live[k]) continue;
+      const size_t off = orow[k] * HDQ + dh * HDV + lane * 8;
+      if (p.out) {
+        const float inv = lg[k] > 0.f ? 1.0f / lg[k] : 0.f;
+        uint4 w4;
+        w4.x = pack_bf16x2(acc[k][0] * inv, acc[k][1] * inv);
+        w4.y = pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv);
+        w4.z = pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv);
+        w4.w = pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv);
+        *reinterpret_cast<uint4*>(p.out + off) = w4;
+      } else {
+        float4* dst = reinterpret_cast<float4*>(p.out_o + off);
+        dst[0] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+        dst[1] = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
+        if (lane == 0 && dh == 0) {
+          p.out_m[orow[k]] = mg[k] * 0.6931471805599453f;
+          p.out_l[orow[k]] = lg[k];
+        }
       }
     }
   }
