@@ -216,7 +216,19 @@ static bool fused_q_prologue_ok(const dg_layer_desc& d) {
   return d.head_dim == 256 && d.rotary_dim == 256 && d.rope_pairing == DG_ROPE_SPLIT_HALF;
 }
 
-static uint32_t choose_splits(const dg_ctx* ctx, uint32_t q_tiles, uint32_t k_tiles) {
+// What a launch costs beside its key tiles, in tenths of a key tile's time: the fixed part of a step (launch, set-up, Q
+// prologue, output) and what exchanging and merging the partial rows of 2, 4 and 8 splits adds.
+struct SplitCost {
+  uint32_t fixed, merge[3];
+};
+// head_dim 256, a tile = 1.4 us.  32 query tiles (one canvas, 8 KV heads), us: 4 key tiles 21.3 unsplit, 20.5 with 2
+// splits, 19.1 with 4; 11 tiles 31.3 / 26.4 / 22.6; 64 query tiles: 4 key tiles 21.8 / 21.0, 11 tiles 31.7 / 27.1
+constexpr SplitCost kCost256 = {120, {14, 18, 55}};
+// splits that meet in memory: head_dim 512, under a bitmap, with the caller's workspace (a bitmap over 5 key tiles of 2 KV
+// heads: 27.9 us unsplit, 34.8 with 4 splits)
+constexpr SplitCost kCostMemory = {70, {36, 44, 55}};
+
+static uint32_t choose_splits(const dg_ctx* ctx, uint32_t q_tiles, uint32_t k_tiles, const SplitCost& cost_of) {
   uint32_t smax = k_tiles < kSm100MaxSplits ? k_tiles : kSm100MaxSplits;
   if (smax < 1) smax = 1;
   if (ctx->forced_splits) return ctx->forced_splits < smax ? ctx->forced_splits : smax;
@@ -224,20 +236,25 @@ static uint32_t choose_splits(const dg_ctx* ctx, uint32_t q_tiles, uint32_t k_ti
   uint32_t best = 1;
   uint64_t best_cost = ~0ull;
   // automatic choice: powers of two up to 8, the split counts that merge inside a cluster
-  for (uint32_t s = 1; s <= smax && s <= 8u; s *= 2) {
+  for (uint32_t s = 1, i = 0; s <= smax && s <= 8u; s *= 2, ++i) {
     const uint64_t waves = (uint64_t(q_tiles) * s + sms - 1) / sms;
-    // in tenths of a key tile's time (about 1.75 us): the fixed cost of a step (launches, set-up, Q
-    // prologue, epilogue: about 12 us) and the measured cost of exchanging and merging the partial rows
-    // of s splits (about 6.3 us for two, 7.7 us for four), so that a short key range is not split at all
-    const uint64_t merge = s == 1 ? 0 : s == 2 ? 36 : s == 4 ? 44 : 55;
-    const uint64_t per = 10 * ((k_tiles + s - 1) / s) + 70 + merge;
-    const uint64_t cost = waves * per;
+    const uint64_t cost = waves * (10 * ((k_tiles + s - 1) / s) + cost_of.fixed + (s == 1 ? 0 : cost_of.merge[i - 1]));
     if (cost < best_cost) {
       best_cost = cost;
       best = s;
     }
   }
   return best;
+}
+
+// CTA pairs halve the shared-memory traffic per query tile (the single form's limiter); they need two query tiles of one
+// KV head to share a key schedule.  Their set-up is longer, and with four splits their merge goes through the workspace:
+// there they pay from about a hundred key tiles on (2 KV heads: 100 tiles 53.6 against 52.3 us, 130 tiles 62.9 / 63.4),
+// with one split or two from eight (four canvases of a sliding layer, 11 tiles: 33.2 against 35.5 us; 8 KV heads, 34
+// tiles: 67.6 / 81.0; two canvases, 24 tiles: 34.2 / 37.5).
+static bool pair_pays(uint32_t tiles_per_head, uint32_t k_tiles, uint32_t single_splits) {
+  if (tiles_per_head < 2) return false;
+  return k_tiles >= 96 || (k_tiles >= 8 && single_splits <= 2 && tiles_per_head % 2 == 0);
 }
 
 static int32_t ensure_split_ws(dg_ctx* ctx, uint32_t splits, uint32_t rows) {
@@ -930,7 +947,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     // even number of tiles (pair mode 1 = the exchange alone, 2 = automatic)
     const bool pair5 = !fixed && c->pair_mode != 0 && !a.packed;
     const bool quad5 = pair5 && c->pair_mode == 2 && sm100_query_tiles(p.C, p.G, 1) % 2 == 0;
-    p.n_splits = choose_splits(c, q_tiles5 * 2, pair5 ? sm100_hd512x_key_steps(p.mask) : sm100_hd512_key_tiles(p.mask));
+    p.n_splits = choose_splits(c, q_tiles5 * 2, pair5 ? sm100_hd512x_key_steps(p.mask) : sm100_hd512_key_tiles(p.mask), kCostMemory);
     p.cluster_splits = 1;
     if (fixed) {
       // as many splits as the fixed arrays hold: [splits][rows][512] partial O, [2 splits][rows] (m, l) pairs
@@ -962,16 +979,15 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     c->last_launches += 1;
     return DG_OK;
   }
-  // CTA pairs halve the shared-memory traffic per query tile (the kernel's limiter); they need two
-  // query tiles of one KV head to share a key schedule, so a head with a single tile runs unpaired
-  // Short key ranges stay unpaired too: the pair form's longer set-up and its workspace merge cost
-  // more than the per-tile saving returns below about a hundred key tiles.
   const uint32_t tiles_per_head = sm100_query_tiles(p.C, p.G, 1);
   const uint32_t k_tiles = sm100_key_tiles(p.mask);
-  const bool pair = !fixed && !a.packed && (c->pair_mode == 1 || (c->pair_mode == 2 && tiles_per_head >= 2 && k_tiles >= 96));
-  const uint32_t q_tiles = pair ? sm100_pair_query_tiles(p.C, p.G, p.Hkv) : sm100_query_tiles(p.C, p.G, p.Hkv);
+  const uint32_t single_tiles = sm100_query_tiles(p.C, p.G, p.Hkv);
+  const SplitCost& cost = fixed || a.packed ? kCostMemory : kCost256;
+  const uint32_t single_splits = choose_splits(c, single_tiles * c->concurrent, k_tiles, cost);
+  const bool pair = !fixed && !a.packed && (c->pair_mode == 1 || (c->pair_mode == 2 && pair_pays(tiles_per_head, k_tiles, single_splits)));
+  const uint32_t q_tiles = pair ? sm100_pair_query_tiles(p.C, p.G, p.Hkv) : single_tiles;
   if (q_tiles > (fixed ? fixed->n_counters : kMaxQueryTiles)) return fail(DG_ERR_UNSUPPORTED, "too many query tiles");
-  p.n_splits = choose_splits(c, q_tiles * c->concurrent, k_tiles);
+  p.n_splits = pair ? choose_splits(c, q_tiles * c->concurrent, k_tiles, cost) : single_splits;
   // Split merge: consecutive splits of a query tile form a thread-block cluster and merge through
   // shared memory; what is left meets in the workspace.  Clusters stay at 4 CTAs in the pair form
   // (2 x 2): too few clusters of 8 are co-resident on the device.
@@ -1178,12 +1194,13 @@ extern "C" int32_t dg_attn_denoise(dg_ctx* c, const dg_layer_desc* d, dg_kv* con
       k_min = kt < k_min ? kt : k_min;
       k_max = kt > k_max ? kt : k_max;
     }
-    const bool pair_lo = c->pair_mode == 1 || (c->pair_mode == 2 && tph >= 2 && k_min >= 96);
-    const bool pair_hi = c->pair_mode == 1 || (c->pair_mode == 2 && tph >= 2 && k_max >= 96);
+    const uint32_t single_splits = choose_splits(c, sm100_query_tiles(d->canvas, G, d->n_kv_heads) * batch, k_max, kCost256);
+    const bool pair_lo = c->pair_mode == 1 || (c->pair_mode == 2 && pair_pays(tph, k_min, single_splits));
+    const bool pair_hi = c->pair_mode == 1 || (c->pair_mode == 2 && pair_pays(tph, k_max, single_splits));
     conc_pair = pair_lo;
     const uint32_t q_tiles = conc_pair ? sm100_pair_query_tiles(d->canvas, G, d->n_kv_heads)
                                        : sm100_query_tiles(d->canvas, G, d->n_kv_heads);
-    conc_splits = choose_splits(c, q_tiles * batch, k_max);
+    conc_splits = choose_splits(c, q_tiles * batch, k_max, kCost256);
     const bool no_ws = conc_splits == 1 || (conc_pair ? conc_splits == 2 : (conc_splits == 2 || conc_splits == 4 || conc_splits == 8));
     concurrent = pair_lo == pair_hi && no_ws && conc_splits <= k_min;
   }
