@@ -1003,11 +1003,11 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     p.ws_o = fixed->o;
     p.ws_ml = fixed->ml;
     p.ws_counters = fixed->counters;
-  } else if (p.n_splits % 2 == 0 && !a.packed) {   // under a bitmap the splits meet as fp32 in the workspace
+  } else if (p.n_splits % 2 == 0) {
     if (pair) p.cluster_splits = 2;
     else if (p.n_splits == 2 || p.n_splits == 4 || p.n_splits == 8) p.cluster_splits = p.n_splits;
   }
-  if (!fixed && p.n_splits / p.cluster_splits > 1) {
+  if (!fixed && (p.n_splits / p.cluster_splits > 1 || (a.packed && p.n_splits > 1))) {   // a bitmap's splits meet there as fp32
     const int32_t r = ensure_split_ws(c, p.n_splits, p.C * p.Hq);
     if (r != DG_OK) return r;
     p.ws_o = c->ws_o;

@@ -186,7 +186,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     }
     mbar_init(bar_addr(bar_base, B_O_FINAL), 1);
     mbar_init(bar_addr(bar_base, B_RX), 1);
-    if (cs > 1) mbar_expect_tx(bar_addr(bar_base, B_RX), (cs - 1u) * (BM / cs) * ROW_BYTES);
+    if (!BITS && cs > 1) mbar_expect_tx(bar_addr(bar_base, B_RX), (cs - 1u) * (BM / cs) * ROW_BYTES);
     ctl[1] = 0u;
     ctl[2] = 0u;
     fence_mbar_init();
@@ -711,7 +711,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
 #pragma unroll
     for (uint32_t k = 0; k < NTR; ++k) l_tot += xch_l[r * NTR + k];
     const bool direct = (p.n_splits == 1);
-    const bool via_dsmem = cs > 1;
+    const bool via_dsmem = !BITS && cs > 1;
     if (via_dsmem) {
       // The partial stays on chip.  Row r of the query tile is merged by CTA r / (BM / S) of the cluster.  Every CTA
       // lays its un-normalised rows out in its own (dead) K/V region, [BM] rows of ROW_BYTES: the row as fp16 with
@@ -854,7 +854,8 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   // CTA's MMAs are complete once its softmax warps have seen O_FINAL, and this barrier collects that, and the staged
   // rows of this CTA, from everybody.
   stamp(p, 13);
-  if (cs > 1) {
+  if (BITS && cs > 1) cluster_sync_all();   // the fp32 partial rows of all splits are in the workspace
+  if (!BITS && cs > 1) {
     cluster_sync_all();
     const uint32_t rank = PAIR ? (crank >> 1) : crank, rpc = BM / cs;
     if (tid < cs && tid != rank) {
@@ -886,7 +887,57 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   }
 
   // ------------------------------------------------------------------ split merge, level 1: inside the cluster
-  if (cs > 1) {
+  if (BITS && cs > 1) {
+    // Under a bitmap partial rows stay fp32 and are too large for shared memory on both sides: they meet in the workspace,
+    // but the cluster still shares the merge, CTA k the rows [k*BM/cs, (k+1)*BM/cs), two rows per warp at a time.
+    // 4,096 rows x 2,304 keys, 4 splits: 41.9 us when the last CTA to arrive merged all rows, 34.4 so.
+    const uint32_t rpc = BM / cs;
+    for (uint32_t rl0 = warp * 2u; rl0 < rpc; rl0 += (THREADS / 32) * 2u) {
+      size_t orow[2];
+      bool live_row[2];
+      float2 ml[2];
+#pragma unroll
+      for (uint32_t k = 0; k < 2; ++k) {
+        const uint32_t R = mt * BM + crank * rpc + rl0 + k;
+        live_row[k] = R < rows_per_head;
+        const uint32_t Rc = live_row[k] ? R : 0u;
+        orow[k] = size_t(Rc / p.G) * p.Hq + kvh * p.G + Rc % p.G;
+        ml[k] = lane < cs ? __ldcg(reinterpret_cast<const float2*>(p.ws_ml) + size_t(lane) * rows_total + orow[k]) : make_float2(-INFINITY, 0.f);
+      }
+      float w_mine[2], mg[2], lg[2], acc[2][8] = {};
+#pragma unroll
+      for (uint32_t k = 0; k < 2; ++k) {
+        mg[k] = ml[k].x;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) mg[k] = fmaxf(mg[k], __shfl_xor_sync(0xffffffffu, mg[k], o));
+        mg[k] = __shfl_sync(0xffffffffu, mg[k], 0);
+        w_mine[k] = (ml[k].x == -INFINITY) ? 0.f : fast_exp2(ml[k].x - mg[k]);
+        lg[k] = w_mine[k] * ml[k].y;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) lg[k] += __shfl_xor_sync(0xffffffffu, lg[k], o);
+        lg[k] = __shfl_sync(0xffffffffu, lg[k], 0);
+      }
+#pragma unroll 2
+      for (uint32_t s2 = 0; s2 < cs; ++s2)
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+          const float w = __shfl_sync(0xffffffffu, w_mine[k], int(s2));
+          const float4* src = reinterpret_cast<const float4*>(p.ws_o + (size_t(s2) * rows_total + orow[k]) * HD + lane * 8);
+          const float4 a = __ldcg(src), b4 = __ldcg(src + 1);
+          acc[k][0] += w * a.x; acc[k][1] += w * a.y; acc[k][2] += w * a.z; acc[k][3] += w * a.w;
+          acc[k][4] += w * b4.x; acc[k][5] += w * b4.y; acc[k][6] += w * b4.z; acc[k][7] += w * b4.w;
+        }
+#pragma unroll
+      for (uint32_t k = 0; k < 2; ++k) {
+        if (!live_row[k]) continue;
+        const float inv = lg[k] > 0.f ? 1.0f / lg[k] : 0.f;
+        *reinterpret_cast<uint4*>(p.out + orow[k] * HD + lane * 8) =
+            make_uint4(pack_bf16x2(acc[k][0] * inv, acc[k][1] * inv), pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv),
+                       pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv), pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv));
+      }
+    }
+  }
+  if (!BITS && cs > 1) {
     // The cs CTAs that hold consecutive splits of this query tile are one thread-block cluster
     // (cluster dims (1, cs, 1), pair form (2, cs, 1)).  CTA k merges rows [k*BM/cs, (k+1)*BM/cs): its own partial where
     // it was staged, the others' where their copies land.
@@ -1246,7 +1297,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   }
   stamp(p, 5);
   // the copies out of this CTA's shared memory have all landed once every CTA of the cluster is through its merge
-  if (cs > 1) cluster_sync_all();
+  if (!BITS && cs > 1) cluster_sync_all();
   if (p.ap_vectors != 0u && tid == 0) {
     // every CTA is past its own share taking and its waits on the append counters by now; the last one to
     // get here puts the share counter and the done counter back to zero for the next launch
