@@ -13,8 +13,8 @@
 //      lowest indices among what equals it;
 //   4. softmax over the kept scores, and the gather of V, a warp per kept key.
 // Lists that outgrow shared memory (many equal scores, clustered ones) take the same steps over the groups in memory.
-// Bound: the gather (4,096 rows x 258 keys x 1 KB = 1.08 GB out of L2 at head_dim 512): 180 us of 372 for the whole call at
-// 33,024 keys.  With bf16 scores, two histograms over all of a row and the exact scores of the kept keys computed again
+// Bound: the gather (4,096 rows x 258 keys x 1 KB = 1.08 GB out of L2 at head_dim 512): 175 us of 349 for the whole call at
+// 33,024 keys, 6.7 TB/s into the SMs.  With bf16 scores, two histograms over all of a row and the exact scores of the kept keys computed again
 // from K (another 1.08 GB gathered) the call took 900 us.
 #include <cuda.h>
 
@@ -72,7 +72,7 @@ __device__ __forceinline__ uint32_t warp_excl_sum(uint32_t v, uint32_t lane, uin
   return incl - v;
 }
 
-__global__ void __launch_bounds__(tk::THREADS, 4) dg_topk_select_pv_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(tk::THREADS, 5) dg_topk_select_pv_kernel(const TopkParams p) {
   using namespace tk;
   __shared__ TopkRadix rad;
   // listed groups, then the winners in index order with their scores (later probabilities)
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(tk::THREADS, 4) dg_topk_select_pv_kernel(const
   const uint4* gmax = reinterpret_cast<const uint4*>(p.gmax + size_t(blockIdx.x) * n_groups);       // eight groups per load
   // 16 keys of group g of this row: float4 (g * 128 + (q >> 1) * 64 + (q & 1)), q = 0..3
   const uint4* row = reinterpret_cast<const uint4*>(p.scores) + (size_t(blockIdx.x / 32u) * n_groups * 512u + (blockIdx.x % 32u) * 8u) / 4u;
-  auto quad = [&](uint32_t g, uint32_t q) { return row[size_t(g) * 128u + (q >> 1) * 64u + (q & 1u)]; };
+  auto quad = [&](uint32_t g, uint32_t q) { return __ldcs(&row[size_t(g) * 128u + (q >> 1) * 64u + (q & 1u)]); };
   auto okey = [](uint32_t bits) { return score_order_key(__uint_as_float(bits)); };
   const uint32_t n_g8 = n_groups / 8u;
 

@@ -8,7 +8,8 @@
 // equal contiguous runs, one per pair, so the last wave is full whatever the key count.
 //
 // Bound: writing the scores.  4,096 rows x 33,024 keys are 541 MB of fp32 against 61 (head_dim 512) or 31 us (256) of
-// MMA work: 150 us in two passes at head_dim 512 (3.6 TB/s of plane).  So the plane is laid out for the writer: 32 rows of 8 keys are one contiguous KB, which a warp (lane = row)
+// MMA work: 150 us in two passes at head_dim 512 (3.6 TB/s of plane, 4.2 TB/s of DRAM traffic; smaller passes that would
+// stay in L2 lose more to their launches: 372 us for the call with 288 MB, 418 with 144, 462 with 72).  So the plane is laid out for the writer: 32 rows of 8 keys are one contiguous KB, which a warp (lane = row)
 // stores with one 32-byte access per lane.  A group of 16 keys of a row is then two whole 32-byte sectors, and the
 // selection reads only the groups whose maximum can matter, about one in eight.
 #include <cuda.h>
@@ -22,14 +23,17 @@ using namespace sm100;
 
 namespace ts {
 constexpr uint32_t TM = 128, TN = 256, BK = 64;
-constexpr uint32_t THREADS = 192;                 // loader, MMA issuer, four epilogue warps
+constexpr uint32_t THREADS = 320;                 // loader, MMA issuer, eight epilogue warps
 constexpr uint32_t ATOM = TM * BK * 2;            // 16 KB: 64 elements of 128 query rows, or of this CTA's 128 keys
 __host__ __device__ constexpr uint32_t stages(uint32_t D) { return D == 512 ? 6u : 8u; }
 __host__ __device__ constexpr uint32_t smem_bytes(uint32_t D) { return (D / BK + stages(D)) * ATOM + 256 + 1024; }
 }  // namespace ts
 
+// A pass of the plane is larger than L2 and one group in eight of it is read, once: marked evict-first it leaves L2 to K,
+// which every row pair reads, and to V (33,024 keys, head_dim 512: 368 us for the call without the mark, 357 with it, 349
+// with the selection's reads of the plane marked as well).
 __device__ __forceinline__ void st_global_v8(void* dst, const uint32_t* v) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+  asm volatile("st.global.L2::evict_first.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
@@ -71,7 +75,7 @@ dg_topk_scores_kernel(const TopkParams p, const __grid_constant__ CUtensorMap tm
     mbar_init(bar_addr(bar_base, B_Q_EMPTY), 1);
     for (uint32_t b = 0; b < 2; ++b) {
       mbar_init(bar_addr(bar_base, B_ACC + b), 1);
-      mbar_init(bar_addr(bar_base, B_ACC_EMPTY + b), 8);   // four epilogue warps of each CTA (the leader's copy is used)
+      mbar_init(bar_addr(bar_base, B_ACC_EMPTY + b), 16);   // eight epilogue warps of each CTA (the leader's copy is used)
     }
     ctl[1] = 0u;
     fence_mbar_init();
@@ -176,7 +180,9 @@ dg_topk_scores_kernel(const TopkParams p, const __grid_constant__ CUtensorMap tm
     }
   } else {
     // ---------------------------------------------------------------- epilogue: lane = one query row
-    const uint32_t q4 = warp & 3u;                        // the 32 TMEM lanes this warp may read
+    // Two warps per 32 rows, 128 of the tile's keys each, 32 at a time with the next 32 on their way out of tensor memory.
+    const uint32_t q4 = warp & 3u, half = warp >= 6u ? 1u : 0u;      // the 32 TMEM lanes this warp may read; which keys
+    constexpr uint32_t NC = TN / 64;                                   // blocks of 32 keys per warp
     const uint32_t rows_per_head = p.C * p.G;
     const MaskParams mk = p.mask;
     for (uint32_t u = u0, n = 0; u < u1; ++u, ++n) {
@@ -185,20 +191,32 @@ dg_topk_scores_kernel(const TopkParams p, const __grid_constant__ CUtensorMap tm
       const uint32_t i_row = R < rows_per_head ? R / p.G : p.C - 1u;
       const RowVis rv = mask_row(mk, i_row);
       const size_t rb = size_t(rp - p.rp0) * 8u + xi * 4u + q4;      // 32-row block of the plane
-      float* plane = p.scores + (rb * p.n_groups + kt * 16u) * 512u + lane * 8u;
+      const uint32_t g0 = kt * 16u + half * 8u;                        // first group of 16 keys
+      float* plane = p.scores + (rb * p.n_groups + g0) * 512u + lane * 8u;
+      const uint32_t t_src = tmem + ((q4 * 32u) << 16) + (n & 1u) * TN + half * 128u;
+      const bool stored = R0 < rows_per_head;      // warp-uniform: blocks past the last row have no place in the selection
       if (!__all_sync(0xffffffffu, mbar_wait(bar_addr(bar_base, B_ACC + (n & 1u)), (n >> 1) & 1u, abort_flag))) break;
       tc_fence_after();
-      uint32_t gm[8];
-#pragma unroll 1
-      for (uint32_t c = 0; c < TN / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tmem + ((q4 * 32u) << 16) + (n & 1u) * TN + c * 32u, v);
+      uint32_t gm[NC], v[2][32];
+      tmem_ld32(t_src, v[0]);
+#pragma unroll
+      for (uint32_t c = 0; c < NC; ++c) {
+        uint32_t(&x)[32] = v[c & 1u];
         tmem_wait_ld();
-        const uint32_t k0 = kt * TN + c * 32u;
+        if (c + 1 < NC) {
+          tmem_ld32(t_src + (c + 1) * 32u, v[(c + 1) & 1u]);
+        } else {
+          // this warp's part of the accumulator is in registers
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(lead_bar(B_ACC_EMPTY + (n & 1u)));
+        }
+        const uint32_t k0 = g0 * 16u + c * 32u;
         if (!mask_range_full(mk, rv, k0, 32u)) {
+          const uint32_t seen = mask_bits16(mk, rv, k0) | (mask_bits16(mk, rv, k0 + 16u) << 16);
 #pragma unroll
           for (uint32_t e = 0; e < 32; ++e)
-            if (!mask_visible_row(mk, rv, k0 + e)) v[e] = 0xff800000u;   // -inf
+            if (!((seen >> e) & 1u)) x[e] = 0xff800000u;   // -inf
         }
         uint32_t key[2];
 #pragma unroll
@@ -206,24 +224,19 @@ dg_topk_scores_kernel(const TopkParams p, const __grid_constant__ CUtensorMap tm
           float m[3];
 #pragma unroll
           for (uint32_t e = 0; e < 3; ++e)
-            m[e] = max3_nan(__uint_as_float(v[h * 16 + e * 5]), __uint_as_float(v[h * 16 + e * 5 + 1]),
-                            max3_nan(__uint_as_float(v[h * 16 + e * 5 + 2]), __uint_as_float(v[h * 16 + e * 5 + 3]),
-                                     __uint_as_float(v[h * 16 + e * 5 + 4])));
-          const float mx = max3_nan(m[0], m[1], max3_nan(m[2], __uint_as_float(v[h * 16 + 15]), __uint_as_float(v[h * 16 + 15])));
+            m[e] = max3_nan(__uint_as_float(x[h * 16 + e * 5]), __uint_as_float(x[h * 16 + e * 5 + 1]),
+                            max3_nan(__uint_as_float(x[h * 16 + e * 5 + 2]), __uint_as_float(x[h * 16 + e * 5 + 3]),
+                                     __uint_as_float(x[h * 16 + e * 5 + 4])));
+          const float mx = max3_nan(m[0], m[1], max3_nan(m[2], __uint_as_float(x[h * 16 + 15]), __uint_as_float(x[h * 16 + 15])));
           key[h] = score_order_key(mx) >> 16;
         }
+        gm[c] = key[0] | (key[1] << 16);
+        if (stored) {
 #pragma unroll
-        for (uint32_t j = 0; j < 8; ++j)
-          if (c == j) gm[j] = key[0] | (key[1] << 16);
-        if (R0 < rows_per_head) {      // warp-uniform: blocks past the last row have no place in the selection
-#pragma unroll
-          for (uint32_t j = 0; j < 4; ++j) st_global_v8(plane + (c * 4u + j) * 256u, &v[j * 8]);
+          for (uint32_t j = 0; j < 4; ++j) st_global_v8(plane + (c * 4u + j) * 256u, &x[j * 8]);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_remote(lead_bar(B_ACC_EMPTY + (n & 1u)));
-      if (R0 < rows_per_head) st_global_v8(p.gmax + (rb * 32u + lane) * p.n_groups + kt * 16u, gm);
+      if (stored) *reinterpret_cast<uint4*>(p.gmax + (rb * 32u + lane) * p.n_groups + g0) = make_uint4(gm[0], gm[1], gm[2], gm[3]);
     }
   }
 
