@@ -1,8 +1,8 @@
 // Denoise-step canvas attention for head_dim 256 on sm_100a: one fused flash-style kernel.
 //
-//   * Q prologue in the kernel: per-head RMSNorm(+weight) + split-half RoPE on the CTA's 128
-//     query rows, rounded to bf16 and written straight into the UMMA shared-memory layout (one warp
-//     per row, the raw rows copied asynchronously into place before the set-up barrier).
+//   * canvas append (where it runs in the launch), then the Q prologue: per-head RMSNorm(+weight) + split-half RoPE on the
+//     CTA's 128 query rows, rounded to bf16 and written straight into the UMMA shared-memory layout (half a warp
+//     per row, the raw rows copied asynchronously into place ahead of the append).
 //   * K/V tiles of 128 keys are TMA-staged (3-D tiled loads, 128-byte swizzle, no multicast) from
 //     the head-major bf16 cache K[Hkv][cap][256], V[Hkv][cap][256]; a ring cache (sliding layers) keeps
 //     key position t in slot t & ring_mask, and because the ring is a multiple of 128 slots a key
@@ -18,9 +18,9 @@
 //     Q 64 KB + K 64 KB + V 64 KB as MMA operands and takes 128 KB of TMA writes = 320 KB against
 //     128 B/clk = 2,560 cycles, the MMAs alone need 2,048); the pair form moves 192 KB per tile.
 //   * intra-GPU split-KV: grid.y CTAs share one query tile.  Consecutive splits form a thread-block
-//     cluster (2 / 4 / 8 in the single-CTA form, 2 pairs in the pair form): every CTA pushes its partial
-//     rows into the shared memory of the CTA that owns them - as fp16 with a power-of-two scale per
-//     row, because an SM moves only about 16 B/clk into another SM - and merges the rows it owns.
+//     cluster (2 / 4 / 8 in the single-CTA form, 2 pairs in the pair form): every CTA stages its partial rows in its own
+//     shared memory - as fp16 with a power-of-two scale per row, half the bytes - and one bulk copy per owner
+//     moves them to the CTA that merges them.
 //     Groups that are left meet in a global workspace, per warp: the warp of the last group to
 //     arrive at a four-row counter folds the others into the rows it still holds.  Split counts
 //     that form no cluster write whole partials to the workspace and the last CTA to arrive merges.
