@@ -78,6 +78,7 @@ class Context:
             # torch owns the stream (so that nothing torch remembers about it can outlive it); the
             # context is told to launch on it
             torch.cuda.set_device(device)
+            self._previous_stream = torch.cuda.current_stream(device)
             self.torch_stream = torch.cuda.Stream(device=device)
             check(self.lib.dg_ctx_set_stream(self.h, C.c_void_p(self.torch_stream.cuda_stream)), "dg_ctx_set_stream")
             torch.cuda.set_stream(self.torch_stream)
@@ -129,9 +130,11 @@ class Context:
             for dep in list(self._dependents):
                 dep.close()
             if self._made_current:
-                # hand torch its default stream back before the context's stream is destroyed
+                # hand torch the stream back that was current before this context, unless it has moved on to another
+                # (a later context's, on which that one's uploads and launches are ordered)
                 torch.cuda.synchronize(self.device)
-                torch.cuda.set_stream(torch.cuda.default_stream(self.device))
+                if torch.cuda.current_stream(self.device) == self.torch_stream:
+                    torch.cuda.set_stream(self._previous_stream)
             self.lib.dg_ctx_destroy(self.h)
             self.h = None
 
