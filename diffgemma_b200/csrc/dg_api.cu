@@ -1048,6 +1048,14 @@ static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
   return DG_OK;
 }
 
+// May a bitmap call take the tensor kernels?  They move whole 16-byte vectors, and its entry point also takes tensors off
+// 16-byte boundaries: those go to the general kernel, which reads and writes element by element.
+static bool bitmap_on_tensor(const AttnCall& a, const void* q, const void* k, const void* v, const void* qw, const void* kw) {
+  for (const void* p : {q, k, v, qw, kw, static_cast<const void*>(a.out)})
+    if (!aligned16(p)) return false;
+  return true;
+}
+
 // one canvas: stage 1 on K/V (+ table), then stage 2 with the fused Q prologue
 static int32_t denoise_one(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, uint32_t kv_len, const void* q,
                            const void* k, const void* v, const void* qw, const void* kw, const uint8_t* attend,
@@ -1058,7 +1066,8 @@ static int32_t denoise_one(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, uint32_
   // leaves nothing queued (a split-KV group then stays in step with its peers)
   r = check_ring_span(kv, make_mask(d, kv_len, a.t0, a.t1, a.include_canvas), d.canvas);
   if (r != DG_OK) return r;
-  const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general;
+  const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general &&
+                      (attend == nullptr || bitmap_on_tensor(a, q, k, v, qw, kw));
   // A bitmap is packed for the tensor kernels on every geometry they have: the packing reads it once (about 3 us for
   // 256 x 2,304), the CUDA-core kernel that other head_dims use visits keys one by one
   if (tensor && attend != nullptr) {

@@ -288,12 +288,15 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append
   }
 }
 
-static bool append_rows_ok(const AppendParams& p, const RopeParams& rp) {
-  if ((p.D != 256 && p.D != 512) || rp.rot_half % 8 != 0 || rp.pair_off % 8 != 0) return false;
+// tensors off 16-byte boundaries go to the general kernel, which reads element by element
+static bool append_aligned(const AppendParams& p) {
   const void* ptrs[] = {p.q_in, p.q_out, p.k_in, p.k_out, p.v_in, p.v_out, p.qw, p.kw};
   for (const void* q : ptrs)
-    if (reinterpret_cast<uintptr_t>(q) & 15u) return false;   // the general kernel reads element by element
+    if (reinterpret_cast<uintptr_t>(q) & 15u) return false;
   return true;
+}
+static bool append_rows_ok(const AppendParams& p, const RopeParams& rp) {
+  return (p.D == 256 || p.D == 512) && rp.rot_half % 8 == 0 && rp.pair_off % 8 == 0 && append_aligned(p);
 }
 
 void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st, bool early) {
@@ -308,7 +311,7 @@ void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st,
   cfg.attrs = attr;
   cfg.numAttrs = early ? 1 : 0;
   if (p.rope_table_in && !p.rope_table && !p.q_in && !p.k_out && !p.v_out && p.D == 256 && rp.rot_half == 128 &&
-      rp.pair_off == 128) {
+      rp.pair_off == 128 && append_aligned(p)) {
     const uint32_t warps = p.n * 2u * p.Hkv;
     cfg.gridDim = dim3((warps + 7u) / 8u);
     cfg.blockDim = dim3(256);

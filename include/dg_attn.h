@@ -254,8 +254,8 @@ int32_t dg_host_pipe_destroy(dg_host_pipe* pipe);
  * the caches and weights of a submitted step must stay valid until it has been waited for.                        */
 int32_t dg_host_pipe_set_deferred_launch(dg_host_pipe* pipe, int32_t on);
 /* General decoder bitmap (reference DecoderAttnMask, src/model/mask.rs:4-27): attend is a
- * device pointer to uint8 [C][kv_len+C], 1 = visible.  head_dim 256 / 512: packed to bits,
- * then the tensor kernels; other head_dims: the general kernel.                                  */
+ * device pointer to uint8 [C][kv_len+C], 1 = visible.  head_dim 256 / 512 with every tensor on a
+ * 16-byte boundary: packed to bits, then the tensor kernels; otherwise the general kernel.       */
 int32_t dg_attn_denoise_bitmap(dg_ctx* ctx, const dg_layer_desc* desc, dg_kv* kv, uint32_t kv_len,
                                const void* q, const void* k, const void* v, const void* qw, const void* kw,
                                const uint8_t* attend, void* out);

@@ -1,0 +1,69 @@
+"""Decoder-bitmap calls at the edges of what the tensor kernels take: whatever they cannot take has to come out as the
+general kernel computes it."""
+import numpy as np
+import pytest
+import torch
+
+from diffgemma_b200 import capi
+from diffgemma_b200.step_attn import AttnLayer, KvCache
+from tests import util
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _layer(hd, canvas, **more):
+    if hd == 512:
+        return AttnLayer(n_kv_heads=2, head_dim=512, canvas=canvas, rotary_dim=128, rope_theta=1e6, v_norm=1,
+                         rope_pairing=capi.ROPE_PROPORTIONAL, **more)
+    return AttnLayer(n_kv_heads=2, canvas=canvas, rope_theta=1e6, **more)
+
+
+def _case(hd, P, canvas, seed, **more):
+    case = util.make_case(_layer(hd, canvas, **more), P, seed=seed, weights=True)
+    seen = np.random.default_rng(seed).random((canvas, P + canvas)) < 0.6
+    args = [util.dev(case, n) for n in ("q", "kc", "vc")] + [torch.from_numpy(seen.astype(np.uint8)).to(DEV)]
+    return case, seen, args + [util.dev(case, "qw"), util.dev(case, "kw")]
+
+
+def _general(ctx, att, kv, P, args):
+    try:
+        ctx.force_general(True)
+        return att.denoise_bitmap(kv, P, *args).clone()
+    finally:
+        ctx.force_general(False)
+
+
+def _off_by_one(t):
+    """The same values two bytes past a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+    out = buf[1:].view(t.shape)
+    out.copy_(t)
+    assert out.data_ptr() % 16 == 2
+    return out
+
+
+@pytest.mark.parametrize("hd", [256, 512])
+@pytest.mark.parametrize("which", ["q", "k", "v", "qw", "kw", "out"])
+def test_tensors_off_16_byte_boundaries(ctx, hd, which):
+    P, canvas = 300, 40
+    case, _, args = _case(hd, P, canvas, seed=hd + 1)
+    kv, att = util.gpu_setup(ctx, case)
+    want = _general(ctx, att, kv, P, args)
+    cache = [t.clone() for t in kv.read(0, P + canvas)]
+    kv.close()
+    kv, att = util.gpu_setup(ctx, case)
+    out = torch.empty_like(args[0])
+    at = {"q": 0, "k": 1, "v": 2, "qw": 4, "kw": 5}
+    if which == "out":
+        out = _off_by_one(out)
+    else:
+        args[at[which]] = _off_by_one(args[at[which]])
+    for step in range(2):       # the second step finds the positions' RoPE table in memory
+        out.fill_(7.0)
+        att.denoise_bitmap(kv, P, *args, out=out)
+        ctx.synchronize()
+        assert torch.equal(out, want), f"step {step}"
+        for got, ref in zip(kv.read(0, P + canvas), cache):
+            assert torch.equal(got, ref)
+    kv.close()
