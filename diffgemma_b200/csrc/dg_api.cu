@@ -868,6 +868,13 @@ struct FixedWs {
   uint32_t n_counters = 0;
 };
 
+static int32_t bitmap_fix(dg_ctx* c, const AttnParams& p) {
+  const cudaError_t e = launch_bitmap_fix(p, launch_stream(c));
+  if (e != cudaSuccess) return fail_cuda(e, "launch_bitmap_fix");
+  c->last_launches += 1;
+  return DG_OK;
+}
+
 static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const AttnCall& a,
                             const FixedWs* fixed = nullptr) {
   AttnParams p;
@@ -977,7 +984,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
       c->ev_used += 2;
     }
     c->last_launches += 1;
-    return DG_OK;
+    return a.packed ? bitmap_fix(c, p) : DG_OK;
   }
   const uint32_t tiles_per_head = sm100_query_tiles(p.C, p.G, 1);
   const uint32_t k_tiles = sm100_key_tiles(p.mask);
@@ -1039,7 +1046,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     c->ev_used += 2;
   }
   c->last_launches += 1;
-  return DG_OK;
+  return a.packed ? bitmap_fix(c, p) : DG_OK;
 }
 
 static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
@@ -1049,11 +1056,15 @@ static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
 }
 
 // May a bitmap call take the tensor kernels?  They move whole 16-byte vectors, and its entry point also takes tensors off
-// 16-byte boundaries: those go to the general kernel, which reads and writes element by element.
-static bool bitmap_on_tensor(const AttnCall& a, const void* q, const void* k, const void* v, const void* qw, const void* kw) {
+// 16-byte boundaries: those go to the general kernel, which reads and writes element by element.  So does an output that
+// lies over the queries: rows that come out non-finite are computed again from those (launch_bitmap_fix).
+static bool bitmap_on_tensor(const dg_layer_desc& d, const AttnCall& a, const void* q, const void* k, const void* v, const void* qw,
+                             const void* kw) {
   for (const void* p : {q, k, v, qw, kw, static_cast<const void*>(a.out)})
     if (!aligned16(p)) return false;
-  return true;
+  const size_t bytes = size_t(d.canvas) * d.n_q_heads * d.head_dim * 2;
+  const uintptr_t qa = reinterpret_cast<uintptr_t>(q), oa = reinterpret_cast<uintptr_t>(a.out);
+  return qa + bytes <= oa || oa + bytes <= qa;
 }
 
 // one canvas: stage 1 on K/V (+ table), then stage 2 with the fused Q prologue
@@ -1067,7 +1078,7 @@ static int32_t denoise_one(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, uint32_
   r = check_ring_span(kv, make_mask(d, kv_len, a.t0, a.t1, a.include_canvas), d.canvas);
   if (r != DG_OK) return r;
   const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general &&
-                      (attend == nullptr || bitmap_on_tensor(a, q, k, v, qw, kw));
+                      (attend == nullptr || bitmap_on_tensor(d, a, q, k, v, qw, kw));
   // A bitmap is packed for the tensor kernels on every geometry they have: the packing reads it once (about 3 us for
   // 256 x 2,304), the CUDA-core kernel that other head_dims use visits keys one by one
   if (tensor && attend != nullptr) {

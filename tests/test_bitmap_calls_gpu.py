@@ -67,3 +67,63 @@ def test_tensors_off_16_byte_boundaries(ctx, hd, which):
         for got, ref in zip(kv.read(0, P + canvas), cache):
             assert torch.equal(got, ref)
     kv.close()
+
+
+@pytest.mark.parametrize("hd,P,canvas,splits", [(256, 300, 40, 0), (256, 1500, 100, 4), (256, 700, 256, 1), (256, 700, 33, 3),
+                                                (512, 200, 17, 0), (512, 900, 100, 3)])
+@pytest.mark.parametrize("bad", ["padding", "holes", "canvas", "visible"])
+def test_keys_without_numbers(ctx, hd, P, canvas, splits, bad):
+    """Infinite and NaN keys and values behind zero bits: hidden from all rows, or from some of them.  A row that sees none
+    of them is the same as over finite keys (against the general kernel one bf16 step, 2^-7 of a value, and what the order of
+    the sums leaves near zero); one that does is what the general kernel makes of it."""
+    case, seen, args = _case(hd, P, canvas, seed=hd + P)
+    if bad == "padding":
+        where = np.arange(0, 130)               # a dead tile and the head of a live one
+    elif bad == "canvas":
+        where = P + np.arange(0, canvas, 5)
+    else:
+        where = np.array([3, 131, 140, P - 1])
+    if bad == "visible":
+        seen[:, where] = False
+        seen[1::3, where[1]] = True
+    else:
+        seen[:, where] = False
+    args[3] = torch.from_numpy(seen.astype(np.uint8)).to(DEV)
+    kinds = torch.tensor([float("nan"), float("inf"), float("-inf")], dtype=torch.bfloat16, device=DEV)
+    kv, att = util.gpu_setup(ctx, case)
+    clean = _general(ctx, att, kv, P, args)
+    if bad == "canvas":
+        for j, t in enumerate(where):
+            args[2][int(t) - P] = kinds[j % 3]
+    else:
+        k, v = case["kp"].to(DEV), case["vp"].to(DEV)
+        for j, t in enumerate(where):
+            v[int(t)] = kinds[j % 3]
+            if bad != "visible":
+                k[int(t), :, ::2] = kinds[(j + 1) % 3]
+        kv.load_prefix(k, v, 0)
+    want = _general(ctx, att, kv, P, args)
+    blind = torch.from_numpy(~seen[:, where].any(axis=1)).to(DEV)
+    assert torch.equal(want[blind], clean[blind])
+    try:
+        ctx.set_splits(splits)
+        for _ in range(2):
+            got = att.denoise_bitmap(kv, P, *args)
+            ctx.synchronize()
+            torch.testing.assert_close(got.float(), want.float(), rtol=2.0 ** -7, atol=2e-3, equal_nan=True)
+    finally:
+        ctx.set_splits(0)
+    assert ctx.device_status()[0] == 0
+    kv.close()
+
+
+@pytest.mark.parametrize("hd", [256, 512])
+def test_output_over_the_queries(ctx, hd):
+    P, canvas = 300, 40
+    case, _, args = _case(hd, P, canvas, seed=hd + 2)
+    kv, att = util.gpu_setup(ctx, case)
+    want = _general(ctx, att, kv, P, args)
+    att.denoise_bitmap(kv, P, *args, out=args[0])
+    ctx.synchronize()
+    assert torch.equal(args[0], want)
+    kv.close()
