@@ -105,7 +105,8 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   const uint32_t sQ = smem_base + OFF_Q, sK = smem_base + OFF_K, sV = smem_base + OFF_V;
   const uint32_t bar_base = smem_base + OFF_BAR;
   volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR + B_COUNT * 8);
-  // ctl[0] = TMEM base address, ctl[1] = abort flag, ctl[2] = "this CTA merges" flag
+  // ctl[0] = TMEM base address, ctl[1] = abort flag, ctl[2] = "this CTA merges" flag, ctl[3], ctl[4] = append shares,
+  // ctl[5] = the wait for the cluster's rows gave up
   float* xch_max = reinterpret_cast<float*>(smem + OFF_XCH);   // [2 tile parities][BM][NTR]
   float* xch_misc = xch_max + 2 * BM * NTR;                     // [BM][NTR]: row maxima of |O| for the fp16 exchange
   float* xch_l = xch_misc + BM * NTR;                           // [BM][NTR]: final softmax denominators
@@ -189,6 +190,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     if (!BITS && cs > 1) mbar_expect_tx(bar_addr(bar_base, B_RX), (cs - 1u) * (BM / cs) * ROW_BYTES);
     ctl[1] = 0u;
     ctl[2] = 0u;
+    ctl[5] = 0u;
     fence_mbar_init();
   }
   if (warp == W_MMA) {
@@ -941,7 +943,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     // The cs CTAs that hold consecutive splits of this query tile are one thread-block cluster
     // (cluster dims (1, cs, 1), pair form (2, cs, 1)).  CTA k merges rows [k*BM/cs, (k+1)*BM/cs): its own partial where
     // it was staged, the others' where their copies land.
-    __all_sync(0xffffffffu, mbar_wait_cluster(bar_addr(bar_base, B_RX), 0u, abort_flag));
+    // Every CTA of the cluster sends its rows, also one whose key loop gave up (as zeros), so this wait has a flag of its
+    // own.  Should it give up all the same, none of these rows is merged or stored, and the end of the kernel reports it.
+    const bool landed = __all_sync(0xffffffffu, mbar_wait_cluster(bar_addr(bar_base, B_RX), 0u, &ctl[5]));
     stamp(p, 14);
     const uint32_t rank = PAIR ? (crank >> 1) : crank;
     const uint32_t rpc = BM / cs;
@@ -952,7 +956,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       // The usual end: a warp takes two rows at a time (lane = eight columns), every lane reading the cs (m, l) pairs
       // itself.  Small on purpose: the code runs once per launch.
       const uint32_t n_warps = THREADS / 32;
-      for (uint32_t rl0 = warp * 2u; rl0 < rpc; rl0 += n_warps * 2u) {
+      for (uint32_t rl0 = landed ? warp * 2u : rpc; rl0 < rpc; rl0 += n_warps * 2u) {
         float mg[2] = {-INFINITY, -INFINITY}, lg[2] = {0.f, 0.f};
         uint64_t acc[2][4] = {};
 #pragma unroll 1
@@ -1033,7 +1037,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
 #pragma unroll
       for (uint32_t k = 0; k < RK1; ++k) {
         const uint32_t R = mt * BM + rank * rpc + rl0 + k;
-        live[k] = rl0 + k < rpc && R < rows_per_head;
+        live[k] = landed && rl0 + k < rpc && R < rows_per_head;
         const uint32_t Rc = live[k] ? R : mt * BM;
         orow[k] = size_t(Rc / p.G) * p.Hq + kvh * p.G + Rc % p.G;
       }
@@ -1297,7 +1301,15 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   }
   stamp(p, 5);
   // the copies out of this CTA's shared memory have all landed once every CTA of the cluster is through its merge
-  if (!BITS && cs > 1) cluster_sync_all();
+  if (!BITS && cs > 1) {
+    if (lane == 0 && ctl[5]) {   // rows that did not come: report it, and give the copies time before the cluster leaves
+      dev_status_set(p.status, DG_DEV_WAIT_TIMEOUT, KID_SM100, blockIdx.x + gridDim.x * blockIdx.y, n_local);
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000ll) {}
+    }
+    __syncwarp();
+    cluster_sync_all();
+  }
   if (p.ap_vectors != 0u && tid == 0) {
     // every CTA is past its own share taking and its waits on the append counters by now; the last one to
     // get here puts the share counter and the done counter back to zero for the next launch
