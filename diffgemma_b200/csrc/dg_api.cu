@@ -57,7 +57,8 @@ struct dg_ctx {
   uint32_t* counters = nullptr;        // [kCounterSlots], zero between launches
   float* ws_o = nullptr;               // split partials
   float* ws_ml = nullptr;
-  size_t ws_splits = 0, ws_rows = 0;   // capacity of ws_o / ws_ml: splits x rows (x 256 / x 2)
+  size_t ws_rows = 0;                  // capacity of ws_o / ws_ml: splits * rows (x 256 / x 2)
+  std::vector<void*> outgrown;         // scratch that has been replaced by a larger buffer (grow_scratch)
   __nv_bfloat16* stage_q = nullptr;    // device staging for host-buffer calls / pre-normed Q
   __nv_bfloat16* stage_k = nullptr;
   __nv_bfloat16* stage_v = nullptr;
@@ -257,58 +258,48 @@ static bool pair_pays(uint32_t tiles_per_head, uint32_t k_tiles, uint32_t single
   return k_tiles >= 96 || (k_tiles >= 8 && single_splits <= 2 && tiles_per_head % 2 == 0);
 }
 
+// Scratch of the attention calls grows without a synchronisation and without freeing: a CUDA graph may hold the address of
+// the buffer in use, work may be queued on it, and the stream may be under capture (the driver then allows the allocation
+// only in the relaxed mode).  Buffers that became too small are kept until the context goes; their successors are twice as
+// large where memory allows, so that a session that grows by a block at a time allocates rarely and all of them together
+// stay below twice the last.  Two buffers of one capacity, na and nb elements of them per unit of it.
+template <class A, class B>
+static int32_t grow_scratch(dg_ctx* ctx, A** a, size_t na, B** b, size_t nb, size_t* cap, size_t need) {
+  if (need <= *cap) return DG_OK;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  DG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  cudaError_t e = cudaSuccess;
+  for (const size_t n : {need > 2 * *cap ? need : 2 * *cap, need}) {
+    A* fa = nullptr;
+    B* fb = nullptr;
+    e = cudaMalloc(&fa, n * na * sizeof(A));
+    if (e == cudaSuccess) e = cudaMalloc(&fb, n * nb * sizeof(B));
+    if (e == cudaSuccess) {
+      if (*a) ctx->outgrown.push_back(*a);
+      if (*b) ctx->outgrown.push_back(*b);
+      *a = fa;
+      *b = fb;
+      *cap = n;
+      break;
+    }
+    cudaGetLastError();
+    cudaFree(fa);
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return e == cudaSuccess ? DG_OK : fail_cuda(e, "scratch allocation");
+}
+
 static int32_t ensure_split_ws(dg_ctx* ctx, uint32_t splits, uint32_t rows) {
-  if (splits <= ctx->ws_splits && rows <= ctx->ws_rows) return DG_OK;
-  const size_t s = splits > ctx->ws_splits ? splits : ctx->ws_splits;
-  const size_t r = rows > ctx->ws_rows ? rows : ctx->ws_rows;
-  DG_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (ctx->ws_o) cudaFree(ctx->ws_o);
-  if (ctx->ws_ml) cudaFree(ctx->ws_ml);
-  ctx->ws_o = ctx->ws_ml = nullptr;
-  ctx->ws_splits = ctx->ws_rows = 0;
-  DG_CUDA(cudaMalloc(&ctx->ws_o, s * r * 256 * sizeof(float)));
-  DG_CUDA(cudaMalloc(&ctx->ws_ml, s * r * 2 * sizeof(float)));
-  ctx->ws_splits = s;
-  ctx->ws_rows = r;
-  return DG_OK;
+  return grow_scratch(ctx, &ctx->ws_o, 256, &ctx->ws_ml, 2, &ctx->ws_rows, size_t(splits) * rows);
 }
 
 static int32_t ensure_stage(dg_ctx* ctx, size_t q_elems, size_t kv_elems) {
-  if (q_elems > ctx->stage_q_elems) {
-    DG_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (ctx->stage_q) cudaFree(ctx->stage_q);
-    if (ctx->stage_o) cudaFree(ctx->stage_o);
-    ctx->stage_q = ctx->stage_o = nullptr;
-    ctx->stage_q_elems = 0;
-    DG_CUDA(cudaMalloc(&ctx->stage_q, q_elems * 2));
-    DG_CUDA(cudaMalloc(&ctx->stage_o, q_elems * 2));
-    ctx->stage_q_elems = q_elems;
-  }
-  if (kv_elems > ctx->stage_kv_elems) {
-    DG_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (ctx->stage_k) cudaFree(ctx->stage_k);
-    if (ctx->stage_v) cudaFree(ctx->stage_v);
-    ctx->stage_k = ctx->stage_v = nullptr;
-    ctx->stage_kv_elems = 0;
-    DG_CUDA(cudaMalloc(&ctx->stage_k, kv_elems * 2));
-    DG_CUDA(cudaMalloc(&ctx->stage_v, kv_elems * 2));
-    ctx->stage_kv_elems = kv_elems;
-  }
-  return DG_OK;
+  const int32_t r = grow_scratch(ctx, &ctx->stage_q, 1, &ctx->stage_o, 1, &ctx->stage_q_elems, q_elems);
+  return r != DG_OK ? r : grow_scratch(ctx, &ctx->stage_k, 1, &ctx->stage_v, 1, &ctx->stage_kv_elems, kv_elems);
 }
 
 static int32_t ensure_bits(dg_ctx* ctx, size_t tiles) {
-  if (tiles <= ctx->bits_tiles) return DG_OK;
-  DG_CUDA(cudaStreamSynchronize(ctx->stream));
-  cudaFree(ctx->bits);
-  cudaFree(ctx->bits_live);
-  ctx->bits = nullptr;
-  ctx->bits_live = nullptr;
-  ctx->bits_tiles = 0;
-  DG_CUDA(cudaMalloc(&ctx->bits, tiles * kMaxCanvas * sizeof(uint4)));
-  DG_CUDA(cudaMalloc(&ctx->bits_live, tiles * pack_attend_runs(kMaxCanvas)));
-  ctx->bits_tiles = tiles;
-  return DG_OK;
+  return grow_scratch(ctx, &ctx->bits, kMaxCanvas, &ctx->bits_live, pack_attend_runs(kMaxCanvas), &ctx->bits_tiles, tiles);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -394,6 +385,7 @@ extern "C" int32_t dg_ctx_destroy(dg_ctx* c) {
   cudaFree(c->topk_plane);
   cudaFree(c->bits);
   cudaFree(c->bits_live);
+  for (void* p : c->outgrown) cudaFree(p);
   for (cudaEvent_t e : c->ev) cudaEventDestroy(e);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
@@ -968,7 +960,8 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
       p.ws_counters = fixed->counters;
     } else if (p.n_splits > 1) {
       const int32_t r5 = ensure_split_ws(c, 2 * p.n_splits, p.C * p.Hq);
-      if (r5 != DG_OK) return r5;
+      if (r5 != DG_OK && !a.packed) return r5;
+      if (r5 != DG_OK) p.n_splits = 1;
       p.ws_o = c->ws_o;
       p.ws_ml = c->ws_ml;
       p.ws_counters = c->counters;
@@ -1016,7 +1009,8 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
   }
   if (!fixed && (p.n_splits / p.cluster_splits > 1 || (a.packed && p.n_splits > 1))) {   // a bitmap's splits meet there as fp32
     const int32_t r = ensure_split_ws(c, p.n_splits, p.C * p.Hq);
-    if (r != DG_OK) return r;
+    if (r != DG_OK && !a.packed) return r;
+    if (r != DG_OK) p.n_splits = p.cluster_splits = 1;   // no memory for a bitmap's splits: none
     p.ws_o = c->ws_o;
     p.ws_ml = c->ws_ml;
     p.ws_counters = c->counters;
@@ -1077,18 +1071,20 @@ static int32_t denoise_one(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, uint32_
   // leaves nothing queued (a split-KV group then stays in step with its peers)
   r = check_ring_span(kv, make_mask(d, kv_len, a.t0, a.t1, a.include_canvas), d.canvas);
   if (r != DG_OK) return r;
-  const bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general &&
-                      (attend == nullptr || bitmap_on_tensor(d, a, q, k, v, qw, kw));
+  bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general && (attend == nullptr || bitmap_on_tensor(d, a, q, k, v, qw, kw));
   // A bitmap is packed for the tensor kernels on every geometry they have: the packing reads it once (about 3 us for
   // 256 x 2,304), the CUDA-core kernel that other head_dims use visits keys one by one
   if (tensor && attend != nullptr) {
     const uint32_t T = kv_len + d.canvas;
-    r = ensure_bits(c, (size_t(T) + 127) / 128);
-    if (r != DG_OK) return r;
-    const cudaError_t e = launch_pack_attend(attend, d.canvas, T, c->bits, c->bits_live, launch_stream(c));
-    if (e != cudaSuccess) return fail_cuda(e, "launch_pack_attend");
-    c->last_launches += 1;
-    a.packed = true;
+    // the general kernel needs no scratch: it serves the call where there is no memory for the packed form
+    tensor = ensure_bits(c, (size_t(T) + 127) / 128) == DG_OK &&
+             (fused_q_prologue_ok(d) || ensure_stage(c, size_t(d.canvas) * d.n_q_heads * d.head_dim, 0) == DG_OK);
+    if (tensor) {
+      const cudaError_t e = launch_pack_attend(attend, d.canvas, T, c->bits, c->bits_live, launch_stream(c));
+      if (e != cudaSuccess) return fail_cuda(e, "launch_pack_attend");
+      c->last_launches += 1;
+      a.packed = true;
+    }
   }
   if (tensor && !fused_q_prologue_ok(d)) {
     // partial / proportional rotary: run the stand-alone Q prologue into the staging buffer

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from diffgemma_b200 import capi
-from diffgemma_b200.step_attn import AttnLayer, KvCache
+from diffgemma_b200.step_attn import AttnLayer, Context, KvCache
 from tests import util
 
 pytestmark = pytest.mark.gpu
@@ -127,3 +127,39 @@ def test_output_over_the_queries(ctx, hd):
     ctx.synchronize()
     assert torch.equal(args[0], want)
     kv.close()
+
+
+@pytest.mark.parametrize("hd", [256, 512])
+def test_captured_before_any_scratch_exists(hd):
+    """A bitmap call is recorded in a context that has run nothing yet, then the scratch grows under eager calls several
+    times: the replay still works on memory of its own."""
+    ctx = Context(0)
+    P, canvas = 900, 40
+    case, seen, args = _case(hd, P, canvas, seed=hd + 3)
+    kv, att = util.gpu_setup(ctx, case)
+    out = torch.empty_like(args[0])
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=ctx.torch_stream):
+        att.denoise_bitmap(kv, P, *args, out=out)
+    others = []
+    for P2, canvas2 in ((1500, 100), (9000, 256)):
+        c2, seen2, args2 = _case(hd, P2, canvas2, seed=P2)
+        kv2, att2 = util.gpu_setup(ctx, c2)
+        for splits in (0, 8):
+            ctx.set_splits(splits)
+            got = util.t2f(att2.denoise_bitmap(kv2, P2, *args2))
+            util.assert_close(got, util.run_oracle(c2, attend=seen2), f"{P2} keys, {splits} splits")
+        ctx.set_splits(0)
+        others.append((att2, kv2, P2, args2))
+    want = util.run_oracle(case, attend=seen)
+    for att2, kv2, P2, args2 in others:
+        att2.denoise_bitmap(kv2, P2, *args2)
+        with torch.cuda.stream(ctx.torch_stream):
+            out.zero_()
+            g.replay()
+        ctx.synchronize()
+        util.assert_close(util.t2f(out), want, "replay")
+    assert ctx.device_status()[0] == 0
+    del g
+    ctx.close()
