@@ -243,6 +243,10 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   const uint32_t ap_units = p.ap_vectors != 0u ? p.ap_vectors / (2u * p.Hkv) * ap_groups : 0u;
   const uint32_t ap_shares = (ap_units + SM_WARPS - 1u) / SM_WARPS;
   static_assert(SM_WARPS == kAppendShareUnits, "one unit per softmax warp");
+  // Does a key tile hold slots that the in-launch append writes?  The canvas positions; and under a bitmap on a ring, which may
+  // show positions that the ring no longer has, what the canvas takes the place of (the mask rules never reach those).
+  const uint32_t ap_alias_end = BITS && p.ring_mask != 0xffffffffu && mk.can_hi > p.ring_mask + 1u ? mk.can_hi - (p.ring_mask + 1u) : 0u;
+  auto holds_canvas = [&](uint32_t jt) { return jt * BN + BN > mk.kv_len || (BITS && jt * BN < ap_alias_end); };
   if (warp < SM_WARPS) {
     // Two things stand between the set-up and the first score tile: this CTA's Q rows and its shares of the canvas append.
     // The append goes first, while the raw Q rows are on their way: other CTAs wait for it (those whose splits hold the
@@ -500,7 +504,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       TileWalk<BITS> walk(p, ts, live, v_begin);
       for (uint32_t n = 0; n < n_local; ++n) {
         const uint32_t jt = walk.next();
-        if (!canvas_ready && jt * BN + BN > mk.kv_len) {
+        if (!canvas_ready && holds_canvas(jt)) {
           if (!wait_counter_gpu(p.ap_ctl + 1, p.ap_vectors, abort_flag)) break;
           canvas_ready = true;
         }
@@ -531,7 +535,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       TileWalk<BITS> walk(p, ts, live, v_begin);
       for (uint32_t n = 0; n < n_local; ++n) {
         const uint32_t jt = walk.next();
-        if (!canvas_ready && jt * BN + BN > mk.kv_len) {
+        if (!canvas_ready && holds_canvas(jt)) {
           if (!wait_counter_gpu(p.ap_ctl + 1, p.ap_vectors, abort_flag)) break;
           canvas_ready = true;
         }

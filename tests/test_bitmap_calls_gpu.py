@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from diffgemma_b200 import capi
-from diffgemma_b200.step_attn import AttnLayer, Context, KvCache
+from diffgemma_b200.step_attn import AttnLayer, CanvasAttention, Context, KvCache
 from tests import util
 
 pytestmark = pytest.mark.gpu
@@ -126,6 +126,26 @@ def test_output_over_the_queries(ctx, hd):
     att.denoise_bitmap(kv, P, *args, out=args[0])
     ctx.synchronize()
     assert torch.equal(args[0], want)
+    kv.close()
+
+
+@pytest.mark.parametrize("P,canvas", [(600, 100), (2000, 256)])
+def test_ring_positions_that_are_gone(ctx, P, canvas):
+    """A bitmap on a ring may show positions that the ring no longer holds: they read what took their slots, the canvas of
+    this very step among it, in the second step too, whose append runs inside the attention launch."""
+    layer = AttnLayer(n_kv_heads=2, canvas=canvas, rope_theta=1e4, window=64, mask_mode=capi.MASK_WINDOW_UNIFORM)
+    kv = KvCache(ctx, layer, ring_slots=512)
+    att = CanvasAttention(ctx, layer)
+    g = torch.Generator(device=DEV).manual_seed(P)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)
+    kv.append(rn(P, 2, 256), rn(P, 2, 256), 0)
+    seen = (torch.rand(canvas, P + canvas, generator=g, device=DEV) < 0.5).to(torch.uint8)
+    for _ in range(3):
+        args = rn(canvas, 16, 256), rn(canvas, 2, 256), rn(canvas, 2, 256), seen
+        got = att.denoise_bitmap(kv, P, *args).clone()
+        want = _general(ctx, att, kv, P, args)
+        torch.testing.assert_close(got.float(), want.float(), rtol=2.0 ** -7, atol=2e-3)
+    assert ctx.device_status()[0] == 0
     kv.close()
 
 
