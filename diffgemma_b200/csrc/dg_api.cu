@@ -2329,7 +2329,10 @@ extern "C" int32_t dg_attn_denoise_topk(dg_ctx* c, const dg_layer_desc* d, dg_kv
   per_pass = per_pass < 1 ? 1 : per_pass > n_rp ? n_rp : per_pass;
   const uint32_t passes = (n_rp + per_pass - 1) / per_pass;
   per_pass = (n_rp + passes - 1) / passes;
-  const size_t need = per_pass * (rp_scores * 4 + rp_gmax * 2);
+  // Several passes allocate a whole plane, however much of it they use: a context that has run its longest range then never
+  // has to grow for a shorter one, whose single pass may fill more of it (and which may be under capture).
+  const size_t rp_bytes = rp_scores * 4 + rp_gmax * 2, full = kTopkPlaneBytes + kTopkPlaneBytes / 32;
+  const size_t need = passes == 1 || rp_bytes > full ? per_pass * rp_bytes : full;
   if (need > c->topk_bytes) {
     DG_CUDA(cudaStreamSynchronize(c->stream));
     cudaFree(c->topk_plane);

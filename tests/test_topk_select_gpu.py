@@ -1,11 +1,12 @@
 """Selection of dg_attn_denoise_topk where its lists are at their limits: bounds below every visible key, keys that
-cluster in few groups, more keys than the lists hold, key counts around the tiles of the score kernel."""
+cluster in few groups, more keys than the lists hold, key counts around the tiles of the score kernel; and the plane of
+scores where it goes through several passes."""
 import numpy as np
 import pytest
 import torch
 
 from diffgemma_b200 import capi
-from diffgemma_b200.step_attn import AttnLayer
+from diffgemma_b200.step_attn import AttnLayer, CanvasAttention, Context, KvCache
 from oracle import attn_oracle as ao
 from tests import util
 from tests.test_topk_gpu import _oracle, _run
@@ -78,3 +79,59 @@ def test_scores_are_no_further_from_64_bits(ctx):
     # (2^-8 of one of 512 products, a relative 1e-4 of a probability); half a bf16 step of the output is 2^-8 of its
     # leading bit at worst
     assert worst <= 2.0 ** -8 + 4e-3, worst
+
+
+def _randn(seed, *shape):
+    return torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda").to(torch.bfloat16)
+
+
+def test_shorter_range_is_capturable_after_a_longer_one():
+    """30,000 keys go through the plane in two passes, 18,400 fill it in one: that call then finds its scratch in place."""
+    ctx = Context(0)
+    layer = AttnLayer(**G256)
+    kv, att = KvCache(ctx, layer, 30000), CanvasAttention(ctx, layer)
+    kv.load_prefix(_randn(1, 29744, 2, 256), _randn(2, 29744, 2, 256))
+    q, k, v = _randn(3, 256, 16, 256), _randn(4, 256, 2, 256), _randn(5, 256, 2, 256)
+    att.denoise_topk(kv, 29744, q, k, v)
+    out = torch.empty_like(q)
+    ctx.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=ctx.torch_stream):
+        att.denoise_topk(kv, 18144, q, k, v, out=out)
+    want = att.denoise_topk(kv, 18144, q, k, v)
+    with torch.cuda.stream(ctx.torch_stream):
+        out.zero_()
+        g.replay()
+    ctx.synchronize()
+    assert out.any() and torch.equal(out, want) and ctx.device_status()[0] == 0
+    del g
+    ctx.close()
+
+
+@pytest.mark.parametrize("lk,n_pass", [
+    (dict(G256, n_kv_heads=8, canvas=250), 1),     # 16 row pairs, every other one ragged, in passes of 6, 6 and 4; a head alone: one
+    (dict(FULL, canvas=256), 2),                   # the same passes; a head alone: two of 4
+])
+def test_passes_over_the_plane(ctx, lk, n_pass):
+    """All heads in one call against a call per KV head: the same rows in other passes, so the same bits."""
+    layer = AttnLayer(**lk)
+    P, C, H, D, G = 42100, layer.canvas, layer.n_kv_heads, layer.head_dim, 16 // layer.n_kv_heads
+    kp, vp = _randn(6, P, H, D), _randn(7, P, H, D)
+    q, k, v = _randn(8, C, 16, D), _randn(9, C, H, D), _randn(10, C, H, D)
+    kv = KvCache(ctx, layer, P + C)
+    kv.load_prefix(kp, vp)
+    got = CanvasAttention(ctx, layer).denoise_topk(kv, P, q, k, v)
+    ctx.synchronize()
+    assert ctx.last_launch_count == 1 + 2 * 3
+    kv.close()
+    one = AttnLayer(**dict(lk, n_q_heads=G, n_kv_heads=1))
+    for h in range(H):
+        kv = KvCache(ctx, one, P + C)
+        kv.load_prefix(kp[:, h:h + 1].contiguous(), vp[:, h:h + 1].contiguous())
+        want = CanvasAttention(ctx, one).denoise_topk(kv, P, q[:, h * G:(h + 1) * G].contiguous(), k[:, h:h + 1].contiguous(),
+                                                      v[:, h:h + 1].contiguous())
+        ctx.synchronize()
+        assert ctx.last_launch_count == 1 + 2 * n_pass
+        assert want.any() and torch.equal(got[:, h * G:(h + 1) * G], want), f"KV head {h}"
+        kv.close()
+    assert ctx.device_status()[0] == 0
