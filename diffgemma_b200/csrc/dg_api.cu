@@ -221,18 +221,22 @@ static bool fused_q_prologue_ok(const dg_layer_desc& d) {
 // prologue, output) and what exchanging and merging the partial rows of 2, 4 and 8 splits adds.
 struct SplitCost {
   uint32_t fixed, merge[3];
+  bool fp16_rows;      // the partial rows travel as fp16
 };
 // head_dim 256, a tile = 1.4 us.  32 query tiles (one canvas, 8 KV heads), us: 4 key tiles 21.3 unsplit, 20.5 with 2
 // splits, 19.1 with 4; 11 tiles 31.3 / 26.4 / 22.6; 64 query tiles: 4 key tiles 21.8 / 21.0, 11 tiles 31.7 / 27.1
-constexpr SplitCost kCost256 = {120, {14, 18, 55}};
+constexpr SplitCost kCost256 = {120, {14, 18, 55}, true};
 // splits that meet in memory: head_dim 512, under a bitmap, with the caller's workspace (a bitmap over 5 key tiles of 2 KV
 // heads: 27.9 us unsplit, 34.8 with 4 splits)
-constexpr SplitCost kCostMemory = {70, {36, 44, 55}};
+constexpr SplitCost kCostMemory = {70, {36, 44, 55}, false};
 
 static uint32_t choose_splits(const dg_ctx* ctx, uint32_t q_tiles, uint32_t k_tiles, const SplitCost& cost_of) {
   uint32_t smax = k_tiles < kSm100MaxSplits ? k_tiles : kSm100MaxSplits;
   if (smax < 1) smax = 1;
   if (ctx->forced_splits) return ctx->forced_splits < smax ? ctx->forced_splits : smax;
+  // A range is not cut into fp16 rows for a microsecond or two: up to six key tiles (seven for 64 query tiles), where splits
+  // that meet as fp32 would not pay, one CTA holds the fp32 sums from the first key to the rounded output.
+  if (cost_of.fp16_rows && choose_splits(ctx, q_tiles, k_tiles, kCostMemory) == 1) return 1;
   const uint32_t sms = ctx->num_sms > 0 ? uint32_t(ctx->num_sms) : 148u;
   uint32_t best = 1;
   uint64_t best_cost = ~0ull;

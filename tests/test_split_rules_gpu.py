@@ -38,7 +38,7 @@ def test_bitmap_splits(ctx, Hkv, canvas, P):
     (8, 200, 1100, 2),      # two canvases
     (2, 256, 770, 3),
     (8, 150, 2000, 1),      # an odd number of query tiles per KV head: no pairs
-    (8, 100, 433, 1),       # four splits of a short range
+    (8, 100, 433, 1),       # a short range, unsplit
     (16, 33, 90, 1), (1, 64, 500, 1),
 ])
 def test_automatic_launch_shapes(ctx, Hkv, canvas, P, batch):
@@ -55,3 +55,25 @@ def test_automatic_launch_shapes(ctx, Hkv, canvas, P, batch):
     for b in range(batch):
         util.assert_close(util.t2f(again[b]), refs[b], f"canvas {b}")
         kvs[b].close()
+
+
+@pytest.mark.parametrize("Hkv,canvas,P,batch", [(8, 100, 333, 1), (8, 256, 500, 1), (2, 256, 200, 1), (2, 64, 700, 1), (8, 256, 600, 2),
+                                                (1, 17, 100, 4)])
+def test_short_ranges_keep_fp32_sums(ctx, Hkv, canvas, P, batch):
+    """Up to six key tiles (seven for 64 query tiles) the automatic choice is one split, whose sums stay fp32 to the rounded
+    output: the same bits as with one split forced."""
+    layer = AttnLayer(n_kv_heads=Hkv, canvas=canvas, rope_theta=1e4, window=1024, mask_mode=capi.MASK_WINDOW_UNIFORM)
+    cases = [util.make_case(layer, P, seed=90 + b) for b in range(batch)]
+    kvs = [util.gpu_setup(ctx, c)[0] for c in cases]
+    att = CanvasAttention(ctx, layer)
+    q, k, v = (torch.stack([c[n] for c in cases]).cuda() for n in ("q", "kc", "vc"))
+    got = att.denoise(kvs, [P] * batch, q, k, v).clone()
+    try:
+        ctx.set_splits(1)
+        want = att.denoise(kvs, [P] * batch, q, k, v)
+        ctx.synchronize()
+    finally:
+        ctx.set_splits(0)
+    assert torch.equal(got, want) and ctx.device_status()[0] == 0
+    for kv in kvs:
+        kv.close()
