@@ -257,9 +257,10 @@ static uint32_t choose_splits(const dg_ctx* ctx, uint32_t q_tiles, uint32_t k_ti
 // there they pay from about a hundred key tiles on (2 KV heads: 100 tiles 53.6 against 52.3 us, 130 tiles 62.9 / 63.4),
 // with one split or two from eight (four canvases of a sliding layer, 11 tiles: 33.2 against 35.5 us; 8 KV heads, 34
 // tiles: 67.6 / 81.0; two canvases, 24 tiles: 34.2 / 37.5).
+constexpr uint32_t kLongTiles = 96;
 static bool pair_pays(uint32_t tiles_per_head, uint32_t k_tiles, uint32_t single_splits) {
   if (tiles_per_head < 2) return false;
-  return k_tiles >= 96 || (k_tiles >= 8 && single_splits <= 2 && tiles_per_head % 2 == 0);
+  return k_tiles >= kLongTiles || (k_tiles >= 8 && single_splits <= 2 && tiles_per_head % 2 == 0);
 }
 
 // Scratch of the attention calls grows without a synchronisation and without freeing: a CUDA graph may hold the address of
@@ -1214,15 +1215,18 @@ extern "C" int32_t dg_attn_denoise(dg_ctx* c, const dg_layer_desc* d, dg_kv* con
       k_min = kt < k_min ? kt : k_min;
       k_max = kt > k_max ? kt : k_max;
     }
+    // The longest canvas chooses the form and the splits: a canvas over few tiles loses a microsecond or two in another's
+    // form, a launch of its own takes 19 (sliding layer, 333 and three times 5,000 keys: 32.6 us in one launch, 90.3 one after
+    // the other; global layer, 500 and three times 4,000: 56.3 / 107.9).  Past a hundred key tiles a canvas alone is cut
+    // into more splits than a batch leaves it: one beside shorter ones than that runs by itself.
     const uint32_t single_splits = choose_splits(c, sm100_query_tiles(d->canvas, G, d->n_kv_heads) * batch, k_max, kCost256);
-    const bool pair_lo = c->pair_mode == 1 || (c->pair_mode == 2 && pair_pays(tph, k_min, single_splits));
-    const bool pair_hi = c->pair_mode == 1 || (c->pair_mode == 2 && pair_pays(tph, k_max, single_splits));
-    conc_pair = pair_lo;
+    conc_pair = c->pair_mode == 1 || (c->pair_mode == 2 && pair_pays(tph, k_max, single_splits));
     const uint32_t q_tiles = conc_pair ? sm100_pair_query_tiles(d->canvas, G, d->n_kv_heads)
                                        : sm100_query_tiles(d->canvas, G, d->n_kv_heads);
     conc_splits = choose_splits(c, q_tiles * batch, k_max, kCost256);
     const bool no_ws = conc_splits == 1 || (conc_pair ? conc_splits == 2 : (conc_splits == 2 || conc_splits == 4 || conc_splits == 8));
-    concurrent = pair_lo == pair_hi && no_ws && conc_splits <= k_min;
+    const bool alike = c->pair_mode != 2 || tph < 2 || (k_min >= kLongTiles) == (k_max >= kLongTiles);
+    concurrent = alike && no_ws && conc_splits <= k_min;
   }
   const uint32_t saved_splits = c->forced_splits;
   const int saved_pair = c->pair_mode;

@@ -1,5 +1,6 @@
 """Key splits under a decoder bitmap (a cluster shares the merge of fp32 rows) and the launch shapes that the split and pair
-rules choose: short key ranges with odd tile counts, several canvases, in-launch appends of every unit size."""
+rules choose: short key ranges with odd tile counts, several canvases of equal and unequal lengths, in-launch
+appends of every unit size."""
 import numpy as np
 import pytest
 import torch
@@ -77,3 +78,26 @@ def test_short_ranges_keep_fp32_sums(ctx, Hkv, canvas, P, batch):
     assert torch.equal(got, want) and ctx.device_status()[0] == 0
     for kv in kvs:
         kv.close()
+
+
+@pytest.mark.parametrize("Hkv,canvas,window,Ps", [
+    (8, 256, 1024, (333, 5000, 5000, 5000)),      # 5 and 11 key tiles: both sides of where pairs begin to pay
+    (8, 256, 1024, (2000, 600, 9000)),
+    (2, 256, 0, (333, 2048)),
+    (2, 256, 0, (500, 4000, 4000, 4000)),
+    (2, 256, 0, (0, 700, 40, 4000, 260)),         # two launches of up to four
+])
+def test_unequal_canvases_share_a_launch(ctx, Hkv, canvas, window, Ps):
+    layer = AttnLayer(n_kv_heads=Hkv, canvas=canvas, rope_theta=1e4, window=window,
+                      mask_mode=capi.MASK_WINDOW_UNIFORM if window else capi.MASK_NONE)
+    cases = [util.make_case(layer, P, seed=70 + b) for b, P in enumerate(Ps)]
+    kvs = [util.gpu_setup(ctx, c)[0] for c in cases]
+    att = CanvasAttention(ctx, layer)
+    q, k, v = (torch.stack([c[n] for c in cases]).cuda() for n in ("q", "kc", "vc"))
+    att.denoise(kvs, list(Ps), q, k, v)
+    got = att.denoise(kvs, list(Ps), q, k, v)      # positions known: the appends run inside the attention launch
+    ctx.synchronize()
+    assert ctx.last_launch_count == (len(Ps) + 3) // 4 and ctx.device_status()[0] == 0
+    for b, case in enumerate(cases):
+        util.assert_close(util.t2f(got[b]), util.run_oracle(case), f"canvas {b}")
+        kvs[b].close()
