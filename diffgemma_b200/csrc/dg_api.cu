@@ -1056,14 +1056,16 @@ static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
 
 // May a bitmap call take the tensor kernels?  They move whole 16-byte vectors, and its entry point also takes tensors off
 // 16-byte boundaries: those go to the general kernel, which reads and writes element by element.  So does an output that
-// lies over the queries: rows that come out non-finite are computed again from those (launch_bitmap_fix).
+// lies over the queries (rows that come out non-finite are computed again from those: launch_bitmap_fix), and a layer of
+// more query tiles than a launch of the tensor kernels takes.
 static bool bitmap_on_tensor(const dg_layer_desc& d, const AttnCall& a, const void* q, const void* k, const void* v, const void* qw,
                              const void* kw) {
   for (const void* p : {q, k, v, qw, kw, static_cast<const void*>(a.out)})
     if (!aligned16(p)) return false;
   const size_t bytes = size_t(d.canvas) * d.n_q_heads * d.head_dim * 2;
   const uintptr_t qa = reinterpret_cast<uintptr_t>(q), oa = reinterpret_cast<uintptr_t>(a.out);
-  return qa + bytes <= oa || oa + bytes <= qa;
+  const uint32_t tiles = sm100_query_tiles(d.canvas, d.n_q_heads / d.n_kv_heads, d.n_kv_heads) * (d.head_dim == 512 ? 2 : 1);
+  return (qa + bytes <= oa || oa + bytes <= qa) && tiles <= kMaxQueryTiles;
 }
 
 // one canvas: stage 1 on K/V (+ table), then stage 2 with the fused Q prologue

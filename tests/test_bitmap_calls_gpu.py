@@ -183,3 +183,18 @@ def test_captured_before_any_scratch_exists(hd):
     assert ctx.device_status()[0] == 0
     del g
     ctx.close()
+
+
+@pytest.mark.parametrize("hd,heads", [(256, 4097), (512, 2049)])
+def test_more_query_tiles_than_a_tensor_launch_takes(ctx, hd, heads):
+    layer = AttnLayer(n_q_heads=heads, n_kv_heads=heads, head_dim=hd, canvas=1, rotary_dim=hd, rope_theta=1e6)
+    kv, att = KvCache(ctx, layer, 101), CanvasAttention(ctx, layer)
+    g = torch.Generator(device=DEV).manual_seed(hd)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)
+    kv.append(rn(100, heads, hd), rn(100, heads, hd), 0)
+    args = rn(1, heads, hd), rn(1, heads, hd), rn(1, heads, hd), (torch.rand(1, 101, generator=g, device=DEV) < 0.5).to(torch.uint8)
+    want = _general(ctx, att, kv, 100, args)
+    got = att.denoise_bitmap(kv, 100, *args)
+    ctx.synchronize()
+    assert want.any() and torch.equal(got, want)
+    kv.close()
