@@ -1058,8 +1058,13 @@ static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
 // 16-byte boundaries: those go to the general kernel, which reads and writes element by element.  So does an output that
 // lies over the queries (rows that come out non-finite are computed again from those: launch_bitmap_fix), and a layer of
 // more query tiles than a launch of the tensor kernels takes.
-static bool bitmap_on_tensor(const dg_layer_desc& d, const AttnCall& a, const void* q, const void* k, const void* v, const void* qw,
-                             const void* kw) {
+// Few rows over few keys are quicker there too: the tensor kernels' launches take 16 to 20 us however little there is to do
+// (head_dim 256, 16 heads, us general / tensor: 1 key, 1 canvas row 8.9 / 16.6; 61 keys 14.5 / 16.6; 77 keys, 17 rows, 8 KV
+// heads 18.7 / 20.4; 301 keys, 1 row 45 / 20; 160 keys, 100 rows 69 / 22; head_dim 512: 61 keys, 1 row 18.7 / 18.6, 77 keys, 17
+// rows 24.2 / 22.3).
+static bool bitmap_on_tensor(const dg_ctx* c, const dg_layer_desc& d, const AttnCall& a, uint32_t kv_len, const void* q, const void* k,
+                             const void* v, const void* qw, const void* kw) {
+  if ((size_t(kv_len) + d.canvas) * d.head_dim <= 80 * 256 && d.canvas * d.n_q_heads <= 2u * uint32_t(c->num_sms)) return false;
   for (const void* p : {q, k, v, qw, kw, static_cast<const void*>(a.out)})
     if (!aligned16(p)) return false;
   const size_t bytes = size_t(d.canvas) * d.n_q_heads * d.head_dim * 2;
@@ -1078,7 +1083,7 @@ static int32_t denoise_one(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, uint32_
   // leaves nothing queued (a split-KV group then stays in step with its peers)
   r = check_ring_span(kv, make_mask(d, kv_len, a.t0, a.t1, a.include_canvas), d.canvas);
   if (r != DG_OK) return r;
-  bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general && (attend == nullptr || bitmap_on_tensor(d, a, q, k, v, qw, kw));
+  bool tensor = tensor_path_ok(d) && kv->has_tmap && !c->force_general && (attend == nullptr || bitmap_on_tensor(c, d, a, kv_len, q, k, v, qw, kw));
   // A bitmap is packed for the tensor kernels on every geometry they have: the packing reads it once (about 3 us for
   // 256 x 2,304), the CUDA-core kernel that other head_dims use visits keys one by one
   if (tensor && attend != nullptr) {

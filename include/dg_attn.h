@@ -255,7 +255,8 @@ int32_t dg_host_pipe_destroy(dg_host_pipe* pipe);
 int32_t dg_host_pipe_set_deferred_launch(dg_host_pipe* pipe, int32_t on);
 /* General decoder bitmap (reference DecoderAttnMask, src/model/mask.rs:4-27): attend is a
  * device pointer to uint8 [C][kv_len+C], 1 = visible.  head_dim 256 / 512 with every tensor on a
- * 16-byte boundary: packed to bits, then the tensor kernels; otherwise the general kernel.       */
+ * 16-byte boundary: packed to bits, then the tensor kernels; otherwise, and where there is little
+ * to do, the general kernel.                                                                     */
 int32_t dg_attn_denoise_bitmap(dg_ctx* ctx, const dg_layer_desc* desc, dg_kv* kv, uint32_t kv_len,
                                const void* q, const void* k, const void* v, const void* qw, const void* kw,
                                const uint8_t* attend, void* out);
@@ -433,8 +434,8 @@ int32_t dg_ctx_kernel_timing(dg_ctx* ctx, int32_t on, uint32_t max_launches);
  * 2 Q prologue done, 3 key loop done, 4 epilogue done, 5 merge done; slots 6-11 hold SM-clock
  * cycles single threads spent waiting inside the key loop (6 MMA issuer on K, 7 on V, 8 on P,
  * 9 the issuer's whole loop, 10 softmax thread 0 on S, 11 on the rescale barrier); slots 12-14 are
- * stamps inside the tail (12 last PV complete, 13 own rows staged, 14 cluster's rows arrived).  The
- * stamps cost time; NULL switches them off.                                                             */
+ * stamps inside the tail (12 last PV complete, 13 own rows staged, 14 cluster's rows arrived), slot 15
+ * the end of the CTA's part of the in-launch append.  The stamps cost time; NULL switches them off.     */
 int32_t dg_ctx_phase_stamps(dg_ctx* ctx, void* device_buffer);
 int32_t dg_ctx_kernel_time(dg_ctx* ctx, double* total_ms, uint32_t* launches);
 

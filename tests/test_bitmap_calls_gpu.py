@@ -198,3 +198,21 @@ def test_more_query_tiles_than_a_tensor_launch_takes(ctx, hd, heads):
     ctx.synchronize()
     assert want.any() and torch.equal(got, want)
     kv.close()
+
+
+@pytest.mark.parametrize("hd,P,canvas,small", [(256, 0, 1, True), (256, 62, 18, True), (256, 63, 18, False), (256, 61, 19, False),
+                                               (512, 22, 18, True), (512, 23, 18, False), (512, 21, 19, False)])
+def test_small_calls(ctx, hd, P, canvas, small):
+    """Both sides of the line below which the general kernel is the quicker one (80 keys of 256, two rows a multiprocessor)."""
+    case, seen, args = _case(hd, P, canvas, seed=hd + P)
+    kv, att = util.gpu_setup(ctx, case)
+    want = _general(ctx, att, kv, P, args)
+    launches = ctx.last_launch_count
+    got = att.denoise_bitmap(kv, P, *args)
+    ctx.synchronize()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert sms != 148 or (ctx.last_launch_count == launches) == small
+    if small:
+        assert torch.equal(got, want)
+    util.assert_close(util.t2f(got), util.run_oracle(case, attend=seen), "bitmap")
+    kv.close()
