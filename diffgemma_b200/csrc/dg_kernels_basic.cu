@@ -142,27 +142,26 @@ __global__ void __launch_bounds__(256) dg_append_table_kernel(const AppendParams
 }
 
 // ------------------------------------------------------------------------------------------
-// The same stage for head_dim 256 and 512 with rotary runs of whole 16-byte chunks: a CTA takes one or a few tokens,
-// computes their (cos, sin) pairs once into shared memory, and a warp handles two head vectors at a time, lane c the
-// 16-byte chunks c and c + 32 together with the chunks that hold their rotation partners.
-// Bound: latency at canvas size, memory on long appends.  The kernel above issues a warp per CTA, 2-byte accesses and
-// a sincos per (vector, pair): a head_dim-512 step took 5 us longer with it (32k keys 295.8 -> 290.8 us, 150 keys
-// 23.4 -> 21.9 us).  Order of operations (chunk-wise sums of squares, butterfly, rotation through
+// The same stage for head_dim 256 and 512 with rotary runs of whole 16-byte chunks: a CTA takes one token, or some of its
+// head vectors, computes the token's (cos, sin) pairs once into shared memory, and a warp handles one or two vectors at a
+// time, lane c the 16-byte chunks c and c + 32 together with the chunks that hold their rotation partners.
+// Bound: latency up to some thousand vectors, memory on long appends.  The kernel above issues a warp per CTA, 2-byte
+// accesses and a sincos per (vector, pair): a head_dim-512 step took 5 us longer with it (32k keys 295.8 -> 290.8 us, 150
+// keys 23.4 -> 21.9 us).  Order of operations (chunk-wise sums of squares, butterfly, rotation through
 // rope_rotate / rope_norm_rotate) as above: both write the same bits.
 // ------------------------------------------------------------------------------------------
-constexpr uint32_t kRowsMaxTok = 4, kRowsMaxWarps = 10, kRowsUnit = 2;
+constexpr uint32_t kRowsMaxWarps = 10, kRowsUnit = 2;
 
 template <uint32_t NS>   // 16-byte chunks of a vector per lane: head_dim 256 -> 1, 512 -> 2
 // head_dim 512: 64 registers, so that three CTAs share an SM (16,000 tokens of 2 x 512: 68.7 us with 90 registers, 54.9 so)
-__global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append_rows_kernel(const AppendParams p, const RopeParams rp, uint32_t tok_per_cta) {
-  __shared__ float2 cs[kRowsMaxTok * kMaxRotHalf];
+__global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append_rows_kernel(const AppendParams p, const RopeParams rp, uint32_t slots_per_cta) {
+  __shared__ __align__(16) float2 cs[kMaxRotHalf];   // read as float4
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");   // see dg_append_kernel
   constexpr uint32_t D = NS * 256u, U = kRowsUnit;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  const uint32_t tok0 = blockIdx.x * tok_per_cta;
-  const uint32_t nt = p.n - tok0 < tok_per_cta ? p.n - tok0 : tok_per_cta;
-  const uint32_t nq = p.q_in ? p.Hq : 0u, slots = nq + 2u * p.Hkv, n_vec = nt * slots;
+  const uint32_t tok = blockIdx.x, pos = p.pos0 + tok;
+  const uint32_t nq = p.q_in ? p.Hq : 0u, slot0 = blockIdx.y * slots_per_cta, slot_end = min(slot0 + slots_per_cta, nq + 2u * p.Hkv);
   const uint32_t rot_chunks = rp.rot_half / 8u, off_chunks = rp.pair_off / 8u;
 
   // chunk of this lane in slot j, the chunk of its rotation partner (itself when not rotated), its first pair index
@@ -178,12 +177,11 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append
     pair0[j] = (low[j] ? c : c - off_chunks) * 8u;
   }
   uint4 x[U][NS], xp[U][NS];
-  auto load = [&](uint32_t v0) {
+  auto load = [&](uint32_t s0) {
 #pragma unroll
     for (uint32_t u = 0; u < U; ++u) {
-      const uint32_t v = v0 + u * n_warps;
-      if (v >= n_vec) break;
-      const uint32_t tok = tok0 + v / slots, slot = v % slots;
+      const uint32_t slot = s0 + u * n_warps;
+      if (slot >= slot_end) break;
       const bool is_q = slot < nq, is_k = !is_q && slot < nq + p.Hkv;
       const uint32_t H = is_q ? p.Hq : p.Hkv, h = is_q ? slot : (slot - nq) % p.Hkv;
       const uint4* src = reinterpret_cast<const uint4*>((is_q ? p.q_in : is_k ? p.k_in : p.v_in) + (size_t(tok) * H + h) * D);
@@ -194,24 +192,22 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append
       }
     }
   };
-  load(warp);
-  // (cos, sin) of the tokens' positions, while the first vectors are on their way
-  for (uint32_t e = threadIdx.x; e < nt * rp.rot_half; e += blockDim.x) {
-    const uint32_t t = e / rp.rot_half, i = e - t * rp.rot_half;
-    const float a = float(p.pos0 + tok0 + t) * rp.inv_freq[i];
+  load(slot0 + warp);
+  // (cos, sin) of the token's position, while the first vectors are on their way
+  for (uint32_t i = threadIdx.x; i < rp.rot_half; i += blockDim.x) {
+    const float a = float(pos) * rp.inv_freq[i];
     const float2 v = make_float2(cosf(a), sinf(a));
-    cs[t * rp.rot_half + i] = v;
-    if (p.rope_table) p.rope_table[size_t(tok0 + t) * rp.rot_half + i] = v;
+    cs[i] = v;
+    if (p.rope_table && blockIdx.y == 0u) p.rope_table[size_t(tok) * rp.rot_half + i] = v;
   }
   __syncthreads();
   auto lo16 = [](uint32_t w) { return __uint_as_float(w << 16); };
   auto hi16 = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
-  for (uint32_t v0 = warp; v0 < n_vec; v0 += U * n_warps) {
+  for (uint32_t s0 = slot0 + warp; s0 < slot_end; s0 += U * n_warps) {
 #pragma unroll
     for (uint32_t u = 0; u < U; ++u) {
-      const uint32_t v = v0 + u * n_warps;
-      if (v >= n_vec) break;                              // warp-uniform
-      const uint32_t t = v / slots, tok = tok0 + t, slot = v % slots, pos = p.pos0 + tok;
+      const uint32_t slot = s0 + u * n_warps;
+      if (slot >= slot_end) break;                        // warp-uniform
       const bool is_q = slot < nq, is_k = !is_q && slot < nq + p.Hkv;
       const uint32_t H = is_q ? p.Hq : p.Hkv, h = is_q ? slot : (slot - nq) % p.Hkv;
       uint4 y[NS];
@@ -240,7 +236,7 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append
             const uint32_t q[4] = {xp[u][j].x, xp[u][j].y, xp[u][j].z, xp[u][j].w};
             const uint4 p4 = wt ? reinterpret_cast<const uint4*>(wt)[partner[j]] : ones;
             const uint32_t wq[4] = {p4.x, p4.y, p4.z, p4.w};
-            const float4* tab = reinterpret_cast<const float4*>(cs + t * rp.rot_half + pair0[j]);
+            const float4* tab = reinterpret_cast<const float4*>(cs + pair0[j]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float4 c2 = tab[e];
@@ -284,7 +280,7 @@ __global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append
         if (stored) reinterpret_cast<uint4*>(cache)[chunk[j]] = y[j];
       }
     }
-    if (v0 + U * n_warps < n_vec) load(v0 + U * n_warps);
+    if (s0 + U * n_warps < slot_end) load(s0 + U * n_warps);
   }
 }
 
@@ -319,14 +315,20 @@ void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st,
     return;
   }
   if (append_rows_ok(p, rp)) {
-    // as many tokens per CTA as give its warps about two vectors each: one where Q or many KV heads come along
+    // Few vectors: a warp for each, up to eight of a token per CTA, and at least four warps for the token's (cos, sin) pairs;
+    // what counts is the latency of one vector.  Many: all of a token's vectors in one CTA, two or more per warp, so that the
+    // pairs are computed once and more loads are in flight.  us with a warp per vector / two per warp: 2 KV heads of 256, 256
+    // tokens 3.3 / 3.9, 1,000 4.3 / 6.0, 2,000 7.5 / 6.7; 16 of 256, 100 tokens 3.4 / 5.5, 256 6.4 / 5.9; 2 of 512, 17 tokens 3.7 /
+    // 4.6, 1,000 6.0 / 8.6, 8,000 29.9 / 27.6; 8 of 512, 256 tokens 7.0 / 7.8, 500 9.4 / 8.4.  (One-warp CTAs of the kernel above:
+    // 2 of 512, 17 tokens 3.7, 1,000 7.1, 8,000 35.6.)
     const uint32_t slots = (p.q_in ? p.Hq : 0u) + 2u * p.Hkv;
-    const uint32_t tok = slots >= 16u ? 1u : (16u / slots < kRowsMaxTok ? 16u / slots : kRowsMaxTok);
-    const uint32_t warps = (tok * slots + kRowsUnit - 1u) / kRowsUnit;
-    cfg.gridDim = dim3((p.n + tok - 1u) / tok);
+    const bool few = size_t(p.n) * slots <= (p.D == 256 ? 4096u : 6144u);
+    const uint32_t groups = few ? (slots + 7u) / 8u : 1u, spc = (slots + groups - 1u) / groups;
+    const uint32_t warps = few ? (spc > 4u ? spc : 4u) : (spc + kRowsUnit - 1u) / kRowsUnit;
+    cfg.gridDim = dim3(p.n, (slots + spc - 1u) / spc);
     cfg.blockDim = dim3(32u * (warps < kRowsMaxWarps ? warps : kRowsMaxWarps));
-    if (p.D == 256) cudaLaunchKernelEx(&cfg, dg_append_rows_kernel<1>, p, rp, tok);
-    else cudaLaunchKernelEx(&cfg, dg_append_rows_kernel<2>, p, rp, tok);
+    if (p.D == 256) cudaLaunchKernelEx(&cfg, dg_append_rows_kernel<1>, p, rp, spc);
+    else cudaLaunchKernelEx(&cfg, dg_append_rows_kernel<2>, p, rp, spc);
     return;
   }
   const uint32_t slots = (p.q_in ? p.Hq : 0u) + 2u * p.Hkv + (p.rope_table ? 1u : 0u);

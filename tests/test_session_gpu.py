@@ -109,3 +109,34 @@ def test_stage_one_in_place_writes_the_same_bits(ctx, lk):
     assert not _same(aligned[0], x[0])
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("hd,Hkv,n", [
+    (256, 16, 128), (256, 16, 129),      # both sides of 4,096 vectors: four groups of eight a token, one CTA a token
+    (256, 5, 7), (256, 9, 40),           # ten and eighteen vectors a token: two groups of five, three of six
+    (256, 1, 2049), (512, 3, 1024), (512, 3, 1025), (512, 11, 3),
+])
+def test_append_groups_write_the_same_bits(ctx, hd, Hkv, n):
+    layer = AttnLayer(n_q_heads=Hkv, n_kv_heads=Hkv, head_dim=hd, rotary_dim=hd // 2, rope_theta=1e5, v_norm=1)
+    k, v, kw = _randn(11, n, Hkv, hd).to(DEV), _randn(12, n, Hkv, hd).to(DEV), (1 + 0.1 * _randn(13, hd)).to(torch.bfloat16).to(DEV)
+    a, b = KvCache(ctx, layer, 77 + n), KvCache(ctx, layer, 77 + n)
+    a.append(k, v, 77, kw)
+    b.append(_off_by_one(k), _off_by_one(v), 77, kw)
+    for x, y in zip(a.read(0, 77 + n), b.read(0, 77 + n)):
+        assert _same(x, y) and x[77:].any() and not x[:77].any()
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("hd,Hkv,canvas", [(256, 2, 17), (256, 8, 128), (256, 8, 129), (512, 2, 256)])
+def test_stage_one_groups_write_the_table(ctx, hd, Hkv, canvas):
+    """The first step at new positions: one group of a token writes its row of the RoPE table, the steps after it read it."""
+    layer = AttnLayer(n_kv_heads=Hkv, head_dim=hd, rotary_dim=hd, rope_theta=1e4, canvas=canvas)
+    q, k, v = _randn(14, 1, canvas, 16, hd).to(DEV), _randn(15, 1, canvas, Hkv, hd).to(DEV), _randn(16, 1, canvas, Hkv, hd).to(DEV)
+    kv, att = KvCache(ctx, layer, 300 + canvas), CanvasAttention(ctx, layer)
+    kv.load_prefix(_randn(17, 300, Hkv, hd), _randn(18, 300, Hkv, hd))
+    first = att.denoise([kv], [300], q, k, v).clone()
+    rows = [t.clone() for t in kv.read(300, canvas)]
+    again = att.denoise([kv], [300], q, k, v)
+    assert _same(first, again) and all(_same(x, y) for x, y in zip(rows, kv.read(300, canvas)))
+    kv.close()
