@@ -865,13 +865,6 @@ struct FixedWs {
   uint32_t n_counters = 0;
 };
 
-static int32_t bitmap_fix(dg_ctx* c, const AttnParams& p) {
-  const cudaError_t e = launch_bitmap_fix(p, launch_stream(c));
-  if (e != cudaSuccess) return fail_cuda(e, "launch_bitmap_fix");
-  c->last_launches += 1;
-  return DG_OK;
-}
-
 static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const AttnCall& a,
                             const FixedWs* fixed = nullptr) {
   AttnParams p;
@@ -982,7 +975,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
       c->ev_used += 2;
     }
     c->last_launches += 1;
-    return a.packed ? bitmap_fix(c, p) : DG_OK;
+    return DG_OK;
   }
   const uint32_t tiles_per_head = sm100_query_tiles(p.C, p.G, 1);
   const uint32_t k_tiles = sm100_key_tiles(p.mask);
@@ -1045,7 +1038,7 @@ static int32_t do_attention(dg_ctx* c, const dg_layer_desc& d, dg_kv* kv, const 
     c->ev_used += 2;
   }
   c->last_launches += 1;
-  return a.packed ? bitmap_fix(c, p) : DG_OK;
+  return DG_OK;
 }
 
 static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
@@ -1056,7 +1049,7 @@ static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
 
 // May a bitmap call take the tensor kernels?  They move whole 16-byte vectors, and its entry point also takes tensors off
 // 16-byte boundaries: those go to the general kernel, which reads and writes element by element.  So does an output that
-// lies over the queries (rows that come out non-finite are computed again from those: launch_bitmap_fix), and a layer of
+// lies over the queries (rows that come out non-finite are computed again from those: bitmap_rows_again), and a layer of
 // more query tiles than a launch of the tensor kernels takes.
 // Few rows over few keys are quicker there too: the tensor kernels' launches take 16 to 20 us however little there is to do
 // (head_dim 256, 16 heads, us general / tensor: 1 key, 1 canvas row 8.9 / 16.6; 61 keys 14.5 / 16.6; 77 keys, 17 rows, 8 KV

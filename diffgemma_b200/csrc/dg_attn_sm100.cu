@@ -106,7 +106,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   const uint32_t bar_base = smem_base + OFF_BAR;
   volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR + B_COUNT * 8);
   // ctl[0] = TMEM base address, ctl[1] = abort flag, ctl[2] = "this CTA merges" flag, ctl[3], ctl[4] = append shares,
-  // ctl[5] = the wait for the cluster's rows gave up
+  // ctl[5] = the wait for the cluster's rows gave up, ctl[6] = this CTA stored a row that is not finite (BITS)
   float* xch_max = reinterpret_cast<float*>(smem + OFF_XCH);   // [2 tile parities][BM][NTR]
   float* xch_misc = xch_max + 2 * BM * NTR;                     // [BM][NTR]: row maxima of |O| for the fp16 exchange
   float* xch_l = xch_misc + BM * NTR;                           // [BM][NTR]: final softmax denominators
@@ -191,6 +191,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     ctl[1] = 0u;
     ctl[2] = 0u;
     ctl[5] = 0u;
+    if (BITS) ctl[6] = 0u;
     fence_mbar_init();
   }
   if (warp == W_MMA) {
@@ -800,6 +801,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       for (uint32_t k = 0; k < 8; ++k) {
         if (Rw + k < rows_per_head) {
           const uint4 w = *reinterpret_cast<const uint4*>(rows16 + ((r0 + k) * HBUF_LD + lane * 8u) * 2u);
+          if (BITS && nonfinite_bf16x8(w)) ctl[6] = 1u;
           *reinterpret_cast<uint4*>(p.out + (size_t(i) * p.Hq + kvh * p.G + g) * HD + lane * 8u) = w;
         }
         if (++g == p.G) { g = 0; ++i; }
@@ -937,9 +939,10 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       for (uint32_t k = 0; k < 2; ++k) {
         if (!live_row[k]) continue;
         const float inv = lg[k] > 0.f ? 1.0f / lg[k] : 0.f;
-        *reinterpret_cast<uint4*>(p.out + orow[k] * HD + lane * 8) =
-            make_uint4(pack_bf16x2(acc[k][0] * inv, acc[k][1] * inv), pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv),
-                       pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv), pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv));
+        const uint4 w = make_uint4(pack_bf16x2(acc[k][0] * inv, acc[k][1] * inv), pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv),
+                                   pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv), pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv));
+        if (nonfinite_bf16x8(w)) ctl[6] = 1u;
+        *reinterpret_cast<uint4*>(p.out + orow[k] * HD + lane * 8) = w;
       }
     }
   }
@@ -1145,7 +1148,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     if (ctl[2]) {
       __threadfence();
       const float2* ml_all = reinterpret_cast<const float2*>(p.ws_ml);
-      if (S == 2) {
+      if (S == 2 && !BITS) {   // a bitmap's two splits form a cluster
         // Two splits: one round trip.  A warp takes four rows, every lane loads
         // both (m, l) pairs and its eight columns of both partials at once.
         constexpr uint32_t RK2 = 4;
@@ -1287,6 +1290,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
             w4.y = pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv);
             w4.z = pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv);
             w4.w = pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv);
+            if (BITS && nonfinite_bf16x8(w4)) ctl[6] = 1u;
             *reinterpret_cast<uint4*>(p.out + orow[k] * HD + lane * 8) = w4;
           } else {
             float4* dst = reinterpret_cast<float4*>(p.out_o + orow[k] * HD + lane * 8);
@@ -1304,6 +1308,12 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
     }
   }
   stamp(p, 5);
+  if (BITS) __syncthreads();
+  if (BITS && ctl[6]) {
+    const uint32_t rpc = BM / cs;
+    bitmap_rows_again<1>(p, kvh, mt, cs > 1 ? crank * rpc : 0u, cs > 1 ? (crank + 1u) * rpc : BM, 0u, abort_flag);
+    __syncthreads();     // every warp is past its wait for the append before the counters may go back to zero
+  }
   // the copies out of this CTA's shared memory have all landed once every CTA of the cluster is through its merge
   if (!BITS && cs > 1) {
     if (lane == 0 && ctl[5]) {   // rows that did not come: report it, and give the copies time before the cluster leaves

@@ -57,7 +57,7 @@ __device__ __forceinline__ void row_pair_sync(uint32_t smw) {
 // BITS: visibility from a packed decoder bitmap, P as the sum of two bf16 (as in the head_dim-256 kernel)
 template <bool BITS>
 __global__ void __launch_bounds__(h5::THREADS, 1)
-dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_k,
+dg_attn_sm100_hd512_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ CUtensorMap tm_k,
                            const __grid_constant__ CUtensorMap tm_v) {
   using namespace h5;
   extern __shared__ uint8_t smem_raw[];
@@ -316,6 +316,7 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
   }
 
   // ------------------------------------------------------------------ epilogue (softmax warps)
+  bool nonfinite = false;      // BITS: this thread stored an infinite or NaN output
   if (warp < SM_WARPS) {
     bool have_o = __all_sync(0xffffffffu, n_local > 0 && !*abort_flag);
     if (have_o) {
@@ -329,7 +330,7 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
     row_pair_sync(smw);
     const float l_tot = xch_max[r * NTR] + xch_max[r * NTR + 1];
     // the Q tile is dead: its shared memory stages the stores
-    store_o_half(p, smem + O_Q, tmem, kvh, mt, split, dh, smw, lane, half, have_o, m_used, l_tot);
+    store_o_half(p, smem + O_Q, tmem, kvh, mt, split, dh, smw, lane, half, have_o, m_used, l_tot, BITS ? &nonfinite : nullptr);
   }
 
   // ------------------------------------------------------------------ teardown
@@ -345,7 +346,8 @@ dg_attn_sm100_hd512_kernel(const AttnParams p, const __grid_constant__ CUtensorM
   if (warp == W_MMA) tmem_dealloc(tmem, TMEM_COLS);
 
   // ------------------------------------------------------------------ split merge by the last CTA to arrive
-  if (p.n_splits > 1) merge_splits_last(p, &ctl[2], kvh, mt, dh, THREADS);
+  if (p.n_splits > 1) merge_splits_last(p, &ctl[2], kvh, mt, dh, THREADS, BITS ? &nonfinite : nullptr);
+  if (BITS && __syncthreads_or(nonfinite)) bitmap_rows_again<2>(p, kvh, mt, 0u, BM, dh * HDV, abort_flag);
 }
 
 cudaError_t sm100_hd512_configure() {

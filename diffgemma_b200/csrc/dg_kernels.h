@@ -11,8 +11,6 @@ void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st,
 // device memory to or from the cache (n_chunks < 2^31, 16-byte aligned tensors)
 cudaError_t launch_kv_copy(const KvCopyParams& p, cudaStream_t st);
 void launch_attn_general(const AttnParams& p, cudaStream_t st);
-// behind a tensor kernel under a bitmap (head_dim 256 / 512): non-finite rows of p.out again, as the general kernel computes them
-cudaError_t launch_bitmap_fix(const AttnParams& p, cudaStream_t st);
 // decoder bitmap [C][T] -> bits [C][ceil(T / 128)], live [pack_attend_runs(C)][ceil(T / 128)]
 uint32_t pack_attend_runs(uint32_t C);
 cudaError_t launch_pack_attend(const uint8_t* attend, uint32_t C, uint32_t T, uint4* bits, uint8_t* live, cudaStream_t st);

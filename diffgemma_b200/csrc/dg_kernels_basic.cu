@@ -390,13 +390,13 @@ cudaError_t launch_kv_copy(const KvCopyParams& p, cudaStream_t st) {
 // ------------------------------------------------------------------------------------------
 constexpr int GEN_WARPS = 4;
 
-// one row by the whole CTA
-__device__ __forceinline__ void attn_general_row(const AttnParams& p, uint32_t row, uint32_t h) {
+__global__ void __launch_bounds__(GEN_WARPS * 32) dg_attn_general_kernel(const AttnParams p) {
   __shared__ float qs[kMaxHeadDim];
   __shared__ float red[GEN_WARPS];
   __shared__ float wm[GEN_WARPS], wl[GEN_WARPS];
   __shared__ float wo[GEN_WARPS][kMaxHeadDim];
 
+  const uint32_t row = blockIdx.x, h = blockIdx.y;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t D = p.D, kvh = h / p.G;
 
@@ -538,69 +538,6 @@ __device__ __forceinline__ void attn_general_row(const AttnParams& p, uint32_t r
     p.out_m[orow] = mg * 0.6931471805599453f;  // log2 units -> natural units
     p.out_l[orow] = lg;
   }
-}
-
-__global__ void __launch_bounds__(GEN_WARPS * 32) dg_attn_general_kernel(const AttnParams p) {
-  attn_general_row(p, blockIdx.x, blockIdx.y);
-}
-
-// ------------------------------------------------------------------------------------------
-// A bitmap hides keys whose K and V rows need not hold numbers (padding that was never written).  The kernel above does
-// not look at them; the tensor kernels multiply every value row of a visited tile by its P, and 0 * inf and 0 * NaN are
-// NaN.  A row that meets one comes out non-finite in some column, whatever it sees: this kernel, launched behind them, looks
-// through the bf16 rows they wrote and computes those that are not finite again the general way, so that the result is the
-// general kernel's also where a visible key is infinite or NaN.
-// Bound: one round trip over 2 MB of rows that L2 holds; every load of a CTA is in flight at once.
-// ------------------------------------------------------------------------------------------
-constexpr uint32_t FIX_ROWS = 16, FIX_PER_WARP = FIX_ROWS / GEN_WARPS;
-
-template <uint32_t NS>   // 16-byte chunks of a row per lane: head_dim 256 -> 1, 512 -> 2
-__global__ void __launch_bounds__(GEN_WARPS * 32) dg_attn_bitmap_fix_kernel(const AttnParams p) {
-  __shared__ uint32_t bad[GEN_WARPS];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, rows = p.C * p.Hq, r0 = blockIdx.x * FIX_ROWS;
-  const uint4* out = reinterpret_cast<const uint4*>(p.out);
-  uint4 x[FIX_PER_WARP][NS];
-#pragma unroll
-  for (uint32_t k = 0; k < FIX_PER_WARP; ++k)
-#pragma unroll
-    for (uint32_t j = 0; j < NS; ++j) {
-      const uint32_t r = r0 + warp * FIX_PER_WARP + k;
-      x[k][j] = r < rows ? out[size_t(r) * (32u * NS) + 32u * j + lane] : make_uint4(0u, 0u, 0u, 0u);
-    }
-  uint32_t mine = 0u;
-#pragma unroll
-  for (uint32_t k = 0; k < FIX_PER_WARP; ++k) {
-    bool nonfinite = false;
-#pragma unroll
-    for (uint32_t j = 0; j < NS; ++j) {
-      const uint32_t w[4] = {x[k][j].x, x[k][j].y, x[k][j].z, x[k][j].w};
-#pragma unroll
-      for (uint32_t e = 0; e < 4; ++e) nonfinite |= (w[e] & 0x7f80u) == 0x7f80u || (w[e] & 0x7f800000u) == 0x7f800000u;
-    }
-    if (__any_sync(0xffffffffu, nonfinite)) mine |= 1u << k;
-  }
-  if (lane == 0) bad[warp] = mine;
-  if (!__syncthreads_or(mine != 0u)) return;
-  for (uint32_t k = 0; k < FIX_ROWS; ++k) {
-    if (!((bad[k / FIX_PER_WARP] >> (k % FIX_PER_WARP)) & 1u)) continue;
-    attn_general_row(p, (r0 + k) / p.Hq, (r0 + k) % p.Hq);
-    __syncthreads();
-  }
-}
-
-cudaError_t launch_bitmap_fix(const AttnParams& p, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((p.C * p.Hq + FIX_ROWS - 1u) / FIX_ROWS);
-  cfg.blockDim = dim3(GEN_WARPS * 32);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return p.D == 256 ? cudaLaunchKernelEx(&cfg, dg_attn_bitmap_fix_kernel<1>, p) : cudaLaunchKernelEx(&cfg, dg_attn_bitmap_fix_kernel<2>, p);
 }
 
 // Decoder bitmap uint8 [C][T] -> one bit per key, 128-key tiles [C][n_bits] of uint4, plus for every run of PACK_ROWS

@@ -207,11 +207,12 @@ def test_small_calls(ctx, hd, P, canvas, small):
     case, seen, args = _case(hd, P, canvas, seed=hd + P)
     kv, att = util.gpu_setup(ctx, case)
     want = _general(ctx, att, kv, P, args)
-    launches = ctx.last_launch_count
+    ctx.kernel_timing(True, 4)       # counts the launches of the tensor kernels
     got = att.denoise_bitmap(kv, P, *args)
-    ctx.synchronize()
+    launches = ctx.kernel_time()[1]
+    ctx.kernel_timing(False)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert sms != 148 or (ctx.last_launch_count == launches) == small
+    assert sms != 148 or launches == (0 if small else 1)
     if small:
         assert torch.equal(got, want)
     util.assert_close(util.t2f(got), util.run_oracle(case, attend=seen), "bitmap")
