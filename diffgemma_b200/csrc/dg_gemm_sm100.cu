@@ -27,12 +27,9 @@ namespace gm {
 constexpr uint32_t GM = 128, BK = 64;   // rows of a tile, contraction elements per stage
 constexpr uint32_t THREADS = 192;
 constexpr uint32_t A_STAGE = GM * BK * 2;   // 16 KB
-// stages of the ring: deep for the projections (44-128 contraction blocks per CTA); two where the contraction is at most
-// eight blocks, so that three CTAs share an SM and one's epilogue overlaps another's loads
-__host__ __device__ constexpr uint32_t stages(uint32_t bn, bool shallow) { return shallow ? 2u : bn >= 128 ? 6u : 8u; }
-__host__ __device__ constexpr uint32_t smem_bytes(uint32_t bn, bool shallow) {
-  return stages(bn, shallow) * (A_STAGE + bn * BK * 2) + 256 + 1024;
-}
+// stages of the ring: deep, a projection has 44-128 contraction blocks per CTA
+__host__ __device__ constexpr uint32_t stages(uint32_t bn) { return bn >= 128 ? 6u : 8u; }
+__host__ __device__ constexpr uint32_t smem_bytes(uint32_t bn) { return stages(bn) * (A_STAGE + bn * BK * 2) + 256 + 1024; }
 // pair form: every CTA stages its own 128 rows of A and HALF of the W tile
 constexpr uint32_t PAIR_STAGES = 8;
 __host__ __device__ constexpr uint32_t smem_bytes_pair(uint32_t bn) { return PAIR_STAGES * (A_STAGE + bn / 2 * BK * 2) + 256 + 1024; }
@@ -42,12 +39,11 @@ __host__ __device__ constexpr uint32_t smem_bytes_pair(uint32_t bn) { return PAI
 // MMA warp issues M = 256 MMAs over both CTAs, each CTA supplies its own 128 rows of A and half of the N extent of W
 // (tm_w then has boxes {64, BN / 2}), so a weight tile is staged once per pair instead of once per CTA: 24 KB instead
 // of 32 KB cross L2 -> SM per CTA and contraction block.
-template <uint32_t BN, bool SHALLOW, bool PAIR>
+template <uint32_t BN, bool PAIR>
 __global__ void __launch_bounds__(gm::THREADS, 1)
 dg_gemm_sm100_kernel(const GemmParams g, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w) {
   using namespace gm;
-  constexpr uint32_t ST = PAIR ? PAIR_STAGES : stages(BN, SHALLOW), B_STAGE = (PAIR ? BN / 2 : BN) * BK * 2,
-                     STAGE = A_STAGE + B_STAGE;
+  constexpr uint32_t ST = PAIR ? PAIR_STAGES : stages(BN), B_STAGE = (PAIR ? BN / 2 : BN) * BK * 2, STAGE = A_STAGE + B_STAGE;
   enum : uint32_t { B_FULL = 0, B_EMPTY = ST, B_ACC = 2 * ST, B_COUNT = 2 * ST + 1 };
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -337,20 +333,11 @@ __global__ void __launch_bounds__(ROW_THREADS) dg_norm_residual_kernel(const flo
 }
 
 cudaError_t sm100_gemm_configure() {
-  cudaError_t e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<128, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(gm::smem_bytes(128, false)));
+  cudaError_t e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gm::smem_bytes(128)));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<64, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(gm::smem_bytes(64, false)));
+    e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gm::smem_bytes(64)));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<128, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(gm::smem_bytes(128, true)));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<64, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(gm::smem_bytes(64, true)));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<128, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(gm::smem_bytes_pair(128)));
+    e = cudaFuncSetAttribute(dg_gemm_sm100_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gm::smem_bytes_pair(128)));
   return e;
 }
 
@@ -372,14 +359,9 @@ cudaError_t launch_gemm_sm100(const GemmParams& g, const CUtensorMap& tm_a, cons
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
   const dim3 grid(g.N / bn, (g.M + gm::GM - 1) / gm::GM, g.part != nullptr ? g.k_slices : 1u);
-  const bool shallow = g.K / gm::BK <= 8;
-  pdl_cfg(cfg, attr, grid, dim3(gm::THREADS), gm::smem_bytes(bn, shallow), st);
-  if (shallow) {
-    if (bn == 128) return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<128, true, false>, g, tm_a, tm_w);
-    return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<64, true, false>, g, tm_a, tm_w);
-  }
-  if (bn == 128) return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<128, false, false>, g, tm_a, tm_w);
-  return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<64, false, false>, g, tm_a, tm_w);
+  pdl_cfg(cfg, attr, grid, dim3(gm::THREADS), gm::smem_bytes(bn), st);
+  if (bn == 128) return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<128, false>, g, tm_a, tm_w);
+  return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<64, false>, g, tm_a, tm_w);
 }
 
 // Pair form: exactly two row tiles (128 < M <= 256), 128 output columns per tile; tm_w has boxes {64, 64, 1}.
@@ -398,7 +380,7 @@ cudaError_t launch_gemm_sm100_pair(const GemmParams& g, const CUtensorMap& tm_a,
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<128, false, true>, g, tm_a, tm_w);
+  return cudaLaunchKernelEx(&cfg, dg_gemm_sm100_kernel<128, true>, g, tm_a, tm_w);
 }
 
 cudaError_t launch_rmsnorm_rows(const void* x, const void* w, void* y, uint32_t rows, uint32_t dim, cudaStream_t st) {
