@@ -1051,13 +1051,13 @@ static int32_t check_ptrs16(std::initializer_list<const void*> ps) {
 // 16-byte boundaries: those go to the general kernel, which reads and writes element by element.  So does an output that
 // lies over the queries (rows that come out non-finite are computed again from those: bitmap_rows_again), and a layer of
 // more query tiles than a launch of the tensor kernels takes.
-// Few rows over few keys are quicker there too: the tensor kernels' launches take 16 to 20 us however little there is to do
-// (head_dim 256, 16 heads, us general / tensor: 1 key, 1 canvas row 8.9 / 16.6; 61 keys 14.5 / 16.6; 77 keys, 17 rows, 8 KV
-// heads 18.7 / 20.4; 301 keys, 1 row 45 / 20; 160 keys, 100 rows 69 / 22; head_dim 512: 61 keys, 1 row 18.7 / 18.6, 77 keys, 17
-// rows 24.2 / 22.3).
+// Few rows over few keys are quicker there too: the tensor kernels' launches take 15 to 19 us however little there is to do
+// (head_dim 256, 16 heads, us general / tensor: 1 key, 1 canvas row 8.9 / 15.5; 61 keys 14.6 / 15.6; 77 keys, 17 rows 18.7 / 17.6
+// with 2 KV heads, 18.7 / 19.1 with 8; 301 keys, 1 row 45 / 20; 160 keys, 100 rows 69 / 21; head_dim 512: 61 keys, 1 row
+// 18.7 / 15.5).
 static bool bitmap_on_tensor(const dg_ctx* c, const dg_layer_desc& d, const AttnCall& a, uint32_t kv_len, const void* q, const void* k,
                              const void* v, const void* qw, const void* kw) {
-  if ((size_t(kv_len) + d.canvas) * d.head_dim <= 80 * 256 && d.canvas * d.n_q_heads <= 2u * uint32_t(c->num_sms)) return false;
+  if ((size_t(kv_len) + d.canvas) * d.head_dim <= 64 * 256 && d.canvas * d.n_q_heads <= 2u * uint32_t(c->num_sms)) return false;
   for (const void* p : {q, k, v, qw, kw, static_cast<const void*>(a.out)})
     if (!aligned16(p)) return false;
   const size_t bytes = size_t(d.canvas) * d.n_q_heads * d.head_dim * 2;

@@ -797,15 +797,17 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
       row_group_sync(smw);
       const uint32_t r0 = smw * 32u + qd * 8u, Rw = mt * BM + r0;
       uint32_t i = Rw / p.G, g = Rw % p.G;
+      Bf16Max largest;
 #pragma unroll
       for (uint32_t k = 0; k < 8; ++k) {
         if (Rw + k < rows_per_head) {
           const uint4 w = *reinterpret_cast<const uint4*>(rows16 + ((r0 + k) * HBUF_LD + lane * 8u) * 2u);
-          if (BITS && nonfinite_bf16x8(w)) ctl[6] = 1u;
+          if (BITS) largest.add(w);
           *reinterpret_cast<uint4*>(p.out + (size_t(i) * p.Hq + kvh * p.G + g) * HD + lane * 8u) = w;
         }
         if (++g == p.G) { g = 0; ++i; }
       }
+      if (BITS && largest.nonfinite()) ctl[6] = 1u;
     } else {
     // Each thread owns a quarter of one row in TMEM, but rows are 1 KB apart in memory.  A 32 x 32
     // chunk goes through a padded per-warp tile in shared memory (the Q tile is dead by now) so that
@@ -941,7 +943,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
         const float inv = lg[k] > 0.f ? 1.0f / lg[k] : 0.f;
         const uint4 w = make_uint4(pack_bf16x2(acc[k][0] * inv, acc[k][1] * inv), pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv),
                                    pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv), pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv));
-        if (nonfinite_bf16x8(w)) ctl[6] = 1u;
+        Bf16Max largest;
+        largest.add(w);
+        if (largest.nonfinite()) ctl[6] = 1u;
         *reinterpret_cast<uint4*>(p.out + orow[k] * HD + lane * 8) = w;
       }
     }
@@ -1290,7 +1294,9 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
             w4.y = pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv);
             w4.z = pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv);
             w4.w = pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv);
-            if (BITS && nonfinite_bf16x8(w4)) ctl[6] = 1u;
+            Bf16Max largest;
+            largest.add(w4);
+            if (BITS && largest.nonfinite()) ctl[6] = 1u;
             *reinterpret_cast<uint4*>(p.out + orow[k] * HD + lane * 8) = w4;
           } else {
             float4* dst = reinterpret_cast<float4*>(p.out_o + orow[k] * HD + lane * 8);

@@ -316,7 +316,7 @@ dg_attn_sm100_hd512_kernel(const __grid_constant__ AttnParams p, const __grid_co
   }
 
   // ------------------------------------------------------------------ epilogue (softmax warps)
-  bool nonfinite = false;      // BITS: this thread stored an infinite or NaN output
+  Bf16Max largest;      // BITS: of the output this thread stores
   if (warp < SM_WARPS) {
     bool have_o = __all_sync(0xffffffffu, n_local > 0 && !*abort_flag);
     if (have_o) {
@@ -330,7 +330,7 @@ dg_attn_sm100_hd512_kernel(const __grid_constant__ AttnParams p, const __grid_co
     row_pair_sync(smw);
     const float l_tot = xch_max[r * NTR] + xch_max[r * NTR + 1];
     // the Q tile is dead: its shared memory stages the stores
-    store_o_half(p, smem + O_Q, tmem, kvh, mt, split, dh, smw, lane, half, have_o, m_used, l_tot, BITS ? &nonfinite : nullptr);
+    store_o_half(p, smem + O_Q, tmem, kvh, mt, split, dh, smw, lane, half, have_o, m_used, l_tot, BITS ? &largest : nullptr);
   }
 
   // ------------------------------------------------------------------ teardown
@@ -346,8 +346,8 @@ dg_attn_sm100_hd512_kernel(const __grid_constant__ AttnParams p, const __grid_co
   if (warp == W_MMA) tmem_dealloc(tmem, TMEM_COLS);
 
   // ------------------------------------------------------------------ split merge by the last CTA to arrive
-  if (p.n_splits > 1) merge_splits_last(p, &ctl[2], kvh, mt, dh, THREADS, BITS ? &nonfinite : nullptr);
-  if (BITS && __syncthreads_or(nonfinite)) bitmap_rows_again<2>(p, kvh, mt, 0u, BM, dh * HDV, abort_flag);
+  if (p.n_splits > 1) merge_splits_last(p, &ctl[2], kvh, mt, dh, THREADS, BITS ? &largest : nullptr);
+  if (BITS && __syncthreads_or(largest.nonfinite())) bitmap_rows_again<2>(p, kvh, mt, 0u, BM, dh * HDV, abort_flag);
 }
 
 cudaError_t sm100_hd512_configure() {

@@ -92,7 +92,7 @@ __device__ __forceinline__ void copy_q_tile(const AttnParams& p, uint8_t* q_smem
 // threads per row (`half` = which 128 columns); `tile_smem` is dead shared memory of at least 8 x 4,608 bytes.
 __device__ __forceinline__ void store_o_half(const AttnParams& p, uint8_t* tile_smem, uint32_t tmem, uint32_t kvh, uint32_t mt,
                                              uint32_t split, uint32_t dh, uint32_t smw, uint32_t lane, uint32_t half,
-                                             bool have_o, float m_used, float l_tot, bool* nonfinite = nullptr) {
+                                             bool have_o, float m_used, float l_tot, Bf16Max* largest = nullptr) {
   const uint32_t rows_per_head = p.C * p.G;
   const uint32_t rows_total = p.C * p.Hq;
   const uint32_t r = smw * 32 + lane;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void store_o_half(const AttnParams& p, uint8_t* tile_
         uint2 w2;
         w2.x = pack_bf16x2(v4.x, v4.y);
         w2.y = pack_bf16x2(v4.z, v4.w);
-        if (nonfinite) *nonfinite |= nonfinite_bf16x8(make_uint4(w2.x, w2.y, 0u, 0u));
+        if (largest) largest->add(make_uint4(w2.x, w2.y, 0u, 0u));
         *reinterpret_cast<uint2*>(p.out + off) = w2;
       } else {
         *reinterpret_cast<float4*>(dst_o + off) = v4;
@@ -171,7 +171,7 @@ __device__ __forceinline__ void store_o_half(const AttnParams& p, uint8_t* tile_
 // partial rows of all splits.  Called by every thread of the CTA after its partial rows are stored;
 // `is_last` is one word of shared memory.
 __device__ __forceinline__ void merge_splits_last(const AttnParams& p, volatile uint32_t* is_last, uint32_t kvh, uint32_t mt,
-                                                  uint32_t dh, uint32_t n_threads, bool* nonfinite = nullptr) {
+                                                  uint32_t dh, uint32_t n_threads, Bf16Max* largest = nullptr) {
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rows_per_head = p.C * p.G;
   const uint32_t rows_total = p.C * p.Hq;
@@ -245,7 +245,7 @@ __device__ __forceinline__ void merge_splits_last(const AttnParams& p, volatile 
         w4.y = pack_bf16x2(acc[k][2] * inv, acc[k][3] * inv);
         w4.z = pack_bf16x2(acc[k][4] * inv, acc[k][5] * inv);
         w4.w = pack_bf16x2(acc[k][6] * inv, acc[k][7] * inv);
-        if (nonfinite) *nonfinite |= nonfinite_bf16x8(w4);
+        if (largest) largest->add(w4);
         *reinterpret_cast<uint4*>(p.out + off) = w4;
       } else {
         float4* dst = reinterpret_cast<float4*>(p.out_o + off);

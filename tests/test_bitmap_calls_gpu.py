@@ -200,10 +200,10 @@ def test_more_query_tiles_than_a_tensor_launch_takes(ctx, hd, heads):
     kv.close()
 
 
-@pytest.mark.parametrize("hd,P,canvas,small", [(256, 0, 1, True), (256, 62, 18, True), (256, 63, 18, False), (256, 61, 19, False),
-                                               (512, 22, 18, True), (512, 23, 18, False), (512, 21, 19, False)])
+@pytest.mark.parametrize("hd,P,canvas,small", [(256, 0, 1, True), (256, 46, 18, True), (256, 47, 18, False), (256, 45, 19, False),
+                                               (512, 14, 18, True), (512, 15, 18, False), (512, 13, 19, False)])
 def test_small_calls(ctx, hd, P, canvas, small):
-    """Both sides of the line below which the general kernel is the quicker one (80 keys of 256, two rows a multiprocessor)."""
+    """Both sides of the line below which the general kernel is the quicker one (64 keys of 256, two rows a multiprocessor)."""
     case, seen, args = _case(hd, P, canvas, seed=hd + P)
     kv, att = util.gpu_setup(ctx, case)
     want = _general(ctx, att, kv, P, args)
