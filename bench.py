@@ -768,7 +768,7 @@ def measure_topk(cfg_idx, args, timed_of, peaks, steps=50):
         rows = lay.canvas * lay.n_q_heads
         return {"workload": f"{cfg.name}: top-k sparse attention, k = {ao.topk_k(T)} of {T} keys per row", "ms_per_step": ms_topk,
                 "ms_dense_attention": ms_dense, "launches_per_step": launches, "steps": steps,
-                "score_plane_bytes": 2.0 * rows * T, "score_gemm_flops": 2.0 * rows * T * lay.head_dim, "parity": par}
+                "score_plane_bytes": 4.0 * rows * T, "score_gemm_flops": 2.0 * rows * T * lay.head_dim, "parity": par}
     finally:
         ctx.close()
 

@@ -226,8 +226,10 @@ struct SplitCost {
 // head_dim 256, a tile = 1.4 us.  32 query tiles (one canvas, 8 KV heads), us: 4 key tiles 21.3 unsplit, 20.5 with 2
 // splits, 19.1 with 4; 11 tiles 31.3 / 26.4 / 22.6; 64 query tiles: 4 key tiles 21.8 / 21.0, 11 tiles 31.7 / 27.1
 constexpr SplitCost kCost256 = {120, {14, 18, 55}, true};
-// splits that meet in memory: head_dim 512, under a bitmap, with the caller's workspace (a bitmap over 5 key tiles of 2 KV
-// heads: 27.9 us unsplit, 34.8 with 4 splits)
+// splits that meet in memory as fp32: head_dim 512, under a bitmap, with the caller's workspace.  Bitmaps, 2 KV heads, 256
+// canvas rows, us unsplit / 2 / 4 splits: 4 key tiles 27.1 / 28.8 / 26.7, 5 28.9 / 30.8 / 28.6, 7 32.5 / 32.7 / 29.1, 10
+// 38.3 / 34.9 / 31.2, 18 54.0 / 43.3 / 35.6, 34 85.4 / 60.1 / 44.8; 8 KV heads within 3 us of these; head_dim 512, 64-key
+// tiles: 10 39.8 / 40.3 / 55.0, 20 58.5 / 49.1 / 63.3, 36 85.0 / 63.7 / 78.3
 constexpr SplitCost kCostMemory = {70, {36, 44, 55}, false};
 
 static uint32_t choose_splits(const dg_ctx* ctx, uint32_t q_tiles, uint32_t k_tiles, const SplitCost& cost_of) {
@@ -254,9 +256,11 @@ static uint32_t choose_splits(const dg_ctx* ctx, uint32_t q_tiles, uint32_t k_ti
 
 // CTA pairs halve the shared-memory traffic per query tile (the single form's limiter); they need two query tiles of one
 // KV head to share a key schedule.  Their set-up is longer, and with four splits their merge goes through the workspace:
-// there they pay from about a hundred key tiles on (2 KV heads: 100 tiles 53.6 against 52.3 us, 130 tiles 62.9 / 63.4),
-// with one split or two from eight (four canvases of a sliding layer, 11 tiles: 33.2 against 35.5 us; 8 KV heads, 34
-// tiles: 67.6 / 81.0; two canvases, 24 tiles: 34.2 / 37.5).
+// there they pay from somewhat above a hundred key tiles on (2 KV heads, us pair / single: 34 tiles 33.8 / 29.9, 64 42.8 / 40.0,
+// 96 52.4 / 51.1, 110 56.9 / 56.4, 130 62.9 / 63.4; the line at 96 costs at most 2.5 % of the few lengths below 115), with one
+// split or two from eight (four canvases of a sliding layer: 8 tiles 28.3 / 29.4, 9 29.5 / 31.3, 11 33.3 / 35.8; two canvases
+// of 8 KV heads, two splits: 8 tiles 24.4 / 24.5, 10 25.7 / 26.0, 12 26.9 / 27.5; two of 2 KV heads: 10 tiles 23.4 / 24.0,
+// 24 32.4 / 34.3, 80 66.1 / 74.8).
 constexpr uint32_t kLongTiles = 96;
 static bool pair_pays(uint32_t tiles_per_head, uint32_t k_tiles, uint32_t single_splits) {
   if (tiles_per_head < 2) return false;

@@ -90,8 +90,9 @@ __device__ __forceinline__ void row_group_sync(uint32_t smw) {
 // blockIdx.z selects one of the independent canvases of the launch: its parameters and tensor maps.
 // BITS (single-CTA form only): visibility comes from a packed decoder bitmap instead of the mask rule.  P then goes to
 // the PV MMAs as the sum of two bf16 (its rounding and what that rounding left), twice the PV work, and key splits meet
-// as fp32 in the workspace: what this path replaces kept P and its partial sums in fp32.  4,096 rows x 2,304 keys of
-// 2 KV heads: 1,933 us in the CUDA-core kernel (a warp per key, bound by L2), 43.6 us here with the packing kernel.
+// as fp32 in the workspace: what this path replaces kept P and its partial sums in fp32 (against 64 bits the outputs of
+// both differ by their rounding to bf16, 1.66e-3, to within 1e-7 of one another).  4,096 rows x 2,304 keys of 2 KV heads:
+// 1,845 us in the CUDA-core kernel (a warp per key, bound by L2), 33.9 us here with the packing kernel.
 template <bool PAIR, bool BITS>
 __global__ void __launch_bounds__(one::THREADS, 1)
 dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
@@ -900,7 +901,7 @@ dg_attn_sm100_kernel(const __grid_constant__ AttnBatch bat) {
   if (BITS && cs > 1) {
     // Under a bitmap partial rows stay fp32 and are too large for shared memory on both sides: they meet in the workspace,
     // but the cluster still shares the merge, CTA k the rows [k*BM/cs, (k+1)*BM/cs), two rows per warp at a time.
-    // 4,096 rows x 2,304 keys, 4 splits: 41.9 us when the last CTA to arrive merged all rows, 34.4 so.
+    // 4,096 rows x 2,304 keys, 4 splits: 41.9 us when the last CTA to arrive merged all rows, 34 so.
     const uint32_t rpc = BM / cs;
     for (uint32_t rl0 = warp * 2u; rl0 < rpc; rl0 += (THREADS / 32) * 2u) {
       size_t orow[2];

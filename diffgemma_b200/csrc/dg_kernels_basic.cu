@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) dg_append_table_kernel(const AppendParams
 constexpr uint32_t kRowsMaxWarps = 10, kRowsUnit = 2;
 
 template <uint32_t NS>   // 16-byte chunks of a vector per lane: head_dim 256 -> 1, 512 -> 2
-// head_dim 512: 64 registers, so that three CTAs share an SM (16,000 tokens of 2 x 512: 68.7 us with 90 registers, 54.9 so)
+// head_dim 512: 64 registers, so that more CTAs share an SM (16,000 tokens of 2 x 512, four tokens a CTA: 68.7 us with 90, 54.9 so)
 __global__ void __launch_bounds__(kRowsMaxWarps * 32, NS == 2 ? 3 : 1) dg_append_rows_kernel(const AppendParams p, const RopeParams rp, uint32_t slots_per_cta) {
   __shared__ __align__(16) float2 cs[kMaxRotHalf];   // read as float4
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -340,7 +340,7 @@ void launch_append(const AppendParams& p, const RopeParams& rp, cudaStream_t st,
 // ------------------------------------------------------------------------------------------
 // Saved sessions: rows of a token-major [n][Hkv][D] tensor to or from the head-major cache, K and V in one launch
 // (blockIdx.y), 16 bytes per access, four in flight per thread.  Bound: memory.  8,192 tokens of 2 x 512 loaded, 2,000
-// appended and all read back: 131.3 us with a strided copy per head, tensor and direction, 45.7 us with this and
+// appended and all read back: 131.3 us with a strided copy per head, tensor and direction, 42.4 us with this and
 // dg_append_rows_kernel (84 MB, 12.8 us at copy bandwidth; the rest is launches and the wait of the read).
 // ------------------------------------------------------------------------------------------
 constexpr uint32_t kCopyChunks = 4;

@@ -13,9 +13,9 @@
 //      lowest indices among what equals it;
 //   4. softmax over the kept scores, and the gather of V, a warp per kept key.
 // Lists that outgrow shared memory (many equal scores, clustered ones) take the same steps over the groups in memory.
-// Bound: the gather (4,096 rows x 258 keys x 1 KB = 1.08 GB out of L2 at head_dim 512): 175 us of 349 for the whole call at
-// 33,024 keys, 6.7 TB/s into the SMs.  With bf16 scores, two histograms over all of a row and the exact scores of the kept keys computed again
-// from K (another 1.08 GB gathered) the call took 900 us.
+// Bound: the gather (4,096 rows x 258 keys x 1 KB = 1.08 GB out of L2 at head_dim 512): 175 us of 354 for the whole call at
+// 33,024 keys, 6.2 TB/s into the SMs.  With bf16 scores, two histograms over all of a row and the exact scores of the kept
+// keys computed again from K (another 1.08 GB gathered) the call took 900 us.
 #include <cuda.h>
 
 #include "dg_common.cuh"

@@ -8,10 +8,11 @@
 // equal contiguous runs, one per pair, so the last wave is full whatever the key count.
 //
 // Bound: writing the scores.  4,096 rows x 33,024 keys are 541 MB of fp32 against 61 (head_dim 512) or 31 us (256) of
-// MMA work: 150 us in two passes at head_dim 512 (3.6 TB/s of plane, 4.2 TB/s of DRAM traffic; smaller passes that would
-// stay in L2 lose more to their launches: 372 us for the call with 288 MB, 418 with 144, 462 with 72).  So the plane is laid out for the writer: 32 rows of 8 keys are one contiguous KB, which a warp (lane = row)
-// stores with one 32-byte access per lane.  A group of 16 keys of a row is then two whole 32-byte sectors, and the
-// selection reads only the groups whose maximum can matter, about one in eight.
+// MMA work: 143 us in two passes at head_dim 512 (3.8 TB/s of plane, 4.0 TB/s of DRAM traffic, tensor pipe 48 %; smaller
+// passes that would stay in L2 lose more to their launches: 372 us for the call with 288 MB, 418 with 144, 462 with 72).  So
+// the plane is laid out for the writer: 32 rows of 8 keys are one contiguous KB, which a warp (lane = row) stores with one
+// 32-byte access per lane.  A group of 16 keys of a row is then two whole 32-byte sectors, and the selection reads only the
+// groups whose maximum can matter, about one in eight.
 #include <cuda.h>
 
 #include "dg_attn_sm100_common.cuh"
@@ -30,8 +31,8 @@ __host__ __device__ constexpr uint32_t smem_bytes(uint32_t D) { return (D / BK +
 }  // namespace ts
 
 // A pass of the plane is larger than L2 and one group in eight of it is read, once: marked evict-first it leaves L2 to K,
-// which every row pair reads, and to V (33,024 keys, head_dim 512: 368 us for the call without the mark, 357 with it, 349
-// with the selection's reads of the plane marked as well).
+// which every row pair reads, and to V (33,024 keys, head_dim 512, one run: 368 us for the call without the mark, 357 with it,
+// 349 with the selection's reads of the plane marked as well).
 __device__ __forceinline__ void st_global_v8(void* dst, const uint32_t* v) {
   asm volatile("st.global.L2::evict_first.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
