@@ -256,7 +256,8 @@ int32_t dg_host_pipe_set_deferred_launch(dg_host_pipe* pipe, int32_t on);
 /* General decoder bitmap (reference DecoderAttnMask, src/model/mask.rs:4-27): attend is a
  * device pointer to uint8 [C][kv_len+C], 1 = visible.  head_dim 256 / 512 with every tensor on a
  * 16-byte boundary: packed to bits, then the tensor kernels; otherwise, and where there is little
- * to do, the general kernel.                                                                     */
+ * to do, the general kernel.  Keys that a row does not see may hold anything, infinities and NaN
+ * included.                                                                                      */
 int32_t dg_attn_denoise_bitmap(dg_ctx* ctx, const dg_layer_desc* desc, dg_kv* kv, uint32_t kv_len,
                                const void* q, const void* k, const void* v, const void* qw, const void* kw,
                                const uint8_t* attend, void* out);

@@ -80,16 +80,17 @@ def test_short_ranges_keep_fp32_sums(ctx, Hkv, canvas, P, batch):
         kv.close()
 
 
-@pytest.mark.parametrize("Hkv,canvas,window,Ps", [
-    (8, 256, 1024, (333, 5000, 5000, 5000)),      # 5 and 11 key tiles: both sides of where pairs begin to pay
-    (8, 256, 1024, (2000, 600, 9000)),
-    (2, 256, 0, (333, 2048)),
-    (2, 256, 0, (500, 4000, 4000, 4000)),
-    (2, 256, 0, (0, 700, 40, 4000, 260)),         # two launches of up to four
+@pytest.mark.parametrize("Hkv,canvas,mask,Ps", [
+    (8, 256, capi.MASK_WINDOW_UNIFORM, (333, 5000, 5000, 5000)),      # 5 and 11 key tiles: both sides of where pairs begin to pay
+    (8, 256, capi.MASK_WINDOW_UNIFORM, (2000, 600, 9000)),
+    (2, 256, capi.MASK_NONE, (333, 2048)),
+    (2, 256, capi.MASK_NONE, (500, 4000, 4000, 4000)),
+    (2, 256, capi.MASK_NONE, (0, 700, 40, 4000, 260)),                # two launches of up to four
+    (8, 256, capi.MASK_CAUSAL, (0, 1500)),                            # query tiles whose first split has no key tile
+    (8, 256, capi.MASK_WINDOW_PER_ROW, (10, 3000)),
 ])
-def test_unequal_canvases_share_a_launch(ctx, Hkv, canvas, window, Ps):
-    layer = AttnLayer(n_kv_heads=Hkv, canvas=canvas, rope_theta=1e4, window=window,
-                      mask_mode=capi.MASK_WINDOW_UNIFORM if window else capi.MASK_NONE)
+def test_unequal_canvases_share_a_launch(ctx, Hkv, canvas, mask, Ps):
+    layer = AttnLayer(n_kv_heads=Hkv, canvas=canvas, rope_theta=1e4, window=1024 if mask else 0, mask_mode=mask)
     cases = [util.make_case(layer, P, seed=70 + b) for b, P in enumerate(Ps)]
     kvs = [util.gpu_setup(ctx, c)[0] for c in cases]
     att = CanvasAttention(ctx, layer)
